@@ -66,6 +66,22 @@ struct SlabSource {
     std::vector<int32_t> count;        // [nsrc * 32] entries per ray
 };
 
+// Geometry of the strip-word path (strip.cu): integer patterns, FP32 method.
+struct StripGeom {
+    int ok = 0;
+    int SB = 0, P = 0;                 // strips per phase, word table pitch (rows)
+    int gpt = 0, nRaysPad = 0;         // 32-ray groups per theta, rays of a pattern's means row
+    int ntask = 0;                     // blocks per unit of patterns
+    int U[2] = {0, 0}, V[2] = {0, 0}, PV[2] = {0, 0};  // strip axis extent (padded), cross axis, its pitch
+    size_t axis1 = 0, unit_elems = 0;  // interleaved elements: by-row copy's start, a unit's count
+    int NC = 0, PC = 0, nseg = 0, SW = 0, np = 0, hb = 0, FW = 0, FC = 0;  // peak kernel tile (see PeakArgs)
+    int nslab = 0;                     // theta slabs of a pattern
+    int capf = 0, sms = 0;
+    int mask_fixed = 0;                // the Radon mask is the same for every theta
+    int64_t ncr = 0;                   // entries of one half of d_st_cr
+    int64_t chunk = 0;                 // patterns per pass over the workspace
+};
+
 struct Workspace {
     void* ptr = nullptr;
     size_t bytes = 0;
@@ -127,8 +143,20 @@ struct ebsd_plan_s {
     // 1 the single tile, 2 theta slabs (ebsd_plan_set_tile, ebsd_plan_autotune)
     int tile_mode = 0;
 
+    // strip-word tables (see strip.cu)
+    ebsd::StripGeom st;
+    void* d_st_tasks = nullptr;    // [ntask] StripTask
+    uint16_t* d_st_lut = nullptr;  // per task [phase][slots / (8 / SB)][thread] 8 table byte offsets
+    uint32_t* d_st_act = nullptr;  // per task [phase][warp] slots with pixels in the phase
+    void* d_st_cr = nullptr;       // per task [slot][thread] float4 count, RN(1 / count), bias, ray; uint16 then uint8
+    uint32_t* d_st_mask = nullptr; // [nTheta][FW / 4] Radon mask, a nibble per lane
+    uint8_t* d_st_used = nullptr;  // [nPx] pixels some ray holds
+
     // ---- workspaces ----
     std::mutex mtx;
+    ebsd::Workspace st_ws;         // strip path: interleaved pixels, Radon means, slab peaks
+    cudaEvent_t st_event = nullptr;    // end of the last call that used st_ws, and its stream
+    cudaStream_t st_stream = nullptr;
     ebsd::Workspace ws;            // per-stage intermediates
     ebsd::Workspace stats;         // per-pattern min/mean
     int64_t ws_chunk = 0;
@@ -219,6 +247,15 @@ void slab_release(ebsd_plan_s* p);
 bool slab_serves(const ebsd_plan_s* p, int method, int dtype);
 int slab_run_chunk(ebsd_plan_s* p, int method, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out,
                    int64_t out_offset, cudaStream_t st, int64_t* launches);
+// Strip-word path: strip.cu ---------------------------------------------------------------
+int strip_prepare(ebsd_plan_s* p, const ebsd_plan_desc* d);
+void strip_release(ebsd_plan_s* p);
+bool strip_serves(const ebsd_plan_s* p, int method, int dtype);
+int strip_reserve(ebsd_plan_s* p);
+bool strip_ready(ebsd_plan_s* p, cudaStream_t st);
+int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
+                    cudaStream_t st, int64_t* launches);
+
 // mixed pattern sizes in one launch: up to 8 plans of one input type and LoG size
 constexpr int kMaxMixedPlans = 8;
 bool slab_mixable(const ebsd_plan_s* p, int dtype);

@@ -40,6 +40,7 @@ void free_plan_tables(ebsd_plan_s* p) {
     cudaFree(p->d_bgf);
     fused_release(p);
     slab_release(p);
+    strip_release(p);
     cudaFree(p->ws.ptr);
     p->ws = Workspace{};
     cudaFree(p->stats.ptr);
@@ -82,7 +83,10 @@ size_t workspace_bytes(const ebsd_plan_s* p, int method, int64_t chunk) {
                             : fused_workspace_bytes(p, method, chunk);
 }
 
-int reserve(ebsd_plan_s* p, int method, int64_t chunk) {
+// Scratch of a call: the strip path's for the input types it takes, else (or when the device has no
+// room for that) the method's own.
+int reserve(ebsd_plan_s* p, int method, int64_t chunk, int dtype, cudaStream_t st) {
+    if (strip_serves(p, method, dtype) && strip_ready(p, st)) return EBSD_OK;
     size_t need = workspace_bytes(p, method, chunk);
     if (need > p->ws.bytes) {
         cudaFree(p->ws.ptr);
@@ -236,7 +240,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
     if (chunk <= 0) chunk = is_plain(method) ? default_chunk(p, method) : 65536;
     if (is_plain(method)) chunk = std::min<int64_t>(chunk, 65535);
     chunk = std::min(chunk, n);
-    int rc = reserve(p, method, chunk);
+    int rc = reserve(p, method, chunk, dtype, p->hstream[0]);
     if (rc != EBSD_OK) return rc;
     const int nB = p->nB;
     const size_t in_bytes = (size_t)chunk * src.pat_bytes;
@@ -628,6 +632,7 @@ int ebsd_plan_create(const ebsd_plan_desc* d, int device, ebsd_plan_t* out) {
     }
     if (rc == EBSD_OK) rc = fused_prepare(p, d);
     if (rc == EBSD_OK) rc = slab_prepare(p, d);
+    if (rc == EBSD_OK) rc = strip_prepare(p, d);
     if (rc != EBSD_OK) {
         free_plan_tables(p);
         delete p;
@@ -670,7 +675,9 @@ int ebsd_plan_reserve(ebsd_plan_t p, int method, int64_t max_chunk) {
     if (rc != EBSD_OK) return rc;
     std::lock_guard<std::mutex> lk(p->mtx);
     if (cudaSetDevice(p->device) != cudaSuccess) return EBSD_E_DEVICE;
-    return reserve(p, method, is_plain(method) ? std::min<int64_t>(max_chunk, 65535) : max_chunk);
+    // every input type: the strip path's scratch (integers) and the method's own
+    if (method == EBSD_FUSED_F32) strip_reserve(p);
+    return reserve(p, method, is_plain(method) ? std::min<int64_t>(max_chunk, 65535) : max_chunk, EBSD_F32, nullptr);
 }
 
 int64_t ebsd_last_launch_count(ebsd_plan_t p) { return p ? p->last_launches : -1; }
@@ -692,9 +699,9 @@ int ebsd_find_bands(ebsd_plan_t p, int method, int dtype, const void* d_pats, in
     if (chunk <= 0) chunk = default_chunk(p, method);
     if (is_plain(method)) chunk = std::min<int64_t>(chunk, 65535);
     chunk = std::min(chunk, n);
-    rc = reserve(p, method, chunk);
-    if (rc != EBSD_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
+    rc = reserve(p, method, chunk, dtype, st);
+    if (rc != EBSD_OK) return rc;
     size_t es = elem_size(dtype);
     for (int64_t s = 0; s < n; s += chunk) {
         int64_t m = std::min(chunk, n - s);
@@ -724,7 +731,16 @@ int ebsd_find_bands_mixed(const ebsd_plan_t* plans, int nplans, int dtype, const
     if (cudaSetDevice(plans[0]->device) != cudaSuccess) return EBSD_E_DEVICE;
     std::vector<ebsd_plan_s*> ps(plans, plans + nplans);
     int64_t launches = 0;
-    const int rc = slab_run_mixed(ps.data(), nplans, dtype, d_pats, n, d_out, (cudaStream_t)stream, &launches);
+    cudaStream_t st = (cudaStream_t)stream;
+    bool strips = true;
+    for (ebsd_plan_s* p : ps) strips = strips && strip_serves(p, EBSD_FUSED_F32, dtype) && strip_ready(p, st);
+    int rc = EBSD_OK;
+    if (strips) {  // size by size: each fills the GPU by itself
+        for (int k = 0; k < nplans && rc == EBSD_OK; ++k)
+            rc = strip_run_chunk(ps[k], dtype, d_pats[k], n[k], &d_out[k], 0, st, &launches);
+    } else {
+        rc = slab_run_mixed(ps.data(), nplans, dtype, d_pats, n, d_out, st, &launches);
+    }
     for (ebsd_plan_s* p : order) p->last_launches = launches;
     return rc;
 }
@@ -880,8 +896,14 @@ int ebsd_plan_autotune(ebsd_plan_t p, int method, int dtype, const void* d_pats,
         if (patterns_per_pass) *patterns_per_pass = 1;
         return EBSD_OK;
     }
-    rc = reserve(p, method, n);
+    rc = reserve(p, method, n, dtype, st);
     if (rc != EBSD_OK) return rc;
+    if (strip_serves(p, method, dtype) && strip_ready(p, st)) {
+        // one variant: the strip path takes these calls whatever the tile shape
+        p->fused_ppp = -1;
+        if (patterns_per_pass) *patterns_per_pass = dtype == EBSD_U8 ? 8 : 1;
+        return EBSD_OK;
+    }
     // the candidates, which give identical records: the single tile with 8, 4, 2 or 1 patterns
     // per block pass, and theta slabs from the widest that fit to three more
     struct Cand {
