@@ -164,7 +164,7 @@ struct ebsd_plan_s {
 
     // host-pipeline buffers (ebsd_find_bands_host)
     cudaStream_t hstream[2] = {nullptr, nullptr};
-    cudaEvent_t hevent[2] = {nullptr, nullptr};
+    cudaEvent_t hpipe[7] = {};     // host pipelines: 3 uploads, 2 detections, 2 result copies done
     void* h_in_dev[2] = {nullptr, nullptr};
     void* h_out_dev[2] = {nullptr, nullptr};
     size_t h_in_bytes = 0, h_out_bytes = 0;

@@ -47,13 +47,15 @@ void free_plan_tables(ebsd_plan_s* p) {
     p->stats = Workspace{};
     for (int i = 0; i < 2; ++i) {
         if (p->hstream[i]) cudaStreamDestroy(p->hstream[i]);
-        if (p->hevent[i]) cudaEventDestroy(p->hevent[i]);
         cudaFree(p->h_in_dev[i]);
         cudaFree(p->h_out_dev[i]);
         p->hstream[i] = nullptr;
-        p->hevent[i] = nullptr;
         p->h_in_dev[i] = nullptr;
         p->h_out_dev[i] = nullptr;
+    }
+    for (cudaEvent_t& e : p->hpipe) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
     }
     for (int i = 0; i < 3; ++i) {
         if (p->h_pin[i]) cudaFreeHost(p->h_pin[i]);
@@ -229,6 +231,22 @@ ebsd_bands chunk_fields(char* base, size_t nb) {
     return d;
 }
 
+// Pageable input of a call that is one chunk, read in place: staging it first (a host copy into a pinned
+// slot, then the upload) has nothing to overlap with.  528 patterns of 80x80 take 365 us per call
+// instead of 610, 8,192 (52 MB) 2.5 ms instead of 3.1; larger scans are chunked and staged, since the GPU
+// reads pageable memory at 24 GB/s only.  The strip path's kernels read every input byte once.
+constexpr size_t kInPlaceBytes = (size_t)64 << 20;
+
+// The host touches the input's pages first, so that a page the system has yet to provide is faulted in
+// here and not under the GPU.
+void touch_pages(const char* mem, size_t bytes) {
+    const size_t page = (size_t)std::max<long>(sysconf(_SC_PAGESIZE), 4096);
+    volatile char sink = 0;
+    for (size_t b = 0; b < bytes; b += page) sink = mem[b];
+    if (bytes) sink = mem[bytes - 1];
+    (void)sink;
+}
+
 // Host-buffer pipeline shared by ebsd_find_bands_host and ebsd_find_bands_file.  Two CUDA
 // streams alternate chunks: chunk k + 1's upload overlaps chunk k's detection (the shared
 // workspace orders the detections through events).  Pageable or file input goes through three
@@ -247,8 +265,9 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
     const size_t out_bytes = (size_t)chunk * nB * (10 * sizeof(float) + 1) + 256;
     for (int i = 0; i < 2; ++i) {
         if (!p->hstream[i]) EBSD_CUDA_TRY(cudaStreamCreateWithFlags(&p->hstream[i], cudaStreamNonBlocking));
-        if (!p->hevent[i]) EBSD_CUDA_TRY(cudaEventCreateWithFlags(&p->hevent[i], cudaEventDisableTiming));
     }
+    for (cudaEvent_t& e : p->hpipe)
+        if (!e) EBSD_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     auto regrow = [](void** bufs, int count, size_t* have, size_t want, bool host) -> int {
         if (want <= *have) return EBSD_OK;
         for (int i = 0; i < count; ++i) {
@@ -263,7 +282,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         *have = want;
         return EBSD_OK;
     };
-    const bool ring = !(src.mem && src.mem_pinned);
+    bool ring = !(src.mem && src.mem_pinned);
     // pinned input read in place by the kernels over the CPU-GPU link (no staging copy) when
     // the device uses the host page tables (GB300's NVLink-C2C) or the caller asked for it
     const char* in_place = nullptr;
@@ -275,6 +294,16 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
             pa.devicePointer)
             in_place = (const char*)pa.devicePointer;
         cudaGetLastError();
+    }
+    if (ring && src.mem && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
+        strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0])) {
+        int coherent = 0;
+        cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
+        if (coherent) {
+            touch_pages(src.mem, in_bytes);
+            in_place = src.mem;
+            ring = false;
+        }
     }
     const bool direct_out = !sink && is_pinned(h_out->max) && is_pinned(h_out->normmax) &&
                             is_pinned(h_out->maxloc) && is_pinned(h_out->avemax) && is_pinned(h_out->aveloc) &&
@@ -326,10 +355,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         });
     }
 
-    cudaEvent_t copied[3], done_compute[2], out_done[2];
-    for (int i = 0; i < 3; ++i) cudaEventCreateWithFlags(&copied[i], cudaEventDisableTiming);
-    for (int i = 0; i < 2; ++i) cudaEventCreateWithFlags(&done_compute[i], cudaEventDisableTiming);
-    for (int i = 0; i < 2; ++i) cudaEventCreateWithFlags(&out_done[i], cudaEventDisableTiming);
+    cudaEvent_t *copied = p->hpipe, *done_compute = p->hpipe + 3, *out_done = p->hpipe + 5;
     int64_t staged_s[2] = {-1, -1}, staged_n[2] = {0, 0};
     auto flush = [&](int ds) {  // staged records of slot ds -> the caller's arrays
         if (staged_s[ds] < 0) return;
@@ -392,19 +418,21 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
             flush(ds);  // chunk k - 2's records leave the staging buffer first
             dst = chunk_fields((char*)p->h_outpin[ds], nb);
         }
+        if (!direct_out) {  // both sides hold the fields one after the other
+            if (cudaMemcpyAsync(dst.max, dev.max, nb * (10 * sizeof(float) + 1), cudaMemcpyDeviceToHost, st) != cudaSuccess)
+                rc = EBSD_E_LAUNCH;
+            cudaEventRecord(out_done[ds], st);
+            staged_s[ds] = s0;
+            staged_n[ds] = cnt;
+        }
         const std::pair<void*, const void*> parts[9] = {
             {dst.max, dev.max}, {dst.normmax, dev.normmax}, {dst.maxloc, dev.maxloc}, {dst.avemax, dev.avemax},
             {dst.aveloc, dev.aveloc}, {dst.width, dev.width}, {dst.theta, dev.theta}, {dst.rho, dev.rho},
             {dst.valid, dev.valid}};
         const size_t sizes[9] = {nb * 4, nb * 4, nb * 8, nb * 4, nb * 8, nb * 4, nb * 4, nb * 4, nb};
-        for (int f = 0; f < 9 && rc == EBSD_OK; ++f)
+        for (int f = 0; f < 9 && direct_out && rc == EBSD_OK; ++f)
             if (cudaMemcpyAsync(parts[f].first, parts[f].second, sizes[f], cudaMemcpyDeviceToHost, st) != cudaSuccess)
                 rc = EBSD_E_LAUNCH;
-        if (!direct_out) {
-            cudaEventRecord(out_done[ds], st);
-            staged_s[ds] = s0;
-            staged_n[ds] = cnt;
-        }
         if (k >= 1) {
             if (ring) {  // chunk k - 1's upload was issued an iteration ago; its slot takes chunk k + 2
                 const int ps = (int)((k - 1) % 3);
@@ -432,9 +460,6 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         flush(0);
         flush(1);
     }
-    for (int i = 0; i < 3; ++i) cudaEventDestroy(copied[i]);
-    for (int i = 0; i < 2; ++i) cudaEventDestroy(done_compute[i]);
-    for (int i = 0; i < 2; ++i) cudaEventDestroy(out_done[i]);
     if (rc != EBSD_OK) return rc;
     if (e0 != cudaSuccess || e1 != cudaSuccess) return EBSD_E_LAUNCH;
     return EBSD_OK;
