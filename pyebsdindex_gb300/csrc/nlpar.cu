@@ -16,6 +16,7 @@
 #include "ebsd_internal.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace ebsd {
 namespace {
@@ -400,11 +401,43 @@ void launch_average_tiled(dim3 grid, dim3 block, size_t smem, cudaStream_t st, c
     }
 }
 
+typedef unsigned long long Pair2;              // two floats in a 64-bit register
+__device__ __forceinline__ Pair2 p2_pack(float a, float b) {
+    Pair2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ float2 p2_unpack(Pair2 p) {
+    float2 d;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(d.x), "=f"(d.y) : "l"(p));
+    return d;
+}
+__device__ __forceinline__ Pair2 p2_add(Pair2 a, Pair2 b) {
+    Pair2 d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// a * b, rounded by itself: the assembler contracts mul.f32x2 with an add that follows it into one
+// multiply-add, so the product is a multiply-add of a zero that it cannot see (z, a run-time value)
+__device__ __forceinline__ Pair2 p2_mul(Pair2 a, Pair2 b, Pair2 z) {
+    Pair2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(z));
+    return d;
+}
+// a - b: b's product with -1 is exact, so the sum is rounded once
+__device__ __forceinline__ Pair2 p2_sub(Pair2 a, Pair2 b, Pair2 minus_one) {
+    Pair2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(minus_one), "l"(a));
+    return d;
+}
+
 // Weighted window sum, register-blocked along the scan row (search radius SR fixed).  A block
-// takes RP neighbouring scan pixels of one row and 4 * kRbThreads pattern values; each thread
-// holds the RP pixels' sums for four consecutive pattern values and streams the window rows'
-// RP + 2 SR columns once: a loaded value feeds every pixel whose window holds its column, and a
-// broadcast weight feeds the four values.  Each sum adds its window slots in window order
+// takes RP neighbouring scan pixels of two rows and 4 * kRbThreads pattern values; each thread
+// holds the 2 RP pixels' sums for four consecutive pattern values and streams the window rows'
+// RP + 2 SR columns once: a loaded value feeds every pixel whose window holds it, and a broadcast
+// weight feeds the four values, two at a time (packed products and sums, each rounded as its own).
+// What bounds it is L2: with one row a block the 98 loads of 16 bytes per 8 pixels came to 9.7 TB/s
+// (128x160 scan of 80x80, radius 3: 0.66 ms packed, 0.80 ms with scalar products).  Each sum adds its window slots in window order
 // (rows, then columns) as fadd(acc, fmul(value, weight)) from zero -- the order and rounding of
 // k_nlpar_average -- so the result equals the tiled kernel's bit for bit.  Needs npx % 4 == 0
 // and 16-byte aligned data.
@@ -427,73 +460,98 @@ template <> __device__ __forceinline__ void store4<uint16_t>(uint16_t* dst, cons
 template <typename O, int SR>
 __global__ void __launch_bounds__(kRbThreads) k_nlpar_average_rb(const float* __restrict__ data, int nrows, int ncols,
                                                                   int npx, const float* __restrict__ w,
-                                                                  O* __restrict__ out) {
+                                                                  O* __restrict__ out, float zero) {
     constexpr int WN = 2 * SR + 1, WS = WN * WN, RP = kRbPix, NC = RP + 2 * SR;
-    __shared__ float ws[RP * WS];
-    const int y = blockIdx.z, p0 = blockIdx.y * RP;
-    const int np = ncols - p0 < RP ? ncols - p0 : RP;
-    for (int i = threadIdx.x; i < np * WS; i += kRbThreads) ws[i] = w[(int64_t)(y * ncols + p0) * WS + i];
+    __shared__ Pair2 ws[2][RP * WS];  // each weight twice: one multiplies two pattern values at a time
+    const Pair2 z = p2_pack(zero, zero);
+    const int y = 2 * blockIdx.z, p0 = blockIdx.y * RP;
+    const int np = ncols - p0 < RP ? ncols - p0 : RP, ny = nrows - y < 2 ? nrows - y : 2;
+    for (int i = threadIdx.x; i < ny * np * WS; i += kRbThreads) {
+        const int k = i / (np * WS), c = i - k * np * WS;
+        const float v = w[((int64_t)(y + k) * ncols + p0) * WS + c];
+        ws[k][c] = p2_pack(v, v);
+    }
     __syncthreads();
     const int k = (blockIdx.x * kRbThreads + threadIdx.x) * 4;
     if (k >= npx) return;
-    int ys, ye;
+    int ys, ye, ys1;
+    window(y + ny - 1, SR, nrows, ys1, ye);  // the second row's window (one row: its own)
+    const int y_last = ye;
     window(y, SR, nrows, ys, ye);
-    float acc[RP][4];
+    const int sh = ys1 - ys;                 // 0 at the scan's top and bottom, else 1
+    Pair2 acc[2][RP][2];
 #pragma unroll
-    for (int m = 0; m < RP; ++m)
+    for (int m = 0; m < RP; ++m) acc[0][m][0] = acc[0][m][1] = acc[1][m][0] = acc[1][m][1] = 0ull;
+    const bool centred = p0 >= SR && p0 + RP + SR <= ncols;
+    int xs[RP];
 #pragma unroll
-        for (int t = 0; t < 4; ++t) acc[m][t] = 0.0f;
-    if (p0 >= SR && p0 + RP + SR <= ncols) {
-        // every window of the block is centred: column j of the strip is slot j - m of pixel m
-#pragma unroll
-        for (int r = 0; r < WN; ++r) {
-            const float* src = data + ((int64_t)(ys + r) * ncols + (p0 - SR)) * npx + k;
+    for (int m = 0; m < RP; ++m) {
+        int xe;
+        window(m < np ? p0 + m : p0 + np - 1, SR, ncols, xs[m], xe);
+    }
+    // window row i of both pixel rows' union: slot row i of the first, i - sh of the second
+    auto row = [&](int i, auto first, auto second) {
+        constexpr bool kA = decltype(first)::value, kB = decltype(second)::value;
+        const Pair2 *wa = ws[0] + i * WN, *wb = ws[1] + (i - sh) * WN;
+        if (centred) {
+            // every window of the block is centred: column j of the strip is slot j - m of pixel m
+            const float* src = data + ((int64_t)(ys + i) * ncols + (p0 - SR)) * npx + k;
 #pragma unroll
             for (int j = 0; j < NC; ++j) {
-                const float4 v = __ldg((const float4*)(src + (int64_t)j * npx));
+                const ulonglong2 v = __ldg((const ulonglong2*)(src + (int64_t)j * npx));
 #pragma unroll
                 for (int m = 0; m < RP; ++m) {
-                    if (j - m >= 0 && j - m < WN) {
-                        const float wv = ws[m * WS + r * WN + (j - m)];
-                        acc[m][0] = wadd(acc[m][0], v.x, wv);
-                        acc[m][1] = wadd(acc[m][1], v.y, wv);
-                        acc[m][2] = wadd(acc[m][2], v.z, wv);
-                        acc[m][3] = wadd(acc[m][3], v.w, wv);
+                    if (j - m < 0 || j - m >= WN) continue;
+                    if (kA) {
+                        const Pair2 wv = wa[m * WS + (j - m)];
+                        acc[0][m][0] = p2_add(acc[0][m][0], p2_mul(v.x, wv, z));
+                        acc[0][m][1] = p2_add(acc[0][m][1], p2_mul(v.y, wv, z));
+                    }
+                    if (kB) {
+                        const Pair2 wv = wb[m * WS + (j - m)];
+                        acc[1][m][0] = p2_add(acc[1][m][0], p2_mul(v.x, wv, z));
+                        acc[1][m][1] = p2_add(acc[1][m][1], p2_mul(v.y, wv, z));
                     }
                 }
             }
-        }
-    } else {
-        // windows shifted inward at the scan's left / right edge: window starts from window()
-        int xs[RP];
-#pragma unroll
-        for (int m = 0; m < RP; ++m) {
-            int xe;
-            window(m < np ? p0 + m : p0 + np - 1, SR, ncols, xs[m], xe);
-        }
-        const int c0 = xs[0], c1 = xs[np - 1] + 2 * SR;  // window starts do not decrease with m
-#pragma unroll
-        for (int r = 0; r < WN; ++r) {
-            const float* src = data + (int64_t)(ys + r) * ncols * npx + k;
-            for (int c = c0; c <= c1; ++c) {
-                const float4 v = __ldg((const float4*)(src + (int64_t)c * npx));
+        } else {
+            // windows shifted inward at the scan's left / right edge (starts do not decrease with m)
+            const float* src = data + (int64_t)(ys + i) * ncols * npx + k;
+            for (int c = xs[0]; c <= xs[RP - 1] + 2 * SR; ++c) {
+                const ulonglong2 v = __ldg((const ulonglong2*)(src + (int64_t)c * npx));
 #pragma unroll
                 for (int m = 0; m < RP; ++m) {
                     const int d = c - xs[m];
-                    if (m < np && d >= 0 && d < WN) {
-                        const float wv = ws[m * WS + r * WN + d];
-                        acc[m][0] = wadd(acc[m][0], v.x, wv);
-                        acc[m][1] = wadd(acc[m][1], v.y, wv);
-                        acc[m][2] = wadd(acc[m][2], v.z, wv);
-                        acc[m][3] = wadd(acc[m][3], v.w, wv);
+                    if (m >= np || d < 0 || d >= WN) continue;
+                    if (kA) {
+                        const Pair2 wv = wa[m * WS + d];
+                        acc[0][m][0] = p2_add(acc[0][m][0], p2_mul(v.x, wv, z));
+                        acc[0][m][1] = p2_add(acc[0][m][1], p2_mul(v.y, wv, z));
+                    }
+                    if (kB) {
+                        const Pair2 wv = wb[m * WS + d];
+                        acc[1][m][0] = p2_add(acc[1][m][0], p2_mul(v.x, wv, z));
+                        acc[1][m][1] = p2_add(acc[1][m][1], p2_mul(v.y, wv, z));
                     }
                 }
             }
         }
+    };
+    for (int i = 0; ys + i < y_last; ++i) {
+        const bool a = i < WN, b = ny == 2 && i >= sh;
+        if (a && b) row(i, std::true_type(), std::true_type());
+        else if (a) row(i, std::true_type(), std::false_type());
+        else row(i, std::false_type(), std::true_type());
     }
 #pragma unroll
-    for (int m = 0; m < RP; ++m)
-        if (m < np) store4<O>(out + (int64_t)(y * ncols + p0 + m) * npx + k, acc[m]);
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int m = 0; m < RP; ++m)
+            if (m < np && h < ny) {
+                const float2 a = p2_unpack(acc[h][m][0]), b = p2_unpack(acc[h][m][1]);
+                const float v[4] = {a.x, a.y, b.x, b.y};
+                store4<O>(out + ((int64_t)(y + h) * ncols + p0 + m) * npx + k, v);
+            }
 }
 
 // The weighted window sum of the pair path: the register-blocked kernel where it applies
@@ -508,11 +566,11 @@ void launch_average(dim3 tgrid, dim3 tblock, size_t tsmem, cudaStream_t st, cons
         return;
     }
     const dim3 grid((unsigned)((npx / 4 + kRbThreads - 1) / kRbThreads), (unsigned)((ncols + kRbPix - 1) / kRbPix),
-                    (unsigned)nrows);
+                    (unsigned)((nrows + 1) / 2));
     switch (sr) {
-        case 1: k_nlpar_average_rb<O, 1><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out); break;
-        case 2: k_nlpar_average_rb<O, 2><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out); break;
-        default: k_nlpar_average_rb<O, 3><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out); break;
+        case 1: k_nlpar_average_rb<O, 1><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out, 0.0f); break;
+        case 2: k_nlpar_average_rb<O, 2><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out, 0.0f); break;
+        default: k_nlpar_average_rb<O, 3><<<grid, kRbThreads, 0, st>>>(data, nrows, ncols, npx, w, out, 0.0f); break;
     }
 }
 
@@ -526,8 +584,6 @@ void launch_average(dim3 tgrid, dim3 tblock, size_t tsmem, cudaStream_t st, cons
 // shifted inward at the scan edges have, are summed directly from memory.  With kSig the
 // kernel also sums the four forward 3x3 neighbours under sigma_numba's saturation level, from
 // which k_nlpar_sigma_pairs takes the noise sigma without another pass over the patterns.
-constexpr int kPairTy = 8;  // threadIdx.y extent of k_nlpar_pairs (blockDim = 32 x 8)
-
 __device__ __forceinline__ int fwd_count(int sr) { return sr * (2 * sr + 1) + sr; }
 __device__ __forceinline__ void fwd_offset(int f, int sr, int& dy, int& dx) {
     if (f < sr) {
@@ -543,99 +599,163 @@ __device__ __forceinline__ int fwd_index(int dy, int dx, int sr) {
     return dy == 0 ? dx - 1 : sr + (dy - 1) * (2 * sr + 1) + (dx + sr);
 }
 
-template <int MPF, bool kSig>
-__global__ void __launch_bounds__(kTileX * kPairTy) k_nlpar_pairs(
+// Register-blocked: a block takes 2 * kPairLanes neighbouring scan pixels of one row; warp dy sums
+// the offsets into row y + dy, each lane two neighbouring pixels x, x + 1 against every dx -- the
+// 2 SR + 2 values of row y + dy under both windows are loaded once as pairs and feed 2 SR + 1 packed
+// (two-pixel) differences, squares and sums, each rounded as its own.  The patterns' next kChunk
+// pixels stream into a second buffer (cp.async) while the current ones are summed, stored with the scan
+// columns along the fast axis.  A chunk with no value at or above a saturation level (nor a NaN) is
+// summed without the per-term tests and counted whole.  Measured, 128x160 scan of 80x80, radius 3: 1.35
+// ms with one pair per thread and step (11 instructions a term, staging exposed).
+constexpr int kPairThreads = 256;              // the warps past SR only stage and check
+constexpr int kPairLanes = 30;                 // 60 pixels and 2 SR halo columns
+constexpr int kPairPitch = 66;                 // staged columns (2 modulo 32: a column's 32 pixels in 16 banks)
+
+__device__ __forceinline__ void stage4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+template <int SR, bool kSig>
+__global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind,
-        int nind, float mxval, float mxsig, int sr, float2* __restrict__ pairs, float2* __restrict__ sigp) {
-    extern __shared__ float sm[];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int y = blockIdx.y, x0 = blockIdx.x * kTileX;
-    const int nF = fwd_count(sr);
-    const int nr = (y + sr < nrows ? y + sr : nrows - 1) - y + 1;  // staged scan rows y .. y + nr - 1
-    const int cx0 = x0 - sr > 0 ? x0 - sr : 0;
-    const int cx1 = x0 + kTileX + sr < ncols ? x0 + kTileX + sr : ncols;
-    const int ncx = cx1 - cx0;
-    float* S = sm;  // [nr][ncx][kSP]
-    const int x = x0 + tx;
-    const bool px_ok = x < ncols;
-    const int self = (px_ok ? x : ncols - 1) - cx0;
-    int slot[MPF];
-    bool ok[MPF];
+        int nind, float mxval, float mxsig, float zero, float2* __restrict__ pairs, float2* __restrict__ sigp) {
+    extern __shared__ __align__(16) float sm[];
+    constexpr int WN = 2 * SR + 1, kRowF = kChunk * kPairPitch, kBufF = (SR + 1) * kRowF, nF = SR * WN + SR;
+    const int lane = threadIdx.x & 31, dy = threadIdx.x >> 5;
+    const int y = blockIdx.y, x0 = blockIdx.x * 2 * kPairLanes;
+    const int nr = min(SR + 1, nrows - y);                        // rows y .. y + nr - 1 exist
+    const int c_lo = max(SR - x0, 0), c_hi = min(kPairPitch, ncols - x0 + SR);  // staged columns that exist
+    const float lim = kSig ? fminf(mxval, mxsig) : mxval;
+    const Pair2 m1 = p2_pack(-1.0f, -1.0f), z = p2_pack(zero, zero);
+    for (int i = threadIdx.x; i < 2 * kBufF; i += kPairThreads) sm[i] = 0.0f;  // columns and rows off the scan stay zero
+    __syncthreads();
+    auto stage = [&](int q0, float* buf) {
+        const int q = q0 + lane;
+        if (q < nind) {
+            const float* src = data + ((int64_t)y * ncols + x0 - SR) * npx + __ldg(ind + q);
+            float* dst = buf + lane * kPairPitch;
+            const int64_t step = (int64_t)(kPairThreads / 32) * npx;
+            for (int r = 0; r < nr; ++r) {
+                const float* p = src + ((int64_t)r * ncols + c_lo + dy) * npx;
+                float* t = dst + r * kRowF;
+#pragma unroll 4
+                for (int c = c_lo + dy; c < c_hi; c += kPairThreads / 32, p += step) stage4(t + c, p);
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const bool mine = lane < kPairLanes && dy < nr;
+    const int cl = mine ? 2 * lane : 0;                           // first staged column under pixel x = x0 + 2 lane
+    Pair2 d[WN], ds[3];
+    float n0 = 0.0f;                                              // terms of the chunks counted whole
+    float na[WN], nb[WN], nsa[3], nsb[3];
 #pragma unroll
-    for (int j = 0; j < MPF; ++j) {
-        const int f = ty + kPairTy * j;
-        int dy = 0, dx = 0;
-        if (f < nF) fwd_offset(f, sr, dy, dx);
-        ok[j] = px_ok && f < nF && x + dx >= 0 && x + dx < ncols && y + dy < nrows;
-        slot[j] = ok[j] ? dy * ncx + (x + dx - cx0) : self;
-    }
-    // sigma's four forward 3x3 neighbours sit at f = 0, 2 sr - 1, 2 sr, 2 sr + 1 (warp-uniform ty)
-    const int sk = ty == 0 ? 0 : (ty == 2 * sr - 1 ? 1 : (ty == 2 * sr ? 2 : (ty == 2 * sr + 1 ? 3 : -1)));
-    const bool near = kSig && sk >= 0 && ok[0];
-    float d[MPF], n[MPF], ds = 0.0f, ns = 0.0f;
+    for (int e = 0; e < WN; ++e) d[e] = 0ull, na[e] = 0.0f, nb[e] = 0.0f;
 #pragma unroll
-    for (int j = 0; j < MPF; ++j) {
-        d[j] = 0.0f;
-        n[j] = 0.0f;
-    }
-    for (int q0 = 0; q0 < nind; q0 += kChunk) {
-        const int qn = nind - q0 < kChunk ? nind - q0 : kChunk;
-        const int k = tx < qn ? __ldg(ind + q0 + tx) : 0;
-        __syncthreads();  // the previous chunk has been consumed
-        int bad = 0, bad_sig = 0;  // a staged value at or above a saturation level
+    for (int e = 0; e < 3; ++e) ds[e] = 0ull, nsa[e] = 0.0f, nsb[e] = 0.0f;
+    // sigma's forward neighbours: dx 1 in the same row; dx -1, 0, 1 in the next
+    const bool near1 = kSig && dy == 1, near0 = kSig && dy == 0;
+    auto terms = [&](const float* q, int dyv, auto tag) {  // one pattern pixel, every term counted
+        constexpr int kKind = decltype(tag)::value;        // 0: the same row (dx > 0), 1: the next, 2: others
+        const float* pa = q + cl + SR;
+        const Pair2 a = (SR & 1) ? p2_pack(pa[0], pa[1]) : *(const Pair2*)pa;
+        const float* pb = q + dyv * kRowF + cl;
+        Pair2 v[SR + 1];
+#pragma unroll
+        for (int k = 0; k <= SR; ++k)
+            if (kKind != 0 || 2 * k + 1 > SR) v[k] = *(const Pair2*)(pb + 2 * k);
+#pragma unroll
+        for (int e = kKind == 0 ? SR + 1 : 0; e < WN; ++e) {
+            const Pair2 b = (e & 1) ? p2_pack(p2_unpack(v[e / 2]).y, p2_unpack(v[e / 2 + 1]).x) : v[e / 2];
+            const Pair2 t = p2_sub(a, b, m1);
+            const Pair2 tt = p2_mul(t, t, z);
+            d[e] = p2_add(d[e], tt);
+            if (kSig && kKind == 0 && e == SR + 1) ds[0] = p2_add(ds[0], tt);
+            if (kSig && kKind == 1 && e >= SR - 1 && e <= SR + 1) ds[e - SR + 1] = p2_add(ds[e - SR + 1], tt);
+        }
+    };
+    stage(0, sm);
+    for (int q0 = 0, it = 0; q0 < nind; q0 += kChunk, ++it) {
+        float* cur = sm + (it & 1) * kBufF;
+        const int qn = min(kChunk, nind - q0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();  // this chunk has arrived, the other buffer has been consumed
+        if (q0 + kChunk < nind) stage(q0 + kChunk, sm + ((it + 1) & 1) * kBufF);
+        bool bad = false;  // a value at or above a saturation level, or a NaN
         for (int r = 0; r < nr; ++r) {
-            const float* prow = data + ((int64_t)(y + r) * ncols + cx0) * npx + k;
-            float* srow = S + r * ncx * kSP + tx;
-            for (int cc = ty; cc < ncx; cc += kPairTy) {
-                const float v = tx < qn ? __ldg(prow + (int64_t)cc * npx) : 0.0f;
-                bad |= !(v < mxval);
-                if (kSig) bad_sig |= !(v < mxsig);
-                srow[cc * kSP] = v;
+            const float2* row = (const float2*)(cur + r * kRowF);
+#pragma unroll 4
+            for (int i = threadIdx.x; i < qn * (kPairPitch / 2); i += kPairThreads) {
+                const float2 v = row[i];
+                bad |= !(v.x < lim) | !(v.y < lim);
             }
         }
-        const int any_bad = __syncthreads_or(bad);
-        const int any_bad_sig = kSig ? __syncthreads_or(bad_sig) : 0;
-        if (any_bad == 0 && any_bad_sig == 0) {
-            // every term of the chunk counts: the squares added without the tests, the chunk
-            // counted whole (the counts are exact integers either way)
-            for (int qq = 0; qq < qn; ++qq) {
-                const float xv = S[self * kSP + qq];
+        if (__syncthreads_or(bad)) {
+            if (mine) {
+                for (int qq = 0; qq < qn; ++qq) {
+                    const float* q = cur + qq * kPairPitch;
+                    const float xa = q[cl + SR], xb = q[cl + SR + 1];
 #pragma unroll
-                for (int j = 0; j < MPF; ++j) {
-                    const float t = __fsub_rn(xv, S[slot[j] * kSP + qq]);
-                    const float tt = __fmul_rn(t, t);
-                    d[j] = __fadd_rn(d[j], tt);
-                    if (kSig && j == 0 && near) ds = __fadd_rn(ds, tt);
+                    for (int e = 0; e < WN; ++e) {
+                        const float ya = q[dy * kRowF + cl + e], yb = q[dy * kRowF + cl + e + 1];
+                        const float ta = __fsub_rn(xa, ya), tb = __fsub_rn(xb, yb);
+                        const float sa = __fmul_rn(ta, ta), sb = __fmul_rn(tb, tb);
+                        float2 s = p2_unpack(d[e]);  // pair_ssd's order: count, difference, square
+                        if (ya < mxval && xa < mxval) s.x = __fadd_rn(s.x, sa), na[e] += 1.0f;
+                        if (yb < mxval && xb < mxval) s.y = __fadd_rn(s.y, sb), nb[e] += 1.0f;
+                        d[e] = p2_pack(s.x, s.y);
+                        const int g = e - SR + 1;
+                        if (kSig && ((near1 && g >= 0 && g <= 2) || (near0 && g == 2))) {
+#pragma unroll
+                            for (int z = 0; z < 3; ++z) {
+                                if (z != (near0 ? 0 : g)) continue;
+                                float2 w = p2_unpack(ds[z]);
+                                if (ya < mxsig && xa < mxsig) w.x = __fadd_rn(w.x, sa), nsa[z] += 1.0f;
+                                if (yb < mxsig && xb < mxsig) w.y = __fadd_rn(w.y, sb), nsb[z] += 1.0f;
+                                ds[z] = p2_pack(w.x, w.y);
+                            }
+                        }
+                    }
                 }
             }
-#pragma unroll
-            for (int j = 0; j < MPF; ++j) n[j] = __fadd_rn(n[j], (float)qn);
-            if (kSig && near) ns = __fadd_rn(ns, (float)qn);
-            continue;
+        } else if (mine) {
+            // every term of the chunk counts (the counts are exact integers either way)
+            if (dy == 0) {
+#pragma unroll 4
+                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 0, std::integral_constant<int, 0>());
+            } else if (dy == 1) {
+#pragma unroll 4
+                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 1, std::integral_constant<int, 1>());
+            } else {
+#pragma unroll 4
+                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, dy, std::integral_constant<int, 2>());
+            }
+            n0 += (float)qn;
         }
-        for (int qq = 0; qq < qn; ++qq) {
-            const float xv = S[self * kSP + qq];
+    }
+    if (!mine) return;
+    const int x = x0 + 2 * lane;
 #pragma unroll
-            for (int j = 0; j < MPF; ++j) {
-                const float yv = S[slot[j] * kSP + qq];
-                if (yv < mxval && xv < mxval) {  // pair_ssd's order: count, difference, square
-                    n[j] = __fadd_rn(n[j], 1.0f);
-                    const float t = __fsub_rn(xv, yv);
-                    d[j] = __fadd_rn(d[j], __fmul_rn(t, t));
-                }
-                if (kSig && j == 0 && near && yv < mxsig && xv < mxsig) {
-                    ns = __fadd_rn(ns, 1.0f);
-                    const float t = __fsub_rn(xv, yv);
-                    ds = __fadd_rn(ds, __fmul_rn(t, t));
+    for (int h = 0; h < 2; ++h) {
+        if (x + h >= ncols) continue;
+        const int64_t pix = (int64_t)y * ncols + x + h;
+#pragma unroll
+        for (int e = 0; e < WN; ++e) {
+            const int dx = e - SR;
+            if ((dy == 0 && dx <= 0) || x + h + dx < 0 || x + h + dx >= ncols) continue;
+            const float2 s = p2_unpack(d[e]);
+            pairs[pix * nF + (dy == 0 ? dx - 1 : SR + (dy - 1) * WN + e)] = make_float2(h ? s.y : s.x, n0 + (h ? nb[e] : na[e]));
+            const int g = dx + 1;
+            if (kSig && ((near1 && g >= 0 && g <= 2) || (near0 && g == 2))) {
+#pragma unroll
+                for (int z = 0; z < 3; ++z) {
+                    if (z != (near0 ? 0 : g)) continue;
+                    const float2 w = p2_unpack(ds[z]);
+                    sigp[pix * 4 + (near0 ? 0 : 1 + g)] = make_float2(h ? w.y : w.x, n0 + (h ? nsb[z] : nsa[z]));
                 }
             }
         }
     }
-    const int64_t pix = (int64_t)y * ncols + x;
-#pragma unroll
-    for (int j = 0; j < MPF; ++j)
-        if (ok[j]) pairs[pix * nF + ty + kPairTy * j] = make_float2(d[j], n[j]);
-    if (near) sigp[pix * 4 + sk] = make_float2(ds, ns);
 }
 
 // sigma_numba (nn = 1) from the pair sums: min over the clipped 3x3 neighbourhood of
@@ -739,102 +859,80 @@ __device__ __forceinline__ int64_t edge_index(int y, int x, int sr, int nrows, i
     return (int64_t)2 * sr * ncols + (int64_t)(y - sr) * 2 * sr + (x < sr ? x : sr + x - (ncols - sr));
 }
 
-// Edge rows: blockIdx.y picks the row (the sr top rows, then the sr bottom rows), blockIdx.x 32
-// neighbouring pixels (one per lane), blockIdx.z a range of kTy window slots (one per thread row).
-// All pixels of the row share the window rows; the patterns of those rows in the columns the
-// block's windows touch are staged.
-__global__ void __launch_bounds__(kTileX * kTy) k_nlpar_edge_rows(
-        const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind, int nind,
-        float mxval, int sr, float2* __restrict__ raw) {
-    extern __shared__ float sm[];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int wn = 2 * sr + 1, winsz = wn * wn;
-    const int y = blockIdx.y < sr ? blockIdx.y : nrows - 2 * sr + blockIdx.y;
-    const int x0 = blockIdx.x * kTileX;
-    int ys, ye;
-    window(y, sr, nrows, ys, ye);
-    const int cx0 = x0 - 2 * sr > 0 ? x0 - 2 * sr : 0;
-    const int cx1 = x0 + kTileX + 2 * sr < ncols ? x0 + kTileX + 2 * sr : ncols;
-    const int ncx = cx1 - cx0;
-    float* S = sm;  // [wn][ncx][kSP]
-    const int x = x0 + tx;
-    const int c = blockIdx.z * kTy + ty;
-    const bool ok = x < ncols && c < winsz;
-    int xs, xe;
-    window(x < ncols ? x : ncols - 1, sr, ncols, xs, xe);
-    const int self = (y - ys) * ncx + ((x < ncols ? x : ncols - 1) - cx0);
-    const int nbs = ok ? (c / wn) * ncx + (xs + c % wn - cx0) : self;
-    float d = 0.0f, n = 0.0f;
-    for (int q0 = 0; q0 < nind; q0 += kChunk) {
-        const int qn = nind - q0 < kChunk ? nind - q0 : kChunk;
-        const int k = tx < qn ? __ldg(ind + q0 + tx) : 0;
-        __syncthreads();
-        for (int r = 0; r < wn; ++r) {
-            const float* prow = data + ((int64_t)(ys + r) * ncols + cx0) * npx + k;
-            float* srow = S + r * ncx * kSP + tx;
-            for (int cc = ty; cc < ncx; cc += kTy) srow[cc * kSP] = tx < qn ? __ldg(prow + (int64_t)cc * npx) : 0.0f;
+// The slots of an edge pixel's window that lie beyond +-sr (the pair sums hold the others).  A block
+// takes two lines of the scan -- an edge line and a partner line more than sr away -- and 32 positions
+// along them, one per lane; warp s sums window slot s along the line.  First the row pairs (edge row y,
+// row y2 of its window; positions are columns, every column's window along x), then the column pairs
+// (edge column x, column x2 of its window; positions are rows, and only slots within +-sr rows: the
+// row pairs have the others).  Pixels stream through two buffers as in k_nlpar_pairs.
+constexpr int kEdgePitch = kChunk + 1;
+
+__global__ void k_nlpar_edge(const float* __restrict__ data, int nrows, int ncols, int npx,
+                             const int32_t* __restrict__ ind, int nind, float mxval, int sr, int row_blocks,
+                             float2* __restrict__ raw) {
+    extern __shared__ __align__(16) float sm[];
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5, wn = 2 * sr + 1, winsz = wn * wn;
+    const bool cols = (int)blockIdx.x >= row_blocks;
+    const int b = cols ? blockIdx.x - row_blocks : blockIdx.x;
+    const int nalong = cols ? nrows : ncols, nacross = cols ? ncols : nrows;
+    const int nblk = (nalong + 31) / 32, line = b / nblk, p0 = (b - line * nblk) * 32;
+    // line pair: side, then (edge line k = 0 .. sr - 1, one of its sr - k partners)
+    const int per = sr * (sr + 1) / 2, side = line / per;
+    int k = 0, t = line - side * per;
+    while (t >= sr - k) t -= sr - k++;
+    const int l1 = side ? nacross - 1 - k : k, l2 = side ? nacross - 1 - (k + sr + 1 + t) : k + sr + 1 + t;
+    // staged: 32 positions of the edge line, then the partner's positions under their windows
+    const int a0 = max(p0 - 2 * sr, 0), a1 = min(p0 + 32 + 2 * sr, nalong);
+    const int n1 = min(32, nalong - p0), nst = n1 + a1 - a0;
+    const int bufn = (32 + 32 + 4 * sr) * kEdgePitch;
+    auto pattern = [&](int along, int across) { return data + ((int64_t)(cols ? along : across) * ncols + (cols ? across : along)) * npx; };
+    auto stage = [&](int q0, float* buf) {
+        const int q = q0 + lane;
+        if (q < nind) {
+            const int px = __ldg(ind + q);
+            for (int i = s; i < nst; i += wn)
+                stage4(buf + i * kEdgePitch + lane, (i < n1 ? pattern(p0 + i, l1) : pattern(a0 + i - n1, l2)) + px);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int p = p0 + lane;
+    int ws, we;
+    window(p < nalong ? p : nalong - 1, sr, nalong, ws, we);
+    const int p2 = ws + s;  // the slot's position along the partner line
+    const bool ok = p < nalong && (!cols || (p2 - p <= sr && p - p2 <= sr));
+    const int self = ok ? lane * kEdgePitch : 0, other = ok ? (n1 + p2 - a0) * kEdgePitch : 0;
+    float d = 0.0f, n = 0.0f;
+    stage(0, sm);
+    for (int q0 = 0, it = 0; q0 < nind; q0 += kChunk, ++it) {
+        const float* cur = sm + (it & 1) * bufn;
+        const int qn = min(kChunk, nind - q0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
         __syncthreads();
+        if (q0 + kChunk < nind) stage(q0 + kChunk, sm + ((it + 1) & 1) * bufn);
+#pragma unroll 8
         for (int qq = 0; qq < qn; ++qq) {
-            const float xv = S[self * kSP + qq], yv = S[nbs * kSP + qq];
+            const float xv = cur[self + qq], yv = cur[other + qq];
+            const float u = __fsub_rn(xv, yv), uu = __fmul_rn(u, u);
             if (yv < mxval && xv < mxval) {  // pair_ssd's order: count, difference, square
                 n = __fadd_rn(n, 1.0f);
-                const float t = __fsub_rn(xv, yv);
-                d = __fadd_rn(d, __fmul_rn(t, t));
+                d = __fadd_rn(d, uu);
             }
         }
     }
-    if (ok) raw[edge_index(y, x, sr, nrows, ncols) * winsz + c] = make_float2(d, n);
+    if (!ok) return;
+    const int y = cols ? p : l1, x = cols ? l1 : p, y2 = cols ? p2 : l2, x2 = cols ? l2 : p2;
+    int ys, ye, xs, xe;
+    window(y, sr, nrows, ys, ye);
+    window(x, sr, ncols, xs, xe);
+    raw[edge_index(y, x, sr, nrows, ncols) * winsz + (y2 - ys) * wn + (x2 - xs)] = make_float2(d, n);
 }
 
-// Edge columns of the middle rows: blockIdx.y the side, blockIdx.x 32 neighbouring rows (one per
-// lane), blockIdx.z a range of kTy (edge column, window slot) combinations.  All edge pixels of
-// one side share the window columns [0, 2 sr] (or the last 2 sr + 1).
-__global__ void __launch_bounds__(kTileX * kTy) k_nlpar_edge_cols(
-        const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind, int nind,
-        float mxval, int sr, float2* __restrict__ raw) {
-    extern __shared__ float sm[];
-    const int tx = threadIdx.x, ty = threadIdx.y;
-    const int wn = 2 * sr + 1, winsz = wn * wn;
-    const int nri = nrows - 2 * sr;
-    const int y0 = sr + blockIdx.x * kTileX;
-    const int nrow = nri - blockIdx.x * kTileX < kTileX ? nri - blockIdx.x * kTileX : kTileX;
-    const int side = blockIdx.y;
-    const int colbase = side ? ncols - wn : 0;
-    const int xe0 = side ? ncols - sr : 0;
-    const int nrs = nrow + 2 * sr;
-    float* S = sm;  // [nrs][wn][kSP]
-    const int idx = blockIdx.z * kTy + ty;
-    const bool ok = tx < nrow && idx < sr * winsz;
-    const int e = ok ? idx / winsz : 0, c = ok ? idx - e * winsz : 0;
-    const int self = ((ok ? tx : 0) + sr) * wn + (xe0 + e - colbase);
-    const int nbs = ok ? (tx + c / wn) * wn + c % wn : self;
-    float d = 0.0f, n = 0.0f;
-    for (int q0 = 0; q0 < nind; q0 += kChunk) {
-        const int qn = nind - q0 < kChunk ? nind - q0 : kChunk;
-        const int k = tx < qn ? __ldg(ind + q0 + tx) : 0;
-        __syncthreads();
-        for (int r = ty; r < nrs; r += kTy) {
-            const float* prow = data + ((int64_t)(y0 - sr + r) * ncols + colbase) * npx + k;
-            float* srow = S + r * wn * kSP + tx;
-            for (int cc = 0; cc < wn; ++cc) srow[cc * kSP] = tx < qn ? __ldg(prow + (int64_t)cc * npx) : 0.0f;
-        }
-        __syncthreads();
-        for (int qq = 0; qq < qn; ++qq) {
-            const float xv = S[self * kSP + qq], yv = S[nbs * kSP + qq];
-            if (yv < mxval && xv < mxval) {  // pair_ssd's order: count, difference, square
-                n = __fadd_rn(n, 1.0f);
-                const float t = __fsub_rn(xv, yv);
-                d = __fadd_rn(d, __fmul_rn(t, t));
-            }
-        }
-    }
-    if (ok) raw[edge_index(y0 + tx, xe0 + e, sr, nrows, ncols) * winsz + c] = make_float2(d, n);
-}
+int edge_blocks(int sr, int nalong) { return sr * (sr + 1) * ((nalong + 31) / 32); }
+size_t edge_smem(int sr) { return (size_t)2 * (64 + 4 * sr) * kEdgePitch * sizeof(float); }
 
 // Normalised window weights of the edge pixels from their raw sums: one block (64 threads) per
 // edge pixel, the arithmetic of k_nlpar_weights_tiled.
-__global__ void k_nlpar_weights_edge(const float2* __restrict__ raw, int nrows, int ncols, int sr,
+__global__ void k_nlpar_weights_edge(const float2* __restrict__ raw, const float2* __restrict__ pairs, int nrows, int ncols, int sr,
                                      const float* __restrict__ sigma, float lam2, float dthresh,
                                      float* __restrict__ wout, const float* __restrict__ coff) {
     __shared__ float W[64];
@@ -865,7 +963,10 @@ __global__ void k_nlpar_weights_edge(const float2* __restrict__ raw, int nrows, 
         if (nb == pix) {
             w = -1.0e6f;
         } else {
-            const float2 e2 = raw[b * winsz + c];
+            const int dy = ys + c / wn - y, dx = xs + c % wn - x, nF = fwd_count(sr);
+            const float2 e2 = dy < -sr || dy > sr || dx < -sr || dx > sr ? raw[b * winsz + c]
+                              : (dy > 0 || (dy == 0 && dx > 0)) ? pairs[pix * nF + fwd_index(dy, dx, sr)]
+                                                               : pairs[nb * nF + fwd_index(-dy, -dx, sr)];
             float s0 = sigma[pix], s1 = sigma[nb];
             s0 = __fmul_rn(s0, s0);
             s1 = __fmul_rn(s1, s1);
@@ -889,16 +990,7 @@ __global__ void k_nlpar_weights_edge(const float2* __restrict__ raw, int nrows, 
     if (c < winsz) wout[pix * winsz + c] = __fdiv_rn(W[c], T);
 }
 
-size_t edge_rows_smem(int sr, int ncols) {
-    const int ncx = std::min(ncols, kTileX + 4 * sr);
-    return (size_t)(2 * sr + 1) * ncx * kSP * sizeof(float);
-}
-size_t edge_cols_smem(int sr) { return (size_t)(kTileX + 2 * sr) * (2 * sr + 1) * kSP * sizeof(float); }
-
-size_t pairs_smem(int sr, int ncols) {
-    const int ncx = std::min(ncols, kTileX + 2 * sr);
-    return (size_t)(sr + 1) * ncx * kSP * sizeof(float);
-}
+size_t pairs_smem(int sr) { return (size_t)2 * (sr + 1) * kChunk * kPairPitch * sizeof(float); }
 
 size_t tiled_smem(int sr, int ncols, size_t elem, bool weights) {
     const int wn = 2 * sr + 1;
@@ -1166,9 +1258,8 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
         nind < 0 || nind > npx || sr < 1 || sr > 3 || !(lam > 0.0f))
         return EBSD_E_ARG;
     if (2 * sr + 1 > nrows || 2 * sr + 1 > ncols) return EBSD_E_ARG;  // window must fit the scan
-    const size_t psm = pairs_smem(sr, ncols), asm_ = tiled_smem(sr, ncols, sizeof(float), false);
-    if (psm > 48 * 1024 || asm_ > 48 * 1024 || edge_rows_smem(sr, ncols) > 48 * 1024 || edge_cols_smem(sr) > 48 * 1024)
-        return EBSD_E_UNSUPPORTED;
+    const size_t psm = pairs_smem(sr), asm_ = tiled_smem(sr, ncols, sizeof(float), false);
+    if (asm_ > 48 * 1024) return EBSD_E_UNSUPPORTED;
     const float mxval = saturation_protect ? datamax * 0.999f : datamax + 1.0f;
     const float mxsig = saturation_protect ? datamax * 0.9961f : datamax + 1.0f;
     const float lam2 = 1.0f / (lam * lam);
@@ -1181,21 +1272,12 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
     float2* pairs = (float2*)(d_work + ((npix * winsz + 1) & ~(int64_t)1));
     float2* sigp = pairs + npix * nF;
     cudaStream_t st = (cudaStream_t)stream;
-    const dim3 pgrid((unsigned)((ncols + kTileX - 1) / kTileX), (unsigned)nrows), pblock(kTileX, kPairTy);
-    const int mpf = (nF + kPairTy - 1) / kPairTy;
-#define EBSD_PAIRS(M, SG)                                                                                     \
-    k_nlpar_pairs<M, SG><<<pgrid, pblock, psm, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, mxsig, sr, \
-                                                     pairs, sigp)
-    if (compute_sigma) {
-        if (mpf == 1) EBSD_PAIRS(1, true);
-        else if (mpf == 2) EBSD_PAIRS(2, true);
-        else EBSD_PAIRS(3, true);
-    } else {
-        if (mpf == 1) EBSD_PAIRS(1, false);
-        else if (mpf == 2) EBSD_PAIRS(2, false);
-        else EBSD_PAIRS(3, false);
-    }
-#undef EBSD_PAIRS
+    const dim3 pgrid((unsigned)((ncols + 2 * kPairLanes - 1) / (2 * kPairLanes)), (unsigned)nrows);
+    typedef void (*PairsFn)(const float*, int, int, int, const int32_t*, int, float, float, float, float2*, float2*);
+    PairsFn fn = compute_sigma ? (sr == 1 ? k_nlpar_pairs<1, true> : sr == 2 ? k_nlpar_pairs<2, true> : k_nlpar_pairs<3, true>)
+                               : (sr == 1 ? k_nlpar_pairs<1, false> : sr == 2 ? k_nlpar_pairs<2, false> : k_nlpar_pairs<3, false>);
+    EBSD_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+    fn<<<pgrid, (unsigned)kPairThreads, psm, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, mxsig, 0.0f, pairs, sigp);
     int rc = launch_status();
     if (rc != EBSD_OK) return rc;
     if (compute_sigma) {
@@ -1207,20 +1289,14 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
                                                        d_sigma, lam2, dthresh, sr, w, d_centre_offset);
     if ((rc = launch_status()) != EBSD_OK) return rc;
     {
-        // edge pixels: raw window sums (rows, then the middle rows' columns), then their weights
+        // edge pixels: the window sums that are no pair sums, then their weights
         float2* raw = sigp + npix * 4;
-        const int nri = nrows - 2 * sr;
-        const unsigned zr = (unsigned)((winsz + kTy - 1) / kTy), zc = (unsigned)((sr * winsz + kTy - 1) / kTy);
-        k_nlpar_edge_rows<<<dim3((unsigned)((ncols + kTileX - 1) / kTileX), (unsigned)(2 * sr), zr), tblock,
-                            edge_rows_smem(sr, ncols), st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, sr, raw);
+        const int nri = nrows - 2 * sr, rb = edge_blocks(sr, ncols);
+        k_nlpar_edge<<<(unsigned)(rb + edge_blocks(sr, nrows)), (unsigned)((2 * sr + 1) * 32), edge_smem(sr), st>>>(
+            d_data, nrows, ncols, npx, d_indices, nind, mxval, sr, rb, raw);
         if ((rc = launch_status()) != EBSD_OK) return rc;
-        if (nri > 0) {
-            k_nlpar_edge_cols<<<dim3((unsigned)((nri + kTileX - 1) / kTileX), 2u, zc), tblock, edge_cols_smem(sr), st>>>(
-                d_data, nrows, ncols, npx, d_indices, nind, mxval, sr, raw);
-            if ((rc = launch_status()) != EBSD_OK) return rc;
-        }
         const int64_t nedge = (int64_t)2 * sr * ncols + (int64_t)nri * 2 * sr;
-        k_nlpar_weights_edge<<<(unsigned)nedge, 64, 0, st>>>(raw, nrows, ncols, sr, d_sigma, lam2, dthresh, w,
+        k_nlpar_weights_edge<<<(unsigned)nedge, 64, 0, st>>>(raw, pairs, nrows, ncols, sr, d_sigma, lam2, dthresh, w,
                                                              d_centre_offset);
         if ((rc = launch_status()) != EBSD_OK) return rc;
     }
