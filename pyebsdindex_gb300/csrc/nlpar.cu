@@ -599,6 +599,92 @@ __device__ __forceinline__ int fwd_index(int dy, int dx, int sr) {
     return dy == 0 ? dx - 1 : sr + (dy - 1) * (2 * sr + 1) + (dx + sr);
 }
 
+constexpr int kPairThreads = 256;
+__device__ __forceinline__ void stage4(float* dst, const float* src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+
+// ---- edge pixels: windows shifted inward, reaching past +-sr ----------------------------------
+// Edge pixels are those of the sr top and bottom rows, and the sr left and right columns of the
+// other rows; index: top rows, bottom rows, then per middle row its 2 sr edge columns.  Their
+// raw window sums (SSD, count per slot, in the reference's pixel order) come from the pair sums and
+// from edge_sums, and k_nlpar_weights_edge turns them into normalised weights, one block per edge
+// pixel.
+__device__ __forceinline__ int64_t edge_index(int y, int x, int sr, int nrows, int ncols) {
+    if (y < sr) return (int64_t)y * ncols + x;
+    if (y >= nrows - sr) return (int64_t)(sr + y - (nrows - sr)) * ncols + x;
+    return (int64_t)2 * sr * ncols + (int64_t)(y - sr) * 2 * sr + (x < sr ? x : sr + x - (ncols - sr));
+}
+
+// The slots of an edge pixel's window that lie beyond +-sr (the pair sums hold the others).  A block
+// takes two lines of the scan -- an edge line and a partner line more than sr away -- and 32 positions
+// along them, one per lane; warp s sums window slot s along the line.  First the row pairs (edge row y,
+// row y2 of its window; positions are columns, every column's window along x), then the column pairs
+// (edge column x, column x2 of its window; positions are rows, and only slots within +-sr rows: the
+// row pairs have the others).  Pixels stream through two buffers as in k_nlpar_pairs.
+constexpr int kEdgePitch = kChunk + 1;
+
+// Part of the pair kernel's launch: these blocks are few and long, and run beside the others.
+__device__ void edge_sums(float* sm, int block, const float* __restrict__ data, int nrows, int ncols, int npx,
+                          const int32_t* __restrict__ ind, int nind, float mxval, int sr, int row_blocks,
+                          float2* __restrict__ raw) {
+    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5, wn = 2 * sr + 1, winsz = wn * wn, nw = blockDim.x >> 5;
+    const bool cols = block >= row_blocks;
+    const int b = cols ? block - row_blocks : block;
+    const int nalong = cols ? nrows : ncols, nacross = cols ? ncols : nrows;
+    const int nblk = (nalong + 31) / 32, line = b / nblk, p0 = (b - line * nblk) * 32;
+    // line pair: side, then (edge line k = 0 .. sr - 1, one of its sr - k partners)
+    const int per = sr * (sr + 1) / 2, side = line / per;
+    int k = 0, t = line - side * per;
+    while (t >= sr - k) t -= sr - k++;
+    const int l1 = side ? nacross - 1 - k : k, l2 = side ? nacross - 1 - (k + sr + 1 + t) : k + sr + 1 + t;
+    // staged: 32 positions of the edge line, then the partner's positions under their windows
+    const int a0 = max(p0 - 2 * sr, 0), a1 = min(p0 + 32 + 2 * sr, nalong);
+    const int n1 = min(32, nalong - p0), nst = n1 + a1 - a0;
+    const int bufn = (32 + 32 + 4 * sr) * kEdgePitch;
+    auto pattern = [&](int along, int across) { return data + ((int64_t)(cols ? along : across) * ncols + (cols ? across : along)) * npx; };
+    auto stage = [&](int q0, float* buf) {
+        const int q = q0 + lane;
+        if (q < nind) {
+            const int px = __ldg(ind + q);
+            for (int i = s; i < nst; i += nw)
+                stage4(buf + i * kEdgePitch + lane, (i < n1 ? pattern(p0 + i, l1) : pattern(a0 + i - n1, l2)) + px);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    const int p = p0 + lane;
+    int ws, we;
+    window(p < nalong ? p : nalong - 1, sr, nalong, ws, we);
+    const int p2 = ws + (s < wn ? s : 0);  // the slot's position along the partner line
+    const bool ok = s < wn && p < nalong && (!cols || (p2 - p <= sr && p - p2 <= sr));
+    const int self = ok ? lane * kEdgePitch : 0, other = ok ? (n1 + p2 - a0) * kEdgePitch : 0;
+    float d = 0.0f, n = 0.0f;
+    stage(0, sm);
+    for (int q0 = 0, it = 0; q0 < nind; q0 += kChunk, ++it) {
+        const float* cur = sm + (it & 1) * bufn;
+        const int qn = min(kChunk, nind - q0);
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        if (q0 + kChunk < nind) stage(q0 + kChunk, sm + ((it + 1) & 1) * bufn);
+        if (s >= wn) continue;
+#pragma unroll 8
+        for (int qq = 0; qq < qn; ++qq) {
+            const float xv = cur[self + qq], yv = cur[other + qq];
+            const float u = __fsub_rn(xv, yv), uu = __fmul_rn(u, u);
+            if (yv < mxval && xv < mxval) {  // pair_ssd's order: count, difference, square
+                n = __fadd_rn(n, 1.0f);
+                d = __fadd_rn(d, uu);
+            }
+        }
+    }
+    if (!ok) return;
+    const int y = cols ? p : l1, x = cols ? l1 : p, y2 = cols ? p2 : l2, x2 = cols ? l2 : p2;
+    int ys, ye, xs, xe;
+    window(y, sr, nrows, ys, ye);
+    window(x, sr, ncols, xs, xe);
+    raw[edge_index(y, x, sr, nrows, ncols) * winsz + (y2 - ys) * wn + (x2 - xs)] = make_float2(d, n);
+}
+
 // Register-blocked: a block takes 2 * kPairLanes neighbouring scan pixels of one row; warp dy sums
 // the offsets into row y + dy, each lane two neighbouring pixels x, x + 1 against every dx -- the
 // 2 SR + 2 values of row y + dy under both windows are loaded once as pairs and feed 2 SR + 1 packed
@@ -607,44 +693,62 @@ __device__ __forceinline__ int fwd_index(int dy, int dx, int sr) {
 // columns along the fast axis.  A chunk with no value at or above a saturation level (nor a NaN) is
 // summed without the per-term tests and counted whole.  Measured, 128x160 scan of 80x80, radius 3: 1.35
 // ms with one pair per thread and step (11 instructions a term, staging exposed).
-constexpr int kPairThreads = 256;              // the warps past SR only stage and check
 constexpr int kPairLanes = 30;                 // 60 pixels and 2 SR halo columns
 constexpr int kPairPitch = 66;                 // staged columns (2 modulo 32: a column's 32 pixels in 16 banks)
-
-__device__ __forceinline__ void stage4(float* dst, const float* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
-}
 
 template <int SR, bool kSig>
 __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind,
-        int nind, float mxval, float mxsig, float zero, float2* __restrict__ pairs, float2* __restrict__ sigp) {
+        int nind, float mxval, float mxsig, float zero, float2* __restrict__ pairs, float2* __restrict__ sigp,
+        int edge_rows, int edge_all, float2* __restrict__ raw) {
     extern __shared__ __align__(16) float sm[];
     constexpr int WN = 2 * SR + 1, kRowF = kChunk * kPairPitch, kBufF = (SR + 1) * kRowF, nF = SR * WN + SR;
     const int lane = threadIdx.x & 31, dy = threadIdx.x >> 5;
-    const int y = blockIdx.y, x0 = blockIdx.x * 2 * kPairLanes;
+    if ((int)blockIdx.x < edge_all) {
+        edge_sums(sm, blockIdx.x, data, nrows, ncols, npx, ind, nind, mxval, SR, edge_rows, raw);
+        return;
+    }
+    __shared__ int bad_s[2];                                      // the buffers' chunks hold a saturated value or a NaN
+    const int nxb = (ncols + 2 * kPairLanes - 1) / (2 * kPairLanes);
+    const int y = ((int)blockIdx.x - edge_all) / nxb, x0 = ((int)blockIdx.x - edge_all - y * nxb) * 2 * kPairLanes;
     const int nr = min(SR + 1, nrows - y);                        // rows y .. y + nr - 1 exist
     const int c_lo = max(SR - x0, 0), c_hi = min(kPairPitch, ncols - x0 + SR);  // staged columns that exist
     const float lim = kSig ? fminf(mxval, mxsig) : mxval;
     const Pair2 m1 = p2_pack(-1.0f, -1.0f), z = p2_pack(zero, zero);
     for (int i = threadIdx.x; i < 2 * kBufF; i += kPairThreads) sm[i] = 0.0f;  // columns and rows off the scan stay zero
     __syncthreads();
-    auto stage = [&](int q0, float* buf) {
-        const int q = q0 + lane;
+    // the warps past SR stage a chunk, wait for it and look it over while the others sum the one before
+    constexpr int kHelpers = kPairThreads / 32 - SR - 1;
+    const int helper = dy - SR - 1;
+    auto stage = [&](int q0, int b) {
+        float* buf = sm + b * kBufF;
+        const int q = q0 + lane, qn = min(kChunk, nind - q0);
+        if (helper == 0 && lane == 0) bad_s[b] = 0;
         if (q < nind) {
             const float* src = data + ((int64_t)y * ncols + x0 - SR) * npx + __ldg(ind + q);
             float* dst = buf + lane * kPairPitch;
-            const int64_t step = (int64_t)(kPairThreads / 32) * npx;
+            const int64_t step = (int64_t)kHelpers * npx;
             for (int r = 0; r < nr; ++r) {
-                const float* p = src + ((int64_t)r * ncols + c_lo + dy) * npx;
+                const float* p = src + ((int64_t)r * ncols + c_lo + helper) * npx;
                 float* t = dst + r * kRowF;
 #pragma unroll 4
-                for (int c = c_lo + dy; c < c_hi; c += kPairThreads / 32, p += step) stage4(t + c, p);
+                for (int c = c_lo + helper; c < c_hi; c += kHelpers, p += step) stage4(t + c, p);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        asm volatile("cp.async.commit_group;\ncp.async.wait_all;" ::: "memory");
+        asm volatile("bar.sync 1, %0;" ::"n"(kHelpers * 32) : "memory");
+        bool bad = false;
+        for (int r = 0; r < nr; ++r) {
+            const float2* row = (const float2*)(buf + r * kRowF);
+#pragma unroll 4
+            for (int i = helper * 32 + lane; i < qn * (kPairPitch / 2); i += kHelpers * 32) {
+                const float2 v = row[i];
+                bad |= !(v.x < lim) | !(v.y < lim);
+            }
+        }
+        if (bad) bad_s[b] = 1;
     };
-    const bool mine = lane < kPairLanes && dy < nr;
+    const bool mine = lane < kPairLanes && dy < nr && helper < 0;
     const int cl = mine ? 2 * lane : 0;                           // first staged column under pixel x = x0 + 2 lane
     Pair2 d[WN], ds[3];
     float n0 = 0.0f;                                              // terms of the chunks counted whole
@@ -674,23 +778,14 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
             if (kSig && kKind == 1 && e >= SR - 1 && e <= SR + 1) ds[e - SR + 1] = p2_add(ds[e - SR + 1], tt);
         }
     };
-    stage(0, sm);
+    if (helper >= 0) stage(0, 0);
+    __syncthreads();
     for (int q0 = 0, it = 0; q0 < nind; q0 += kChunk, ++it) {
-        float* cur = sm + (it & 1) * kBufF;
+        const float* cur = sm + (it & 1) * kBufF;
         const int qn = min(kChunk, nind - q0);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();  // this chunk has arrived, the other buffer has been consumed
-        if (q0 + kChunk < nind) stage(q0 + kChunk, sm + ((it + 1) & 1) * kBufF);
-        bool bad = false;  // a value at or above a saturation level, or a NaN
-        for (int r = 0; r < nr; ++r) {
-            const float2* row = (const float2*)(cur + r * kRowF);
-#pragma unroll 4
-            for (int i = threadIdx.x; i < qn * (kPairPitch / 2); i += kPairThreads) {
-                const float2 v = row[i];
-                bad |= !(v.x < lim) | !(v.y < lim);
-            }
-        }
-        if (__syncthreads_or(bad)) {
+        if (helper >= 0) {
+            if (q0 + kChunk < nind) stage(q0 + kChunk, (it + 1) & 1);
+        } else if (bad_s[it & 1]) {
             if (mine) {
                 for (int qq = 0; qq < qn; ++qq) {
                     const float* q = cur + qq * kPairPitch;
@@ -732,6 +827,7 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
             }
             n0 += (float)qn;
         }
+        __syncthreads();  // the next chunk is in place, this one's buffer free
     }
     if (!mine) return;
     const int x = x0 + 2 * lane;
@@ -847,88 +943,7 @@ __global__ void __launch_bounds__(kTileX * kTy) k_nlpar_weights_pairs(
     }
 }
 
-// ---- edge pixels: windows shifted inward, reaching past +-sr ----------------------------------
-// Edge pixels are those of the sr top and bottom rows, and the sr left and right columns of the
-// other rows; index: top rows, bottom rows, then per middle row its 2 sr edge columns.  Their
-// raw window sums (SSD, count per slot, in the reference's pixel order) are computed by two
-// kernels that split the slots over many blocks, then k_nlpar_weights_edge turns them into
-// normalised weights, one block per edge pixel.
-__device__ __forceinline__ int64_t edge_index(int y, int x, int sr, int nrows, int ncols) {
-    if (y < sr) return (int64_t)y * ncols + x;
-    if (y >= nrows - sr) return (int64_t)(sr + y - (nrows - sr)) * ncols + x;
-    return (int64_t)2 * sr * ncols + (int64_t)(y - sr) * 2 * sr + (x < sr ? x : sr + x - (ncols - sr));
-}
-
-// The slots of an edge pixel's window that lie beyond +-sr (the pair sums hold the others).  A block
-// takes two lines of the scan -- an edge line and a partner line more than sr away -- and 32 positions
-// along them, one per lane; warp s sums window slot s along the line.  First the row pairs (edge row y,
-// row y2 of its window; positions are columns, every column's window along x), then the column pairs
-// (edge column x, column x2 of its window; positions are rows, and only slots within +-sr rows: the
-// row pairs have the others).  Pixels stream through two buffers as in k_nlpar_pairs.
-constexpr int kEdgePitch = kChunk + 1;
-
-__global__ void k_nlpar_edge(const float* __restrict__ data, int nrows, int ncols, int npx,
-                             const int32_t* __restrict__ ind, int nind, float mxval, int sr, int row_blocks,
-                             float2* __restrict__ raw) {
-    extern __shared__ __align__(16) float sm[];
-    const int lane = threadIdx.x & 31, s = threadIdx.x >> 5, wn = 2 * sr + 1, winsz = wn * wn;
-    const bool cols = (int)blockIdx.x >= row_blocks;
-    const int b = cols ? blockIdx.x - row_blocks : blockIdx.x;
-    const int nalong = cols ? nrows : ncols, nacross = cols ? ncols : nrows;
-    const int nblk = (nalong + 31) / 32, line = b / nblk, p0 = (b - line * nblk) * 32;
-    // line pair: side, then (edge line k = 0 .. sr - 1, one of its sr - k partners)
-    const int per = sr * (sr + 1) / 2, side = line / per;
-    int k = 0, t = line - side * per;
-    while (t >= sr - k) t -= sr - k++;
-    const int l1 = side ? nacross - 1 - k : k, l2 = side ? nacross - 1 - (k + sr + 1 + t) : k + sr + 1 + t;
-    // staged: 32 positions of the edge line, then the partner's positions under their windows
-    const int a0 = max(p0 - 2 * sr, 0), a1 = min(p0 + 32 + 2 * sr, nalong);
-    const int n1 = min(32, nalong - p0), nst = n1 + a1 - a0;
-    const int bufn = (32 + 32 + 4 * sr) * kEdgePitch;
-    auto pattern = [&](int along, int across) { return data + ((int64_t)(cols ? along : across) * ncols + (cols ? across : along)) * npx; };
-    auto stage = [&](int q0, float* buf) {
-        const int q = q0 + lane;
-        if (q < nind) {
-            const int px = __ldg(ind + q);
-            for (int i = s; i < nst; i += wn)
-                stage4(buf + i * kEdgePitch + lane, (i < n1 ? pattern(p0 + i, l1) : pattern(a0 + i - n1, l2)) + px);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    const int p = p0 + lane;
-    int ws, we;
-    window(p < nalong ? p : nalong - 1, sr, nalong, ws, we);
-    const int p2 = ws + s;  // the slot's position along the partner line
-    const bool ok = p < nalong && (!cols || (p2 - p <= sr && p - p2 <= sr));
-    const int self = ok ? lane * kEdgePitch : 0, other = ok ? (n1 + p2 - a0) * kEdgePitch : 0;
-    float d = 0.0f, n = 0.0f;
-    stage(0, sm);
-    for (int q0 = 0, it = 0; q0 < nind; q0 += kChunk, ++it) {
-        const float* cur = sm + (it & 1) * bufn;
-        const int qn = min(kChunk, nind - q0);
-        asm volatile("cp.async.wait_all;" ::: "memory");
-        __syncthreads();
-        if (q0 + kChunk < nind) stage(q0 + kChunk, sm + ((it + 1) & 1) * bufn);
-#pragma unroll 8
-        for (int qq = 0; qq < qn; ++qq) {
-            const float xv = cur[self + qq], yv = cur[other + qq];
-            const float u = __fsub_rn(xv, yv), uu = __fmul_rn(u, u);
-            if (yv < mxval && xv < mxval) {  // pair_ssd's order: count, difference, square
-                n = __fadd_rn(n, 1.0f);
-                d = __fadd_rn(d, uu);
-            }
-        }
-    }
-    if (!ok) return;
-    const int y = cols ? p : l1, x = cols ? l1 : p, y2 = cols ? p2 : l2, x2 = cols ? l2 : p2;
-    int ys, ye, xs, xe;
-    window(y, sr, nrows, ys, ye);
-    window(x, sr, ncols, xs, xe);
-    raw[edge_index(y, x, sr, nrows, ncols) * winsz + (y2 - ys) * wn + (x2 - xs)] = make_float2(d, n);
-}
-
 int edge_blocks(int sr, int nalong) { return sr * (sr + 1) * ((nalong + 31) / 32); }
-size_t edge_smem(int sr) { return (size_t)2 * (64 + 4 * sr) * kEdgePitch * sizeof(float); }
 
 // Normalised window weights of the edge pixels from their raw sums: one block (64 threads) per
 // edge pixel, the arithmetic of k_nlpar_weights_tiled.
@@ -990,7 +1005,9 @@ __global__ void k_nlpar_weights_edge(const float2* __restrict__ raw, const float
     if (c < winsz) wout[pix * winsz + c] = __fdiv_rn(W[c], T);
 }
 
-size_t pairs_smem(int sr) { return (size_t)2 * (sr + 1) * kChunk * kPairPitch * sizeof(float); }
+size_t pairs_smem(int sr) {
+    return std::max((size_t)2 * (sr + 1) * kChunk * kPairPitch, (size_t)2 * (64 + 4 * sr) * kEdgePitch) * sizeof(float);
+}
 
 size_t tiled_smem(int sr, int ncols, size_t elem, bool weights) {
     const int wn = 2 * sr + 1;
@@ -1272,12 +1289,17 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
     float2* pairs = (float2*)(d_work + ((npix * winsz + 1) & ~(int64_t)1));
     float2* sigp = pairs + npix * nF;
     cudaStream_t st = (cudaStream_t)stream;
-    const dim3 pgrid((unsigned)((ncols + 2 * kPairLanes - 1) / (2 * kPairLanes)), (unsigned)nrows);
-    typedef void (*PairsFn)(const float*, int, int, int, const int32_t*, int, float, float, float, float2*, float2*);
+    float2* raw = sigp + npix * 4;  // the edge pixels' window sums that are no pair sums
+    const int edge_rows = edge_blocks(sr, ncols), edge_all = edge_rows + edge_blocks(sr, nrows);
+    const int64_t pgrid = edge_all + (int64_t)((ncols + 2 * kPairLanes - 1) / (2 * kPairLanes)) * nrows;
+    if (pgrid > 0x7fffffff) return EBSD_E_UNSUPPORTED;
+    typedef void (*PairsFn)(const float*, int, int, int, const int32_t*, int, float, float, float, float2*, float2*, int, int,
+                            float2*);
     PairsFn fn = compute_sigma ? (sr == 1 ? k_nlpar_pairs<1, true> : sr == 2 ? k_nlpar_pairs<2, true> : k_nlpar_pairs<3, true>)
                                : (sr == 1 ? k_nlpar_pairs<1, false> : sr == 2 ? k_nlpar_pairs<2, false> : k_nlpar_pairs<3, false>);
     EBSD_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-    fn<<<pgrid, (unsigned)kPairThreads, psm, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, mxsig, 0.0f, pairs, sigp);
+    fn<<<(unsigned)pgrid, (unsigned)kPairThreads, psm, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, mxsig, 0.0f,
+                                                             pairs, sigp, edge_rows, edge_all, raw);
     int rc = launch_status();
     if (rc != EBSD_OK) return rc;
     if (compute_sigma) {
@@ -1289,12 +1311,8 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
                                                        d_sigma, lam2, dthresh, sr, w, d_centre_offset);
     if ((rc = launch_status()) != EBSD_OK) return rc;
     {
-        // edge pixels: the window sums that are no pair sums, then their weights
-        float2* raw = sigp + npix * 4;
-        const int nri = nrows - 2 * sr, rb = edge_blocks(sr, ncols);
-        k_nlpar_edge<<<(unsigned)(rb + edge_blocks(sr, nrows)), (unsigned)((2 * sr + 1) * 32), edge_smem(sr), st>>>(
-            d_data, nrows, ncols, npx, d_indices, nind, mxval, sr, rb, raw);
-        if ((rc = launch_status()) != EBSD_OK) return rc;
+        // edge pixels: their weights
+        const int nri = nrows - 2 * sr;
         const int64_t nedge = (int64_t)2 * sr * ncols + (int64_t)nri * 2 * sr;
         k_nlpar_weights_edge<<<(unsigned)nedge, 64, 0, st>>>(raw, pairs, nrows, ncols, sr, d_sigma, lam2, dthresh, w,
                                                              d_centre_offset);
