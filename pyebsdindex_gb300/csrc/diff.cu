@@ -137,47 +137,80 @@ __global__ void k_nlpar_weights2(const float* __restrict__ data, int nrows, int 
     }
 }
 
+// The list of the scan pixels p near q that `take(p, jp, ip)` accepts, in raster order, made by
+// one warp: candidates within reach of q (|dj|, |di| <= reach, inside the grid), the accepted
+// ones numbered by ballot from `base` on and handed to `put(index, p, jp, ip)`.  Returns the end.
+template <typename Take, typename Put>
+__device__ __forceinline__ int list_near(int q, int nrows, int ncols, int reach, int lane, int base, Take take, Put put) {
+    const int jq = q / ncols, iq = q - (q / ncols) * ncols, w = 2 * reach + 1;
+    for (int c0 = 0; c0 < w * w; c0 += 32) {
+        const int c = c0 + lane, jp = jq + c / w - reach, ip = iq + c % w - reach;
+        const int p = ip + ncols * jp;
+        const bool ok = c < w * w && jp >= 0 && jp < nrows && ip >= 0 && ip < ncols && take(p, jp, ip);
+        const unsigned m = __ballot_sync(0xffffffffu, ok);
+        if (ok) put(base + __popc(m & ((1u << lane) - 1u)), p, jp, ip);
+        base += __popc(m);
+    }
+    return base;
+}
+
+// The window slot in which pixel (jp, ip) holds (jq, iq), or -1.
+__device__ __forceinline__ int slot_of(int jp, int ip, int jq, int iq, int sr, int nrows, int ncols) {
+    int xs, xe, ys, ye;
+    window(ip, sr, ncols, xs, xe);
+    window(jp, sr, nrows, ys, ye);
+    return jq >= ys && jq < ye && iq >= xs && iq < xe ? (jq - ys) * (2 * sr + 1) + (iq - xs) : -1;
+}
+
 // out[q][k] = sum over scan pixels p whose window holds q of w[p][slot] * g[p][k].
+// One scan pixel q per blockIdx.y: the windows that hold q (pixel p, slot c) are listed by the
+// block's first warp in the scan order of the sum, then each thread adds w[p][c] g[p][k] over the
+// list for four pattern values at once (four loads in flight a term: with one, their latency was
+// the bound).  1024 pixels of 14400 values, radius 2: 364 us before, 115 now.
+constexpr int kAtVals = 4;
 template <typename T>
 __global__ void __launch_bounds__(256) k_nlpar_apply_t(const T* __restrict__ g, int nrows, int ncols, int npx,
                                                        const T* __restrict__ w, int sr, T* __restrict__ out) {
-    // one scan pixel q per blockIdx.y: the windows that hold q (pixel p, slot c) are listed
-    // once per block in the scan order of the sum, then each pattern value k adds
-    // w[p][c] g[p][k] over the list with fused multiply-adds
-    extern __shared__ unsigned char atsm[];
+    extern __shared__ __align__(16) unsigned char atsm[];
     const int q = blockIdx.y;
-    const int winsz = (2 * sr + 1) * (2 * sr + 1), wx = 2 * sr + 1;
+    const int winsz = (2 * sr + 1) * (2 * sr + 1);
     const int maxt = (4 * sr + 1) * (4 * sr + 1);
     T* wt = (T*)atsm;                 // [maxt] weights
     int* pt = (int*)(wt + maxt);      // [maxt] pixels
     __shared__ int nterm;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {
         const int jq = q / ncols, iq = q - (q / ncols) * ncols;
-        const int j0 = jq - 2 * sr < 0 ? 0 : jq - 2 * sr, j1 = jq + 2 * sr > nrows - 1 ? nrows - 1 : jq + 2 * sr;
-        const int i0 = iq - 2 * sr < 0 ? 0 : iq - 2 * sr, i1 = iq + 2 * sr > ncols - 1 ? ncols - 1 : iq + 2 * sr;
-        int t = 0;
-        for (int jp = j0; jp <= j1; ++jp) {
-            int ys, ye;
-            window(jp, sr, nrows, ys, ye);
-            if (jq < ys || jq >= ye) continue;
-            for (int ip = i0; ip <= i1; ++ip) {
-                int xs, xe;
-                window(ip, sr, ncols, xs, xe);
-                if (iq < xs || iq >= xe) continue;
-                const int p = ip + ncols * jp;
-                wt[t] = w[(int64_t)p * winsz + (jq - ys) * wx + (iq - xs)];
-                pt[t++] = p;
-            }
-        }
-        nterm = t;
+        const int nt = list_near(
+            q, nrows, ncols, 2 * sr, threadIdx.x, 0,
+            [&](int, int jp, int ip) { return slot_of(jp, ip, jq, iq, sr, nrows, ncols) >= 0; },
+            [&](int t, int p, int jp, int ip) {
+                wt[t] = w[(int64_t)p * winsz + slot_of(jp, ip, jq, iq, sr, nrows, ncols)];
+                pt[t] = p;
+            });
+        if (threadIdx.x == 0) nterm = nt;
     }
     __syncthreads();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= npx) return;
+    const int k0 = blockIdx.x * (blockDim.x * kAtVals) + threadIdx.x;
+    if (k0 >= npx) return;
     const int nt = nterm;
-    T acc = (T)0;
-    for (int t = 0; t < nt; ++t) acc = fma(wt[t], __ldg(g + (int64_t)pt[t] * npx + k), acc);
-    out[(int64_t)q * npx + k] = acc;
+    int64_t kk[kAtVals];
+    T acc[kAtVals];
+#pragma unroll
+    for (int i = 0; i < kAtVals; ++i) {
+        const int k = k0 + i * (int)blockDim.x;
+        kk[i] = k < npx ? k : k0;
+        acc[i] = (T)0;
+    }
+#pragma unroll 2
+    for (int t = 0; t < nt; ++t) {
+        const T* row = g + (int64_t)pt[t] * npx;
+        const T c = wt[t];
+#pragma unroll
+        for (int i = 0; i < kAtVals; ++i) acc[i] = fma(c, __ldg(row + kk[i]), acc[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < kAtVals; ++i)
+        if (k0 + i * (int)blockDim.x < npx) out[(int64_t)q * npx + kk[i]] = acc[i];
 }
 
 // Per scan pixel: sum_c dw_pc/dlambda * (g_p . x_c); block reduction over the pattern pixels.
@@ -223,7 +256,8 @@ __global__ void k_nlpar_lam_grad(const T* __restrict__ g, const T* __restrict__ 
 // (torch's "reflect" padding followed by a correlation), and its adjoint
 //   out[i] = sum_o sum_t taps[t + r] v[o] [refl(o + t) == i]
 // as a gather: the direct terms o = i - t, the mirror of the low edge (o + t = -i, 1 <= i <= r)
-// and of the high edge (o + t = 2(L-1) - i, L-1-r <= i <= L-2).  Requires r < L.
+// and of the high edge (o + t = 2(L-1) - i, L-1-r <= i <= L-2).  Requires r < L.  A thread per
+// output: double values (the FP64 pipe bounds them however they are read), r < 3, longest lines.
 template <typename T>
 __global__ void k_blur1d(const T* __restrict__ in, T* __restrict__ out, int64_t total, int H, int W, int axis,
                          const T* __restrict__ taps, int r) {
@@ -268,40 +302,284 @@ __global__ void k_blur1d_t(const T* __restrict__ v, T* __restrict__ out, int64_t
     out[idx] = acc;
 }
 
+// The same sums in the same order for float lines of moderate length (r >= 3): a block stages 32
+// whole lines in shared memory, a warp takes kBlurR neighbouring outputs of the 32 lines (a lane
+// per line, lines at a pitch of 33 floats: no bank conflicts along either axis), so each staged
+// value read feeds kBlurR multiply-adds and sixteen taps come in four 16-byte broadcasts.
+// Per output the positions ascend: the first and last kBlurR - 1 reach part of the outputs
+// (triangles unrolled), those between reach all of them.  What bounds it is issue: of the ~12
+// instructions a position costs 8 are the multiply-adds; the one-output-a-thread kernels above
+// spend 21 a tap.  1024 120x120 patterns, r = 30, per pass: 643 / 452 us along y / x before,
+// 94 / 109 now (the adjoint 384 / 526 before, 86 / 106 now).
+constexpr int kBlurR = 8, kBlurWarps = 4, kBlurLines = 32, kBlurPitch = 33, kBlurPad = 20;
+
+__host__ __device__ inline int blur_tap_off(int r) { return kBlurPad + ((4 - ((2 * r + 2 + kBlurPad) & 3)) & 3); }
+__host__ __device__ inline int blur_tap_len(int r) { return (blur_tap_off(r) + 2 * r + 1 + kBlurPad + 3) & ~3; }
+inline size_t blur_smem(int L, int axis, int r) {
+    return ((size_t)L * kBlurPitch * (axis == 1 ? 2 : 1) + (size_t)blur_tap_len(r)) * sizeof(float);
+}
+
+// acc[j] += sum of taps[c0 + j - o + r] line[o] (kCorr false, the positions o inside the line) or
+// of taps[o - c0 - j + r] line[refl(o)] (kCorr true), o ascending; tp holds the taps as the sum
+// meets them (kCorr reversed), tp[t] with t = c0 + j - o + r falling as o rises.
+template <bool kCorr, bool kRev>
+__device__ __forceinline__ void blur_sum(float (&acc)[kBlurR], const float* __restrict__ line,
+                                         const float* __restrict__ tp, int r, int c0, int L) {
+    auto at = [&](int o, bool& ok) -> int {
+        if (kCorr) {
+            ok = true;
+            o = o < 0 ? -o : o;
+            return o >= L ? 2 * (L - 1) - o : o;
+        }
+        ok = (unsigned)o < (unsigned)L;
+        return o;
+    };
+    const int base = c0 - r;
+    if (kCorr || base + kBlurR - 2 >= 0) {
+        float tq[kBlurR - 1];
+#pragma unroll
+        for (int i = 0; i < kBlurR - 1; ++i) tq[i] = tp[2 * r - i];
+#pragma unroll
+        for (int s = 0; s < kBlurR - 1; ++s) {
+            bool ok;
+            const int o = at(base + s, ok);
+            if (ok) {
+                const float v = line[o * kBlurPitch];
+#pragma unroll
+                for (int j = 0; j <= s; ++j) {
+                    float& a = acc[kRev ? kBlurR - 1 - j : j];
+                    a = fmaf(tq[s - j], v, a);
+                }
+            }
+        }
+    }
+    const int m0 = base + kBlurR - 1, m1 = c0 + r;  // positions that reach all outputs: [m0, m1]
+    for (int o0 = m0; o0 <= m1; o0 += kBlurR) {
+        if (!kCorr && (o0 + kBlurR - 1 < 0 || o0 >= L)) continue;
+        float t[2 * kBlurR];
+        const float4* t4 = reinterpret_cast<const float4*>(tp + (c0 - o0 - (kBlurR - 1) + r));
+#pragma unroll
+        for (int i = 0; i < 2 * kBlurR / 4; ++i) {
+            const float4 f = t4[i];
+            t[4 * i] = f.x; t[4 * i + 1] = f.y; t[4 * i + 2] = f.z; t[4 * i + 3] = f.w;
+        }
+#pragma unroll
+        for (int s = 0; s < kBlurR; ++s) {
+            bool ok;
+            const int o = at(o0 + s, ok);
+            if (ok && o0 + s <= m1) {
+                const float v = line[o * kBlurPitch];
+#pragma unroll
+                for (int j = 0; j < kBlurR; ++j) {
+                    float& a = acc[kRev ? kBlurR - 1 - j : j];
+                    a = fmaf(t[kBlurR - 1 - s + j], v, a);
+                }
+            }
+        }
+    }
+    if (kCorr || m1 + 1 < L) {
+        float tq[kBlurR - 1];
+#pragma unroll
+        for (int i = 0; i < kBlurR - 1; ++i) tq[i] = tp[i];
+#pragma unroll
+        for (int s = 0; s < kBlurR - 1; ++s) {
+            bool ok;
+            const int o = at(m1 + 1 + s, ok);
+            if (ok) {
+                const float v = line[o * kBlurPitch];
+#pragma unroll
+                for (int j = s + 1; j < kBlurR; ++j) {
+                    float& a = acc[kRev ? kBlurR - 1 - j : j];
+                    a = fmaf(tq[j - 1 - s], v, a);
+                }
+            }
+        }
+    }
+}
+
+template <int kAxis, bool kAdj>
+__global__ void __launch_bounds__(32 * kBlurWarps) k_blur_lines(const float* __restrict__ in, float* __restrict__ out,
+                                                                int64_t nlines, int H, int W,
+                                                                const float* __restrict__ taps, int r) {
+    extern __shared__ __align__(16) float blsm[];
+    const int L = kAxis == 0 ? H : W, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int tlen = blur_tap_len(r), toff = blur_tap_off(r);
+    float* tile = blsm + tlen;
+    float* otile = tile + L * kBlurPitch;   // along x only
+    for (int i = threadIdx.x; i < tlen; i += 32 * kBlurWarps) {
+        const int t = i - toff;
+        blsm[i] = (unsigned)t <= 2u * r ? taps[kAdj ? t : 2 * r - t] : 0.0f;
+    }
+    const int64_t l0 = (int64_t)blockIdx.x * kBlurLines;
+    const int nl = nlines - l0 < kBlurLines ? (int)(nlines - l0) : kBlurLines;
+    int64_t cb = 0;   // along y: the lane's column
+    if (kAxis == 0) {
+        const int64_t l = l0 + (lane < nl ? lane : nl - 1), p = l / W;
+        cb = p * H * W + (l - p * W);
+        for (int q = warp; q < L; q += kBlurWarps) tile[q * kBlurPitch + lane] = __ldg(in + cb + (int64_t)q * W);
+    } else {
+        for (int row = warp; row < nl; row += kBlurWarps)
+            for (int q = lane; q < L; q += 32) tile[q * kBlurPitch + row] = __ldg(in + (l0 + row) * L + q);
+    }
+    __syncthreads();
+    const float* line = tile + (lane < nl ? lane : 0);
+    const float* tp = blsm + toff;
+    for (int g0 = warp * kBlurR; g0 < L; g0 += kBlurWarps * kBlurR) {
+        // the last outputs of a ragged line: a group that ends with the line, some of them twice
+        const int i0 = g0 + kBlurR <= L || L < kBlurR ? g0 : L - kBlurR;
+        float acc[kBlurR];
+#pragma unroll
+        for (int j = 0; j < kBlurR; ++j) acc[j] = 0.0f;
+        if (!kAdj) {
+            if (L >= kBlurR) {
+                blur_sum<true, false>(acc, line, tp, r, i0, L);
+            } else {  // a line shorter than a group: output by output
+                for (int j = 0; j < L - i0; ++j) {
+                    float a = 0.0f;
+                    for (int t = 0; t <= 2 * r; ++t) {
+                        int o = i0 + j + t - r;
+                        o = o < 0 ? -o : (o >= L ? 2 * (L - 1) - o : o);
+                        a = fmaf(tp[2 * r - t], line[o * kBlurPitch], a);
+                    }
+#pragma unroll
+                    for (int jj = 0; jj < kBlurR; ++jj) if (jj == j) acc[jj] = a;
+                }
+            }
+        } else {
+            blur_sum<false, false>(acc, line, tp, r, i0, L);
+            if (i0 <= r) {  // the low edge's mirror images, output 0 not among them
+                const float keep = acc[0];
+                blur_sum<false, true>(acc, line, tp, r, -i0 - (kBlurR - 1), L);
+                if (i0 == 0) acc[0] = keep;
+            }
+            if (i0 + kBlurR - 1 >= L - 1 - r) {  // the high edge's, without output L - 1
+                float keep[kBlurR];
+#pragma unroll
+                for (int j = 0; j < kBlurR; ++j) keep[j] = acc[j];
+                blur_sum<false, true>(acc, line, tp, r, 2 * (L - 1) - i0 - (kBlurR - 1), L);
+#pragma unroll
+                for (int j = 0; j < kBlurR; ++j) if (i0 + j == L - 1) acc[j] = keep[j];
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < kBlurR; ++j) {
+            if (i0 + j < L) {
+                if (kAxis == 1) otile[(i0 + j) * kBlurPitch + lane] = acc[j];
+                else if (lane < nl) out[cb + (int64_t)(i0 + j) * W] = acc[j];
+            }
+        }
+    }
+    if (kAxis == 1) {
+        __syncthreads();
+        for (int row = warp; row < nl; row += kBlurWarps)
+            for (int q = lane; q < L; q += 32) out[(l0 + row) * L + q] = otile[q * kBlurPitch + row];
+    }
+}
+
+// Whether the blocked kernel takes the call: three and more taps a side (the triangles need
+// 2 r + 2 >= kBlurR) and lines that leave two blocks an SM (<= 96 KB of shared memory);
+// the others keep a thread per output.
+constexpr size_t kBlurSmemMax = 96 * 1024;
+inline bool blur_blocked(int64_t n, int H, int W, int axis, int r) {
+    const int64_t lines = axis == 0 ? n * W : n * H;
+    return r >= (kBlurR - 2) / 2 && blur_smem(axis == 0 ? H : W, axis, r) <= kBlurSmemMax &&
+           (lines + kBlurLines - 1) / kBlurLines <= 0x7fffffff;
+}
+
+template <int kAxis, bool kAdj>
+int launch_blur(const float* in, int64_t n, int H, int W, const float* taps, int r, float* out, cudaStream_t st) {
+    const size_t sm = blur_smem(kAxis == 0 ? H : W, kAxis, r);
+    if (sm > 48 * 1024 && cudaFuncSetAttribute(k_blur_lines<kAxis, kAdj>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               (int)kBlurSmemMax) != cudaSuccess)
+        return launch_status();
+    const int64_t lines = kAxis == 0 ? n * W : n * H;
+    k_blur_lines<kAxis, kAdj><<<(unsigned)((lines + kBlurLines - 1) / kBlurLines), 32 * kBlurWarps, sm, st>>>(
+        in, out, lines, H, W, taps, r);
+    return launch_status();
+}
+
 // ---- soft-argmax band sharpness ------------------------------------------------------------
 // Per pattern (one block): J_p = sum_i s_i c_i over the Radon-mask cells, s = softmax(c / tau),
 // and dJ_p / dc_i = s_i (1 + (c_i - J_p) / tau) (zero off the mask).  Sums in float64.
+//
+// Float patterns take the exponentials in float of arguments formed in double, and round the
+// gradient to float once.  The FP64 pipe issues a warp operation in sixteen cycles, and two dozen
+// of them a cell (products, divisions, conversions) were all that bounded the kernel, so the
+// float kernel leaves on it the two additions of the sums alone: the maximum is taken of the
+// floats (a product with inv_tau > 0 keeps their order), a float widens by integer shifts, and
+// the argument and the gradient are formed in pairs of floats (products and sums with their
+// rounding errors kept, ~2^-45 relative) before their one rounding to float.  Blocks whose values
+// would leave the float range in between (|c / tau| above 2^100) take the double expressions.
+// 1024 patterns of 180x180 cells: 1275 us before, 495 now.
+struct FloatPair { float h, l; };
+__device__ __forceinline__ FloatPair fp_of(double d) {
+    FloatPair r;
+    r.h = (float)d;
+    r.l = (float)(d - (double)r.h);
+    return r;
+}
+// v * b + a, as an unevaluated pair
+__device__ __forceinline__ FloatPair fp_fma(float v, FloatPair b, FloatPair a) {
+    const float p = __fmul_rn(v, b.h), pe = fmaf(v, b.l, fmaf(v, b.h, -p));
+    const float s = __fadd_rn(p, a.h), bb = __fsub_rn(s, p);
+    const float e = __fadd_rn(__fsub_rn(p, __fsub_rn(s, bb)), __fsub_rn(a.h, bb));
+    FloatPair r;
+    r.h = s;
+    r.l = __fadd_rn(e, __fadd_rn(pe, a.l));
+    return r;
+}
+__device__ __forceinline__ double widen(float f) {
+    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
+    if (m - 0x00800000u < 0x7f000000u)  // a normal number: the exponent rebiased
+        return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(u << 29));
+    return m == 0 ? 0.0 : (double)f;
+}
+
 template <typename T>
 __global__ void k_softargmax(const T* __restrict__ c, int64_t ncell, const int32_t* __restrict__ cells, int ncm,
                              double inv_tau, double* __restrict__ Jp, T* __restrict__ grad) {
-    // float patterns take the exponentials in float (their arguments formed in double), double
-    // patterns in double; the sums are double either way
-    __shared__ double red[64];
+    constexpr bool kF = sizeof(T) == 4;
+    __shared__ double red[66];
     const int64_t p = blockIdx.x;
     const T* cp = c + p * ncell;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
-    double mx = -INFINITY;
-    for (int k = tid; k < ncm; k += blockDim.x) mx = fmax(mx, (double)cp[cells[k]] * inv_tau);
-    for (int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_down_sync(0xffffffffu, mx, o));
-    if (lane == 0) red[warp] = mx;
+    T vx = (T)-INFINITY, vn = (T)INFINITY;
+    for (int k = tid; k < ncm; k += blockDim.x) {
+        const T v = cp[__ldg(cells + k)];
+        vx = v > vx ? v : vx;
+        vn = v < vn ? v : vn;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        const T a = __shfl_down_sync(0xffffffffu, vx, o), b = __shfl_down_sync(0xffffffffu, vn, o);
+        vx = a > vx ? a : vx;
+        vn = b < vn ? b : vn;
+    }
+    if (lane == 0) { red[warp] = (double)vx; red[32 + warp] = (double)vn; }
     __syncthreads();
     if (tid == 0) {
-        double m = red[0];
-        for (int w = 1; w < nw; ++w) m = fmax(m, red[w]);
-        red[63] = m;
+        double m = red[0], n = red[32];
+        for (int w = 1; w < nw; ++w) { m = fmax(m, red[w]); n = fmin(n, red[32 + w]); }
+        red[64] = m * inv_tau;
+        red[65] = n * inv_tau;
     }
     __syncthreads();
-    mx = red[63];
-    auto expo = [&](double v) -> double {
-        if (sizeof(T) == 4) return (double)expf((float)(v * inv_tau - mx));
-        return exp(v * inv_tau - mx);
+    const double mx = red[64];
+    constexpr double kBig = 1.2676506002282294e30;  // 2^100
+    const bool pairs = kF && fabs(mx) < kBig && fabs(red[65]) < kBig && inv_tau < kBig && inv_tau > 1.0 / kBig;
+    const FloatPair bt = fp_of(pairs ? inv_tau : 1.0), am = fp_of(pairs ? -mx : 0.0);
+    auto expo = [&](T v) -> float {  // float patterns
+        if (pairs) {
+            const FloatPair a = fp_fma((float)v, bt, am);
+            return expf(__fadd_rn(a.h, a.l));
+        }
+        return expf((float)((double)v * inv_tau - mx));
     };
     double s0 = 0.0, s1 = 0.0;
     for (int k = tid; k < ncm; k += blockDim.x) {
-        const double v = (double)cp[cells[k]];
-        const double e = expo(v);
+        const T v = cp[__ldg(cells + k)];
+        const double e = kF ? widen(expo(v)) : exp((double)v * inv_tau - mx);
         s0 += e;
-        s1 += e * v;
+        s1 += e * (kF ? widen((float)v) : (double)v);
     }
     for (int o = 16; o > 0; o >>= 1) {
         s0 += __shfl_down_sync(0xffffffffu, s0, o);
@@ -313,17 +591,27 @@ __global__ void k_softargmax(const T* __restrict__ c, int64_t ncell, const int32
     if (tid == 0) {
         double a = 0.0, b = 0.0;
         for (int w = 0; w < nw; ++w) { a += red[w]; b += red[32 + w]; }
-        red[62] = a;
-        red[61] = b / a;
+        red[64] = a;
+        red[65] = b / a;
         Jp[p] = b / a;
     }
     __syncthreads();
-    const double S0 = red[62], J = red[61];
+    const double S0 = red[64], J = red[65];
+    const FloatPair is = fp_of(pairs ? 1.0 / S0 : 0.0), aj = fp_of(pairs ? 1.0 - J * inv_tau : 0.0);
     T* gp = grad + p * ncell;
     for (int k = tid; k < ncm; k += blockDim.x) {
-        const double v = (double)cp[cells[k]];
-        const double si = expo(v) / S0;
-        gp[cells[k]] = (T)(si * (1.0 + (v - J) * inv_tau));
+        const int cell = __ldg(cells + k);
+        const T v = cp[cell];
+        if (pairs) {
+            const float e = expo(v);
+            const FloatPair q = fp_fma((float)v, bt, aj);
+            const float t = __fmul_rn(e, is.h), te = fmaf(e, is.l, fmaf(e, is.h, -t));
+            const float g = __fmul_rn(t, q.h);
+            gp[cell] = (T)__fadd_rn(g, fmaf(t, q.l, fmaf(te, q.h, fmaf(t, q.h, -g))));
+        } else {
+            const double si = (kF ? (double)expo(v) : exp((double)v * inv_tau - mx)) / S0;
+            gp[cell] = (T)(si * (1.0 + ((double)v - J) * inv_tau));
+        }
     }
 }
 
@@ -433,10 +721,14 @@ __global__ void k_nlpar_weights_d(const float* __restrict__ data, int nrows, int
 }
 
 // G[p][c] = g_p . x_c over all pattern pixels (float64 sums); one block per scan pixel, one warp
-// per window slot at a time.
+// per kDotSlots window slots at a time: g_p is read once for them, and their sums are
+// independent chains (with one slot a warp, the compensated sum's four dependent additions and
+// the loads' latency were the bound).  1024 pixels of 14400 values, radius 2: 340 us before,
+// 276 now.
+constexpr int kDotSlots = 4;
 template <typename T>
-__global__ void k_nlpar_dots(const T* __restrict__ g, const T* __restrict__ x, int nrows, int ncols, int npx, int sr,
-                             double* __restrict__ G) {
+__global__ void __launch_bounds__(256) k_nlpar_dots(const T* __restrict__ g, const T* __restrict__ x, int nrows,
+                                                    int ncols, int npx, int sr, double* __restrict__ G) {
     const int p = blockIdx.x;
     const int jp = p / ncols, ip = p - (p / ncols) * ncols;
     int xs, xe, ys, ye;
@@ -445,26 +737,46 @@ __global__ void k_nlpar_dots(const T* __restrict__ g, const T* __restrict__ x, i
     const int wx = xe - xs, winsz = (2 * sr + 1) * (2 * sr + 1);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const T* gp = g + (int64_t)p * npx;
-    for (int c = warp; c < winsz; c += nw) {
-        const int nb = (xs + c % wx) + ncols * (ys + c / wx);
-        const T* xc = x + (int64_t)nb * npx;
-        double acc = 0.0;
+    for (int c0 = warp * kDotSlots; c0 < winsz; c0 += nw * kDotSlots) {
+        const T* xc[kDotSlots];
+        double acc[kDotSlots];
+#pragma unroll
+        for (int i = 0; i < kDotSlots; ++i) {
+            const int c = c0 + i < winsz ? c0 + i : winsz - 1;
+            xc[i] = x + (int64_t)((xs + c % wx) + ncols * (ys + c / wx)) * npx;
+            acc[i] = 0.0;
+        }
         if (sizeof(T) == 4) {
             // float patterns: each lane's products summed in float with Kahan's compensation
             // (off the slow FP64 pipe), the lanes' sums combined in double
-            float sum = 0.0f, comp = 0.0f;
+            float sum[kDotSlots], comp[kDotSlots];
+#pragma unroll
+            for (int i = 0; i < kDotSlots; ++i) sum[i] = comp[i] = 0.0f;
+#pragma unroll 2
             for (int k = lane; k < npx; k += 32) {
-                const float y = __fsub_rn(__fmul_rn((float)__ldg(gp + k), (float)__ldg(xc + k)), comp);
-                const float t = __fadd_rn(sum, y);
-                comp = __fsub_rn(__fsub_rn(t, sum), y);
-                sum = t;
+                const float gk = (float)__ldg(gp + k);
+#pragma unroll
+                for (int i = 0; i < kDotSlots; ++i) {
+                    const float y = __fsub_rn(__fmul_rn(gk, (float)__ldg(xc[i] + k)), comp[i]);
+                    const float t = __fadd_rn(sum[i], y);
+                    comp[i] = __fsub_rn(__fsub_rn(t, sum[i]), y);
+                    sum[i] = t;
+                }
             }
-            acc = (double)sum - (double)comp;
+#pragma unroll
+            for (int i = 0; i < kDotSlots; ++i) acc[i] = (double)sum[i] - (double)comp[i];
         } else {
-            for (int k = lane; k < npx; k += 32) acc += (double)__ldg(gp + k) * (double)__ldg(xc + k);
+            for (int k = lane; k < npx; k += 32) {
+                const double gk = (double)__ldg(gp + k);
+#pragma unroll
+                for (int i = 0; i < kDotSlots; ++i) acc[i] += gk * (double)__ldg(xc[i] + k);
+            }
         }
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
-        if (lane == 0) G[(int64_t)p * winsz + c] = acc;
+#pragma unroll
+        for (int i = 0; i < kDotSlots; ++i) {
+            for (int o = 16; o > 0; o >>= 1) acc[i] += __shfl_down_sync(0xffffffffu, acc[i], o);
+            if (lane == 0 && c0 + i < winsz) G[(int64_t)p * winsz + c0 + i] = acc[i];
+        }
     }
 }
 
@@ -523,90 +835,102 @@ __global__ void k_nlpar_gamma(const double* __restrict__ beta, int nrows, int nc
 // dJ/dx_q[k] from the weights' dependence on the patterns: the pair SSDs of q's own window, of
 // the windows that hold q, and the noise sigma's minimising pair (q's own, and those of the
 // 3x3 neighbours whose minimum pairs with q).  Masked pixels only, each pair's saturation test.
-// d/dx of the weights' pattern dependence, one block per scan pixel q, its threads over the
-// pattern values k.  The terms that reach q -- its own window slots (the pair distances it
-// enters as the centre), the windows of the pixels whose windows hold q, and the noise sigma
-// of q and of the neighbours whose sigma pairs end at q -- are listed once per block with
-// their coefficients (2 alpha, gamma / n), then every value k adds coef * (x_q - x_n) for the
-// terms whose two values pass the saturation test of their kind.  Sums in the pixel's order;
-// float patterns accumulate in float (the coefficients rounded once), double in double.
+// One scan pixel q per blockIdx.x, the threads over the pattern values k.  The block's first warp
+// lists the pixels n that share a pair with q and their coefficients -- 2 alpha of the pair as q's
+// slot plus 2 alpha as n's slot, added in double, then gamma / n of the sigma pairs -- and every
+// value adds coef * (x_q - x_n) for the terms whose two values pass the saturation test of their
+// kind (a value of q that fails it, or lies off the mask, compares with -infinity).  Float
+// patterns accumulate in float (the coefficients rounded once), double in double.  A thread takes
+// four values, so four loads are in flight a term: with one value a thread and a list of both
+// orders of each pair made by one thread, latency was the bound.  1024 pixels of 14400 values,
+// radius 2: 1520 us before, 211 now.
+constexpr int kDxVals = 4, kDxThreads = 256;
 template <typename T>
-__global__ void __launch_bounds__(128) k_nlpar_dx(const T* __restrict__ x, int nrows, int ncols, int npx, int sr,
-                                                  const uint8_t* __restrict__ pmask, float mxw, float mxs,
-                                                  const double* __restrict__ alpha, const double* __restrict__ gamma,
-                                                  const int* __restrict__ arg, const float* __restrict__ nsig,
-                                                  T* __restrict__ out) {
-    extern __shared__ unsigned char dxsm[];
+__global__ void __launch_bounds__(kDxThreads) k_nlpar_dx(const T* __restrict__ x, int nrows, int ncols, int npx, int sr,
+                                                         const uint8_t* __restrict__ pmask, float mxw, float mxs,
+                                                         const double* __restrict__ alpha,
+                                                         const double* __restrict__ gamma, const int* __restrict__ arg,
+                                                         const float* __restrict__ nsig, T* __restrict__ out) {
+    extern __shared__ __align__(16) unsigned char dxsm[];
     const int q = blockIdx.x;
-    const int winsz = (2 * sr + 1) * (2 * sr + 1), wx = 2 * sr + 1;
-    const int maxt = winsz + (4 * sr + 1) * (4 * sr + 1) + 9;
+    const int winsz = (2 * sr + 1) * (2 * sr + 1);
+    const int maxt = (4 * sr + 1) * (4 * sr + 1) + 10;
     T* co = (T*)dxsm;                        // [maxt] coefficients
-    int* nbs = (int*)(co + maxt);           // [maxt] the other pixel; bit 31: a sigma term
-    __shared__ int nterm;
-    if (threadIdx.x == 0) {
-        int t = 0;
-        const int jq = q / ncols, iq = q - (q / ncols) * ncols;
-        {
-            int xs, xe, ys, ye;
-            window(iq, sr, ncols, xs, xe);
-            window(jq, sr, nrows, ys, ye);
-            const int wq = xe - xs;
-            for (int c = 0; c < winsz; ++c) {
-                const int nb = (xs + c % wq) + ncols * (ys + c / wq);
-                if (nb == q) continue;
-                co[t] = (T)(2.0 * alpha[(int64_t)q * winsz + c]);
-                nbs[t++] = nb;
-            }
-        }
-        const int j0 = jq - 2 * sr < 0 ? 0 : jq - 2 * sr, j1 = jq + 2 * sr > nrows - 1 ? nrows - 1 : jq + 2 * sr;
-        const int i0 = iq - 2 * sr < 0 ? 0 : iq - 2 * sr, i1 = iq + 2 * sr > ncols - 1 ? ncols - 1 : iq + 2 * sr;
-        for (int jp = j0; jp <= j1; ++jp) {
-            int ys, ye;
-            window(jp, sr, nrows, ys, ye);
-            if (jq < ys || jq >= ye) continue;
-            for (int ip = i0; ip <= i1; ++ip) {
-                int xs, xe;
-                window(ip, sr, ncols, xs, xe);
-                if (iq < xs || iq >= xe) continue;
-                const int p = ip + ncols * jp;
-                if (p == q) continue;
-                co[t] = (T)(2.0 * alpha[(int64_t)p * winsz + (jq - ys) * wx + (iq - xs)]);
-                nbs[t++] = p;
-            }
-        }
+    int* nbs = (int*)(co + maxt);           // [maxt] the other pixel
+    __shared__ int nwt, nterm;
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x, jq = q / ncols, iq = q - (q / ncols) * ncols;
+        const int nw = list_near(
+            q, nrows, ncols, 2 * sr, lane, 0,
+            [&](int p, int jp, int ip) {
+                return p != q && (slot_of(jp, ip, jq, iq, sr, nrows, ncols) >= 0 ||
+                                  slot_of(jq, iq, jp, ip, sr, nrows, ncols) >= 0);
+            },
+            [&](int t, int p, int jp, int ip) {
+                const int mine = slot_of(jq, iq, jp, ip, sr, nrows, ncols);
+                const int theirs = slot_of(jp, ip, jq, iq, sr, nrows, ncols);
+                double a = 0.0;
+                if (mine >= 0) a = 2.0 * alpha[(int64_t)q * winsz + mine];
+                if (theirs >= 0) a += 2.0 * alpha[(int64_t)p * winsz + theirs];
+                co[t] = (T)a;
+                nbs[t] = p;
+            });
         // noise sigma: sigma_p^2 = SSD(p, arg_p) / (2 n_p)
+        int nt = nw;
         const int aq = arg[q];
         if (aq >= 0) {
-            co[t] = (T)(gamma[q] / (double)nsig[q]);
-            nbs[t++] = aq | (int)0x80000000u;
-        }
-        for (int dj = -1; dj <= 1; ++dj)
-            for (int di = -1; di <= 1; ++di) {
-                const int jn = jq + dj, in_ = iq + di;
-                if ((dj == 0 && di == 0) || jn < 0 || jn >= nrows || in_ < 0 || in_ >= ncols) continue;
-                const int p = in_ + ncols * jn;
-                if (arg[p] != q) continue;
-                co[t] = (T)(gamma[p] / (double)nsig[p]);
-                nbs[t++] = p | (int)0x80000000u;
+            if (lane == 0) {
+                co[nt] = (T)(gamma[q] / (double)nsig[q]);
+                nbs[nt] = aq;
             }
-        nterm = t;
+            ++nt;
+        }
+        nt = list_near(
+            q, nrows, ncols, 1, lane, nt, [&](int p, int, int) { return p != q && arg[p] == q; },
+            [&](int t, int p, int, int) {
+                co[t] = (T)(gamma[p] / (double)nsig[p]);
+                nbs[t] = p;
+            });
+        if (lane == 0) {
+            nwt = nw;
+            nterm = nt;
+        }
     }
     __syncthreads();
-    const int nt = nterm;
+    const int nw = nwt, nt = nterm;
     const T* xq_row = x + (int64_t)q * npx;
-    for (int k = threadIdx.x; k < npx; k += blockDim.x) {
-        T acc = (T)0;
-        if (pmask[k]) {
-            const T xq = xq_row[k];
-            const bool qw = xq < (T)mxw, qs = xq < (T)mxs;
-            for (int t = 0; t < nt; ++t) {
-                const int e = nbs[t];
-                const bool sigma_term = e < 0;
-                const T xn = x[(int64_t)(e & 0x7fffffff) * npx + k];
-                if (sigma_term ? (qs && xn < (T)mxs) : (qw && xn < (T)mxw)) acc += co[t] * (xq - xn);
-            }
+    for (int k0 = blockIdx.y * (kDxThreads * kDxVals) + threadIdx.x; k0 < npx;
+         k0 += gridDim.y * (kDxThreads * kDxVals)) {
+        int kk[kDxVals];
+        T xq[kDxVals], lim[kDxVals], acc[kDxVals];
+        bool on[kDxVals];
+#pragma unroll
+        for (int i = 0; i < kDxVals; ++i) {
+            const int k = k0 + i * kDxThreads;
+            kk[i] = k < npx ? k : k0;
+            on[i] = pmask[kk[i]] != 0;
+            xq[i] = xq_row[kk[i]];
+            lim[i] = on[i] && xq[i] < (T)mxw ? (T)mxw : (T)-INFINITY;
+            acc[i] = (T)0;
         }
-        out[(int64_t)q * npx + k] = acc;
+        auto add = [&](int t) {
+            const T* xn_row = x + (int64_t)nbs[t] * npx;
+            const T c = co[t];
+            T xn[kDxVals];
+#pragma unroll
+            for (int i = 0; i < kDxVals; ++i) xn[i] = __ldg(xn_row + kk[i]);
+#pragma unroll
+            for (int i = 0; i < kDxVals; ++i)
+                if (xn[i] < lim[i]) acc[i] += c * (xq[i] - xn[i]);
+        };
+#pragma unroll 2
+        for (int t = 0; t < nw; ++t) add(t);
+#pragma unroll
+        for (int i = 0; i < kDxVals; ++i) lim[i] = on[i] && xq[i] < (T)mxs ? (T)mxs : (T)-INFINITY;
+        for (int t = nw; t < nt; ++t) add(t);
+#pragma unroll
+        for (int i = 0; i < kDxVals; ++i)
+            if (k0 + i * kDxThreads < npx) out[(int64_t)q * npx + kk[i]] = acc[i];
     }
 }
 
@@ -725,6 +1049,11 @@ int ebsd_blur1d(int fp64, int adjoint, int axis, const void* d_in, int64_t n, in
     if (fp64) {
         if (adjoint) k_blur1d_t<double><<<blocks, 256, 0, st>>>((const double*)d_in, (double*)d_out, total, H, W, axis, (const double*)d_taps, r);
         else k_blur1d<double><<<blocks, 256, 0, st>>>((const double*)d_in, (double*)d_out, total, H, W, axis, (const double*)d_taps, r);
+    } else if (blur_blocked(n, H, W, axis, r)) {
+        const float *in = (const float*)d_in, *tp = (const float*)d_taps;
+        float* o = (float*)d_out;
+        if (axis == 0) return adjoint ? launch_blur<0, true>(in, n, H, W, tp, r, o, st) : launch_blur<0, false>(in, n, H, W, tp, r, o, st);
+        return adjoint ? launch_blur<1, true>(in, n, H, W, tp, r, o, st) : launch_blur<1, false>(in, n, H, W, tp, r, o, st);
     } else {
         if (adjoint) k_blur1d_t<float><<<blocks, 256, 0, st>>>((const float*)d_in, (float*)d_out, total, H, W, axis, (const float*)d_taps, r);
         else k_blur1d<float><<<blocks, 256, 0, st>>>((const float*)d_in, (float*)d_out, total, H, W, axis, (const float*)d_taps, r);
@@ -792,17 +1121,20 @@ int ebsd_nlpar_weights_grad(int fp64, const void* d_g, const void* d_x, int32_t 
     k_nlpar_coef<<<(unsigned)((npix + 127) / 128), 128, 0, st>>>(G, d_w, d_m, d_dS, d_dsig, npix, winsz, lam, alpha,
                                                                  beta, d_glam);
     k_nlpar_gamma<<<(unsigned)((npix + 127) / 128), 128, 0, st>>>(beta, nrows, ncols, sr, gamma);
-    const size_t maxt = (size_t)winsz + (size_t)(4 * sr + 1) * (4 * sr + 1) + 9;
+    const size_t maxt = (size_t)(4 * sr + 1) * (4 * sr + 1) + 10;
     const size_t dsm = maxt * ((fp64 ? sizeof(double) : sizeof(float)) + sizeof(int));
-    if (fp64) k_nlpar_dx<double><<<(unsigned)npix, 128, dsm, st>>>((const double*)d_x, nrows, ncols, npx, sr, d_pmask, mxw, mxs, alpha, gamma, d_arg, d_nsig, (double*)d_gx);
-    else k_nlpar_dx<float><<<(unsigned)npix, 128, dsm, st>>>((const float*)d_x, nrows, ncols, npx, sr, d_pmask, mxw, mxs, alpha, gamma, d_arg, d_nsig, (float*)d_gx);
+    // the values of a pixel over as many blocks as it takes to fill the chip (sixteen an SM)
+    const int chunks = (npx + kDxThreads * kDxVals - 1) / (kDxThreads * kDxVals), want = (152 * 16 + npix - 1) / npix;
+    const dim3 xgrid((unsigned)npix, (unsigned)(want < chunks ? want : chunks));
+    if (fp64) k_nlpar_dx<double><<<xgrid, kDxThreads, dsm, st>>>((const double*)d_x, nrows, ncols, npx, sr, d_pmask, mxw, mxs, alpha, gamma, d_arg, d_nsig, (double*)d_gx);
+    else k_nlpar_dx<float><<<xgrid, kDxThreads, dsm, st>>>((const float*)d_x, nrows, ncols, npx, sr, d_pmask, mxw, mxs, alpha, gamma, d_arg, d_nsig, (float*)d_gx);
     return launch_status();
 }
 
 int ebsd_nlpar_apply_t(const float* d_g, int32_t nrows, int32_t ncols, int32_t npx, const float* d_w, int32_t sr,
                        float* d_out, void* stream) {
     if (!d_g || !d_w || !d_out || nrows <= 0 || ncols <= 0 || npx <= 0 || sr < 0 || sr > 10) return EBSD_E_ARG;
-    dim3 grid((unsigned)((npx + 255) / 256), (unsigned)(nrows * ncols));
+    dim3 grid((unsigned)((npx + 256 * kAtVals - 1) / (256 * kAtVals)), (unsigned)(nrows * ncols));
     k_nlpar_apply_t<float><<<grid, 256, (size_t)(4 * sr + 1) * (4 * sr + 1) * (sizeof(float) + sizeof(int)),
                              (cudaStream_t)stream>>>(d_g, nrows, ncols, npx, d_w, sr, d_out);
     return launch_status();
@@ -811,7 +1143,7 @@ int ebsd_nlpar_apply_t(const float* d_g, int32_t nrows, int32_t ncols, int32_t n
 int ebsd_nlpar_apply_t64(const double* d_g, int32_t nrows, int32_t ncols, int32_t npx, const double* d_w,
                          int32_t sr, double* d_out, void* stream) {
     if (!d_g || !d_w || !d_out || nrows <= 0 || ncols <= 0 || npx <= 0 || sr < 0 || sr > 10) return EBSD_E_ARG;
-    dim3 grid((unsigned)((npx + 255) / 256), (unsigned)(nrows * ncols));
+    dim3 grid((unsigned)((npx + 256 * kAtVals - 1) / (256 * kAtVals)), (unsigned)(nrows * ncols));
     k_nlpar_apply_t<double><<<grid, 256, (size_t)(4 * sr + 1) * (4 * sr + 1) * (sizeof(double) + sizeof(int)),
                               (cudaStream_t)stream>>>(d_g, nrows, ncols, npx, d_w, sr, d_out);
     return launch_status();

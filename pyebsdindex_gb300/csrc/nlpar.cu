@@ -1335,8 +1335,7 @@ int ebsd_nlpar_apply(const float* d_x, int32_t nrows, int32_t ncols, int32_t npx
     const size_t asm_ = tiled_smem(sr, ncols, sizeof(float), false);
     if (asm_ <= 48 * 1024) {
         const dim3 tgrid((unsigned)((ncols + kTileX - 1) / kTileX), (unsigned)nrows), tblock(kTileX, kTy);
-        launch_average_tiled<float, float>(tgrid, tblock, asm_, (cudaStream_t)stream, d_x, nrows, ncols, npx, d_w, sr,
-                                           d_out);
+        launch_average<float>(tgrid, tblock, asm_, (cudaStream_t)stream, d_x, nrows, ncols, npx, d_w, sr, d_out);
         return launch_status();
     }
     dim3 grid((unsigned)((npx + 255) / 256), (unsigned)(nrows * ncols));
