@@ -474,10 +474,16 @@ int ebsd_linop_apply(ebsd_linop_t op, int fp64, const void* d_x, int64_t n, void
 
 /* The same with the patterns along the fast axis: x^T [ncols][ldx] and y^T [nrows][ldy] hold
  * pattern b in column b (b < n <= ldx, ldy).  Results equal ebsd_linop_apply's bit for bit;
- * the operator's rows are read once per 32 patterns and the reads of x^T are coalesced, which
+ * the operator's rows are read once per 128 patterns and the reads of x^T are coalesced, which
  * is the layout a batch of thousands of patterns wants. */
 int ebsd_linop_apply_cols(ebsd_linop_t op, int fp64, const void* d_xT, int64_t ldx, int64_t n, void* d_yT,
                           int64_t ldy, void* stream);
+
+/* Row length of the image that the operator's rows index, row by row (rays by angle, pixels by
+ * column; 0 <= width <= nrows, 0: none).  ebsd_linop_apply_cols takes its rows in tiles of that
+ * image, where neighbours read the same columns; results do not depend on it.  Not to be called
+ * while another thread applies the operator. */
+int ebsd_linop_set_width(ebsd_linop_t op, int64_t width);
 
 int ebsd_linop_destroy(ebsd_linop_t op);
 
@@ -535,6 +541,18 @@ int ebsd_nlpar_weights_d(const float* d_data, int32_t nrows, int32_t ncols, int3
                          const int32_t* d_indices, int32_t nind, float datamax, float lam, int32_t sr,
                          float dthresh, const float* d_sig2, int saturation_protect, float* d_w, float* d_m,
                          float* d_dS, float* d_dsig, void* stream);
+
+/* Both of the above from one pass over the patterns, for a radius of 1 to 3: each pair's
+ * distance is summed once (as ebsd_nlpar_pairs_out does) and read by both its pixels; results
+ * equal theirs bit for bit.  compute_sigma = 1 fills d_sig2, d_arg and d_nsig first, 0 reads
+ * d_sig2 (d_arg, d_nsig may be null).  d_work: ebsd_nlpar_sigma_weights_d_work() floats, 8-byte
+ * aligned (0: this radius or grid is not served). */
+int64_t ebsd_nlpar_sigma_weights_d_work(int32_t nrows, int32_t ncols, int32_t sr);
+int ebsd_nlpar_sigma_weights_d(const float* d_data, int32_t nrows, int32_t ncols, int32_t npx,
+                               const int32_t* d_indices, int32_t nind, float datamax, float lam, int32_t sr,
+                               float dthresh, int compute_sigma, int saturation_protect, float* d_work,
+                               float* d_sig2, int32_t* d_arg, float* d_nsig, float* d_w, float* d_m,
+                               float* d_dS, float* d_dsig, void* stream);
 
 /* Backward of the weights for y = W(lambda, x) x given g = dL/dy: into d_gx the part of dL/dx
  * that flows through the weights -- each pair's SSD over the masked pixels d_pmask[npx] where

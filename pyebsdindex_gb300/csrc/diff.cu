@@ -15,6 +15,7 @@
 //                     dw_pc/dlambda = w_pc (2 / lambda^3) (m_pc - sum_c' w_pc' m_pc')
 #include "ebsd_internal.cuh"
 
+#include <cstring>
 #include <new>
 
 struct ebsd_linop_s {
@@ -24,6 +25,8 @@ struct ebsd_linop_s {
     int32_t* col = nullptr;
     float* val = nullptr;
     double* val64 = nullptr;
+    int2* ent = nullptr;     // (column, float value) of each nonzero
+    int64_t width = 0;       // the rows' image width, or 0: where neighbouring rows lie
 };
 
 namespace ebsd {
@@ -43,25 +46,107 @@ __global__ void k_csr_gather(const int64_t* __restrict__ rowptr, const int32_t* 
 }
 
 // The same products with the patterns along the fast axis: x^T [ncols][ldx], y^T [nrows][ldy]
-// hold pattern b in column b.  A warp takes one operator row for 32 patterns (lanes): each
-// nonzero's column of x^T is one coalesced load, and the row's entries are read once per 32
-// patterns.  Each output adds its row's terms in CSR order with fused multiply-adds, as
-// k_csr_gather, so the results are the same bit for bit.
-template <typename T>
-__global__ void __launch_bounds__(256) k_csr_gather_cols(const int64_t* __restrict__ rowptr,
-                                                         const int32_t* __restrict__ col,
-                                                         const T* __restrict__ val, const T* __restrict__ xT,
-                                                         int64_t ldx, T* __restrict__ yT, int64_t ldy,
-                                                         int64_t nrows, int64_t n) {
-    const int64_t row = (int64_t)blockIdx.x * 8 + threadIdx.y;
-    const int64_t b = (int64_t)blockIdx.y * 32 + threadIdx.x;
-    if (row >= nrows || b >= n) return;
-    const int64_t e1 = __ldg(rowptr + row + 1);
-    T acc = (T)0;
+// hold pattern b in column b.  Each output adds its row's terms in CSR order with fused
+// multiply-adds, as k_csr_gather, so the results are the same bit for bit.
+//
+// Rows that neighbour in the image they index (rays of near angle and offset, near pixels) meet
+// the same columns at about the same place of their rows, so a block takes a tile of
+// kCsrTileY x kCsrTileX rows of that image and its reads of x^T hit L1 instead of L2.  A warp
+// takes kCsrRows neighbouring rows at once and 32 NV patterns: a nonzero costs one 8-byte
+// broadcast, and NV coalesced loads feed NV multiply-adds of independent chains.  Bound by the
+// L1's 128 bytes a cycle.  1024 patterns, 120x120 pixels, 180x180 rays: Radon 1261 us with a row
+// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 912 now; its adjoint 1235, 1110
+// now; the LoG 451, 318 now.
+constexpr int kCsrTileY = 4, kCsrTileX = 8, kCsrRows = 4;
+
+template <typename T> struct CsrEnt;
+template <> struct CsrEnt<float> {
+    const int2* e;
+    __device__ __forceinline__ void get(int64_t i, int& c, float& v) const {
+        const int2 t = __ldg(e + i);
+        c = t.x;
+        v = __int_as_float(t.y);
+    }
+};
+template <> struct CsrEnt<double> {
+    const int32_t* col;
+    const double* val;
+    __device__ __forceinline__ void get(int64_t i, int& c, double& v) const {
+        c = __ldg(col + i);
+        v = __ldg(val + i);
+    }
+};
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(256) k_csr_gather_cols(const int64_t* __restrict__ rowptr, CsrEnt<T> ent,
+                                                         const T* __restrict__ xT, int64_t ldx, T* __restrict__ yT,
+                                                         int64_t ldy, int64_t nrows, int64_t width, int64_t n) {
+    static_assert(kCsrTileY * kCsrTileX == 8 * kCsrRows, "eight warps a tile");
+    constexpr int kWarpsX = kCsrTileX / kCsrRows;
+    const int64_t tx = (width + kCsrTileX - 1) / kCsrTileX, ty = blockIdx.x / tx;
+    const int64_t gx = (blockIdx.x - ty * tx) * kCsrTileX + (threadIdx.y % kWarpsX) * kCsrRows;
+    const int64_t gy = ty * kCsrTileY + threadIdx.y / kWarpsX, row = gy * width + gx;
+    if (gx >= width || row >= nrows) return;
+    const int64_t b0 = (int64_t)blockIdx.y * (32 * NV) + threadIdx.x;
+    int64_t e[kCsrRows];
+    int len[kCsrRows];
+    int common = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < kCsrRows; ++i) {
+        const int64_t r = gx + i < width && row + i < nrows ? row + i : row;  // past the image: the first row again
+        e[i] = __ldg(rowptr + r);
+        len[i] = (int)(__ldg(rowptr + r + 1) - e[i]);
+        common = len[i] < common ? len[i] : common;
+    }
+    int64_t off[NV];  // patterns past the last read column 0 and are not stored
+#pragma unroll
+    for (int v = 0; v < NV; ++v) off[v] = b0 + 32 * v < n ? b0 + 32 * v : 0;
+    T acc[kCsrRows][NV];
+#pragma unroll
+    for (int i = 0; i < kCsrRows; ++i)
+#pragma unroll
+        for (int v = 0; v < NV; ++v) acc[i][v] = (T)0;
+#pragma unroll 2
+    for (int t = 0; t < common; ++t)
+#pragma unroll
+        for (int i = 0; i < kCsrRows; ++i) {
+            int c;
+            T a;
+            ent.get(e[i] + t, c, a);
+            const T* xr = xT + (int64_t)c * ldx;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
+        }
+#pragma unroll
+    for (int i = 0; i < kCsrRows; ++i) {
 #pragma unroll 4
-    for (int64_t e = __ldg(rowptr + row); e < e1; ++e)
-        acc = fma(__ldg(val + e), __ldg(xT + (int64_t)__ldg(col + e) * ldx + b), acc);
-    yT[row * ldy + b] = acc;
+        for (int t = common; t < len[i]; ++t) {
+            int c;
+            T a;
+            ent.get(e[i] + t, c, a);
+            const T* xr = xT + (int64_t)c * ldx;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
+        }
+        if (gx + i < width && row + i < nrows)
+#pragma unroll
+            for (int v = 0; v < NV; ++v)
+                if (b0 + 32 * v < n) yT[(row + i) * ldy + b0 + 32 * v] = acc[i][v];
+    }
+}
+
+// Patterns a warp: 128 in float, 64 in double; a batch of fewer takes what it fills.
+template <typename T>
+void launch_csr_cols(cudaStream_t st, const int64_t* rowptr, CsrEnt<T> ent, const T* xT, int64_t ldx, T* yT, int64_t ldy,
+                     int64_t nrows, int64_t width, int64_t n) {
+    const unsigned tiles = (unsigned)(((width + kCsrTileX - 1) / kCsrTileX) * ((nrows + width * kCsrTileY - 1) / (width * kCsrTileY)));
+    const dim3 block(32, 8);
+    if (n > 64 && sizeof(T) == 4)
+        k_csr_gather_cols<T, 4><<<dim3(tiles, (unsigned)((n + 127) / 128)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
+    else if (n > 32)
+        k_csr_gather_cols<T, 2><<<dim3(tiles, (unsigned)((n + 63) / 64)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
+    else
+        k_csr_gather_cols<T, 1><<<dim3(tiles, (unsigned)((n + 31) / 32)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
 }
 
 __device__ __forceinline__ void window(int i, int sr, int n, int& start, int& end) {
@@ -510,7 +595,7 @@ int launch_blur(const float* in, int64_t n, int H, int W, const float* taps, int
 // the argument and the gradient are formed in pairs of floats (products and sums with their
 // rounding errors kept, ~2^-45 relative) before their one rounding to float.  Blocks whose values
 // would leave the float range in between (|c / tau| above 2^100) take the double expressions.
-// 1024 patterns of 180x180 cells: 1275 us before, 495 now.
+// 1024 patterns of 180x180 cells: 1275 us before, 377 now.
 struct FloatPair { float h, l; };
 __device__ __forceinline__ FloatPair fp_of(double d) {
     FloatPair r;
@@ -528,11 +613,21 @@ __device__ __forceinline__ FloatPair fp_fma(float v, FloatPair b, FloatPair a) {
     r.l = __fadd_rn(e, __fadd_rn(pe, a.l));
     return r;
 }
+// (double)f by integer operations (a conversion instruction runs at the FP64 pipe's rate)
 __device__ __forceinline__ double widen(float f) {
-    const unsigned u = __float_as_uint(f), m = u & 0x7fffffffu;
-    if (m - 0x00800000u < 0x7f000000u)  // a normal number: the exponent rebiased
-        return __hiloint2double((int)((u & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(u << 29));
-    return m == 0 ? 0.0 : (double)f;
+    const unsigned u = __float_as_uint(f), sign = u & 0x80000000u;
+    unsigned m = u & 0x7fffffffu, bias = 0x38000000u;  // the exponent rebiased by 1023 - 127
+    if (m - 0x00800000u >= 0x7f000000u) {
+        if (m == 0) return __hiloint2double((int)sign, 0);
+        if (m >= 0x7f800000u) {
+            bias = 0x70000000u;                        // infinity, NaN
+        } else {
+            const int sh = __clz(m) - 8;               // subnormal: normalised
+            m = (m << sh) & 0x7fffffu;
+            bias = (unsigned)(897 - sh) << 20;
+        }
+    }
+    return __hiloint2double((int)(sign | ((m >> 3) + bias)), (int)(m << 29));
 }
 
 template <typename T>
@@ -540,10 +635,12 @@ __global__ void k_softargmax(const T* __restrict__ c, int64_t ncell, const int32
                              double inv_tau, double* __restrict__ Jp, T* __restrict__ grad) {
     constexpr bool kF = sizeof(T) == 4;
     __shared__ double red[66];
+    __shared__ FloatPair cst[4];  // inv_tau, -max c / tau, 1 / sum, 1 - J / tau
     const int64_t p = blockIdx.x;
     const T* cp = c + p * ncell;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nw = blockDim.x >> 5;
     T vx = (T)-INFINITY, vn = (T)INFINITY;
+#pragma unroll 8
     for (int k = tid; k < ncm; k += blockDim.x) {
         const T v = cp[__ldg(cells + k)];
         vx = v > vx ? v : vx;
@@ -566,20 +663,36 @@ __global__ void k_softargmax(const T* __restrict__ c, int64_t ncell, const int32
     const double mx = red[64];
     constexpr double kBig = 1.2676506002282294e30;  // 2^100
     const bool pairs = kF && fabs(mx) < kBig && fabs(red[65]) < kBig && inv_tau < kBig && inv_tau > 1.0 / kBig;
-    const FloatPair bt = fp_of(pairs ? inv_tau : 1.0), am = fp_of(pairs ? -mx : 0.0);
-    auto expo = [&](T v) -> float {  // float patterns
-        if (pairs) {
-            const FloatPair a = fp_fma((float)v, bt, am);
-            return expf(__fadd_rn(a.h, a.l));
-        }
-        return expf((float)((double)v * inv_tau - mx));
+    if (tid == 0 && pairs) {
+        cst[0] = fp_of(inv_tau);
+        cst[1] = fp_of(-mx);
+    }
+    __syncthreads();
+    const FloatPair bt = cst[0], am = cst[1];
+    auto epair = [&](T v) -> float {
+        const FloatPair a = fp_fma((float)v, bt, am);
+        return expf(__fadd_rn(a.h, a.l));
+    };
+    auto eplain = [&](T v) -> double {
+        const double a = (double)v * inv_tau - mx;
+        return kF ? (double)expf((float)a) : exp(a);
     };
     double s0 = 0.0, s1 = 0.0;
-    for (int k = tid; k < ncm; k += blockDim.x) {
-        const T v = cp[__ldg(cells + k)];
-        const double e = kF ? widen(expo(v)) : exp((double)v * inv_tau - mx);
-        s0 += e;
-        s1 += e * (kF ? widen((float)v) : (double)v);
+    if (pairs) {
+#pragma unroll 4
+        for (int k = tid; k < ncm; k += blockDim.x) {
+            const T v = cp[__ldg(cells + k)];
+            const double e = widen(epair(v));
+            s0 += e;
+            s1 += e * widen((float)v);
+        }
+    } else {
+        for (int k = tid; k < ncm; k += blockDim.x) {
+            const T v = cp[__ldg(cells + k)];
+            const double e = eplain(v);
+            s0 += e;
+            s1 += e * (double)v;
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         s0 += __shfl_down_sync(0xffffffffu, s0, o);
@@ -594,23 +707,31 @@ __global__ void k_softargmax(const T* __restrict__ c, int64_t ncell, const int32
         red[64] = a;
         red[65] = b / a;
         Jp[p] = b / a;
+        if (pairs) {
+            cst[2] = fp_of(1.0 / a);
+            cst[3] = fp_of(1.0 - b / a * inv_tau);
+        }
     }
     __syncthreads();
     const double S0 = red[64], J = red[65];
-    const FloatPair is = fp_of(pairs ? 1.0 / S0 : 0.0), aj = fp_of(pairs ? 1.0 - J * inv_tau : 0.0);
+    const FloatPair is = cst[2], aj = cst[3];
     T* gp = grad + p * ncell;
-    for (int k = tid; k < ncm; k += blockDim.x) {
-        const int cell = __ldg(cells + k);
-        const T v = cp[cell];
-        if (pairs) {
-            const float e = expo(v);
+    if (pairs) {
+#pragma unroll 4
+        for (int k = tid; k < ncm; k += blockDim.x) {
+            const int cell = __ldg(cells + k);
+            const T v = cp[cell];
+            const float e = epair(v);
             const FloatPair q = fp_fma((float)v, bt, aj);
             const float t = __fmul_rn(e, is.h), te = fmaf(e, is.l, fmaf(e, is.h, -t));
             const float g = __fmul_rn(t, q.h);
             gp[cell] = (T)__fadd_rn(g, fmaf(t, q.l, fmaf(te, q.h, fmaf(t, q.h, -g))));
-        } else {
-            const double si = (kF ? (double)expo(v) : exp((double)v * inv_tau - mx)) / S0;
-            gp[cell] = (T)(si * (1.0 + ((double)v - J) * inv_tau));
+        }
+    } else {
+        for (int k = tid; k < ncm; k += blockDim.x) {
+            const int cell = __ldg(cells + k);
+            const T v = cp[cell];
+            gp[cell] = (T)(eplain(v) / S0 * (1.0 + ((double)v - J) * inv_tau));
         }
     }
 }
@@ -724,7 +845,7 @@ __global__ void k_nlpar_weights_d(const float* __restrict__ data, int nrows, int
 // per kDotSlots window slots at a time: g_p is read once for them, and their sums are
 // independent chains (with one slot a warp, the compensated sum's four dependent additions and
 // the loads' latency were the bound).  1024 pixels of 14400 values, radius 2: 340 us before,
-// 276 now.
+// 258 now (the loop unrolled by four: 319).
 constexpr int kDotSlots = 4;
 template <typename T>
 __global__ void __launch_bounds__(256) k_nlpar_dots(const T* __restrict__ g, const T* __restrict__ x, int nrows,
@@ -957,21 +1078,29 @@ int ebsd_linop_create(int64_t nrows, int64_t ncols, const int64_t* rowptr, const
     op->ncols = ncols;
     op->nnz = nnz;
     std::vector<double> v64(val, val + nnz);
+    std::vector<int2> ent((size_t)nnz);
+    for (int64_t e = 0; e < nnz; ++e) {
+        ent[e].x = col[e];
+        std::memcpy(&ent[e].y, &val[e], sizeof(float));
+    }
     bool ok = cudaMalloc((void**)&op->rowptr, (nrows + 1) * sizeof(int64_t)) == cudaSuccess &&
               cudaMalloc((void**)&op->col, std::max<int64_t>(nnz, 1) * sizeof(int32_t)) == cudaSuccess &&
               cudaMalloc((void**)&op->val, std::max<int64_t>(nnz, 1) * sizeof(float)) == cudaSuccess &&
-              cudaMalloc((void**)&op->val64, std::max<int64_t>(nnz, 1) * sizeof(double)) == cudaSuccess;
+              cudaMalloc((void**)&op->val64, std::max<int64_t>(nnz, 1) * sizeof(double)) == cudaSuccess &&
+              cudaMalloc((void**)&op->ent, std::max<int64_t>(nnz, 1) * sizeof(int2)) == cudaSuccess;
     ok = ok && cudaMemcpy(op->rowptr, rowptr, (nrows + 1) * sizeof(int64_t), cudaMemcpyHostToDevice) == cudaSuccess;
     if (ok && nnz > 0) {
         ok = cudaMemcpy(op->col, col, nnz * sizeof(int32_t), cudaMemcpyHostToDevice) == cudaSuccess &&
              cudaMemcpy(op->val, val, nnz * sizeof(float), cudaMemcpyHostToDevice) == cudaSuccess &&
-             cudaMemcpy(op->val64, v64.data(), nnz * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess;
+             cudaMemcpy(op->val64, v64.data(), nnz * sizeof(double), cudaMemcpyHostToDevice) == cudaSuccess &&
+             cudaMemcpy(op->ent, ent.data(), nnz * sizeof(int2), cudaMemcpyHostToDevice) == cudaSuccess;
     }
     if (!ok) {
         cudaFree(op->rowptr);
         cudaFree(op->col);
         cudaFree(op->val);
         cudaFree(op->val64);
+        cudaFree(op->ent);
         delete op;
         return EBSD_E_NOMEM;
     }
@@ -999,16 +1128,24 @@ int ebsd_linop_apply_cols(ebsd_linop_t op, int fp64, const void* d_xT, int64_t l
                           int64_t ldy, void* stream) {
     if (!op || n < 0 || (n > 0 && (!d_xT || !d_yT)) || ldx < n || ldy < n || (n + 31) / 32 > 65535) return EBSD_E_ARG;
     if (n == 0) return EBSD_OK;
-    if ((op->nrows + 7) / 8 > 0x7fffffff) return EBSD_E_ARG;
     if (cudaSetDevice(op->device) != cudaSuccess) return EBSD_E_DEVICE;
-    const dim3 grid((unsigned)((op->nrows + 7) / 8), (unsigned)((n + 31) / 32)), block(32, 8);
+    // without an image the rows stand as one of kCsrTileX columns: a tile is 32 rows in a row
+    const int64_t width = op->width > 0 ? op->width : kCsrTileX;
+    if ((op->nrows + kCsrTileY * width - 1) / (kCsrTileY * width) * ((width + kCsrTileX - 1) / kCsrTileX) > 0x7fffffff) return EBSD_E_ARG;
+    cudaStream_t st = (cudaStream_t)stream;
     if (fp64)
-        k_csr_gather_cols<double><<<grid, block, 0, (cudaStream_t)stream>>>(
-            op->rowptr, op->col, op->val64, (const double*)d_xT, ldx, (double*)d_yT, ldy, op->nrows, n);
+        launch_csr_cols<double>(st, op->rowptr, CsrEnt<double>{op->col, op->val64}, (const double*)d_xT, ldx, (double*)d_yT, ldy,
+                                op->nrows, width, n);
     else
-        k_csr_gather_cols<float><<<grid, block, 0, (cudaStream_t)stream>>>(
-            op->rowptr, op->col, op->val, (const float*)d_xT, ldx, (float*)d_yT, ldy, op->nrows, n);
+        launch_csr_cols<float>(st, op->rowptr, CsrEnt<float>{op->ent}, (const float*)d_xT, ldx, (float*)d_yT, ldy, op->nrows,
+                               width, n);
     return launch_status();
+}
+
+int ebsd_linop_set_width(ebsd_linop_t op, int64_t width) {
+    if (!op || width < 0 || width > op->nrows) return EBSD_E_ARG;
+    op->width = width;
+    return EBSD_OK;
 }
 
 int ebsd_linop_destroy(ebsd_linop_t op) {
@@ -1018,6 +1155,7 @@ int ebsd_linop_destroy(ebsd_linop_t op) {
     cudaFree(op->col);
     cudaFree(op->val);
     cudaFree(op->val64);
+    cudaFree(op->ent);
     delete op;
     return EBSD_OK;
 }

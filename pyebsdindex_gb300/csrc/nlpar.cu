@@ -1009,6 +1009,108 @@ size_t pairs_smem(int sr) {
     return std::max((size_t)2 * (sr + 1) * kChunk * kPairPitch, (size_t)2 * (64 + 4 * sr) * kEdgePitch) * sizeof(float);
 }
 
+// The pair sums of the scan, with sigma's own when asked, and the edge pixels' other window sums.
+int launch_pairs(cudaStream_t st, const float* data, int nrows, int ncols, int npx, const int32_t* ind, int nind,
+                 float datamax, int saturation_protect, int sr, bool with_sigma, float2* pairs, float2* sigp, float2* raw) {
+    const float mxval = saturation_protect ? datamax * 0.999f : datamax + 1.0f;
+    const float mxsig = saturation_protect ? datamax * 0.9961f : datamax + 1.0f;
+    const int edge_rows = edge_blocks(sr, ncols), edge_all = edge_rows + edge_blocks(sr, nrows);
+    const int64_t pgrid = edge_all + (int64_t)((ncols + 2 * kPairLanes - 1) / (2 * kPairLanes)) * nrows;
+    if (pgrid > 0x7fffffff) return EBSD_E_UNSUPPORTED;
+    typedef void (*PairsFn)(const float*, int, int, int, const int32_t*, int, float, float, float, float2*, float2*, int, int,
+                            float2*);
+    PairsFn fn = with_sigma ? (sr == 1 ? k_nlpar_pairs<1, true> : sr == 2 ? k_nlpar_pairs<2, true> : k_nlpar_pairs<3, true>)
+                            : (sr == 1 ? k_nlpar_pairs<1, false> : sr == 2 ? k_nlpar_pairs<2, false> : k_nlpar_pairs<3, false>);
+    const size_t psm = pairs_smem(sr);
+    EBSD_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+    fn<<<(unsigned)pgrid, (unsigned)kPairThreads, psm, st>>>(data, nrows, ncols, npx, ind, nind, mxval, mxsig, 0.0f, pairs,
+                                                             sigp, edge_rows, edge_all, raw);
+    return launch_status();
+}
+
+// ---- the weights with the pieces of their derivative, from the pair sums ----------------------
+// 1024 pixels of 14400 values, radius 2: k_sigma_arg and k_nlpar_weights_d, which sum every pair once
+// for each of its pixels and slots with a serial, uncoalesced pair_ssd, took 1010 + 1165 us; the pair
+// kernel (844, its 32 blocks' serial chains) and these two (6 + 6) take their place at radius 1-3.
+// sigma^2 with the neighbour that attains the minimum and its pair count: k_sigma_arg's scan of the
+// eight neighbours in raster order, the sums read instead of made.
+__global__ void k_nlpar_sigma_arg_pairs(const float2* __restrict__ sigp, int nrows, int ncols, float* __restrict__ sig2,
+                                        int* __restrict__ arg, float* __restrict__ nsig) {
+    const int64_t pix = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (pix >= (int64_t)nrows * ncols) return;
+    const int j = (int)(pix / ncols), i = (int)(pix - (int64_t)j * ncols);
+    float best = 1e24f, bn = 0.0f;
+    int ba = -1;
+    for (int kk = 0; kk < 9; ++kk) {
+        const int dy = kk / 3 - 1, dx = kk % 3 - 1, jn = j + dy, inn = i + dx;
+        if (kk == 4 || jn < 0 || jn >= nrows || inn < 0 || inn >= ncols) continue;
+        const int64_t nb = (int64_t)jn * ncols + inn;
+        // forward neighbours: dx 1 in the same row; dx -1, 0, 1 in the next
+        const float2 e = kk > 4 ? sigp[pix * 4 + (kk == 5 ? 0 : 2 + dx)] : sigp[nb * 4 + (kk == 3 ? 0 : 2 - dx)];
+        const float n2 = __fadd_rn(e.y, 1.0e-12f);
+        if (!(e.x >= 1.e-3f)) continue;
+        const float v = __fdiv_rn(e.x, __fmul_rn(n2, 2.0f));
+        if (v < best) { best = v; ba = (int)nb; bn = n2; }
+    }
+    const float sg = sqrtf(best);
+    sig2[pix] = __fmul_rn(sg, sg);
+    arg[pix] = ba;
+    nsig[pix] = bn;
+}
+
+// k_nlpar_weights_d's arithmetic, one block (64 threads) per scan pixel, a thread per window slot.
+__global__ void k_nlpar_weights_d_pairs(const float2* __restrict__ pairs, const float2* __restrict__ raw, int nrows,
+                                        int ncols, int sr, const float* __restrict__ sig2, float lam2, float dthresh,
+                                        float* __restrict__ wout, float* __restrict__ mout, float* __restrict__ dsout,
+                                        float* __restrict__ dgout) {
+    __shared__ float W[64];
+    __shared__ float T;
+    const int wn = 2 * sr + 1, winsz = wn * wn, nF = fwd_count(sr), c = threadIdx.x;
+    const int64_t pix = blockIdx.x;
+    const int y = (int)(pix / ncols), x = (int)(pix - (int64_t)y * ncols);
+    int ys, ye, xs, xe;
+    window(y, sr, nrows, ys, ye);
+    window(x, sr, ncols, xs, xe);
+    float m = 0.0f, dS = 0.0f, dg = 0.0f;
+    if (c < winsz) {
+        const int dy = ys + c / wn - y, dx = xs + c % wn - x;
+        const int64_t nb = pix + (int64_t)dy * ncols + dx;
+        float w = -1.0e6f;
+        if (nb != pix) {
+            const float2 e = dy < -sr || dy > sr || dx < -sr || dx > sr ? raw[edge_index(y, x, sr, nrows, ncols) * winsz + c]
+                             : (dy > 0 || (dy == 0 && dx > 0)) ? pairs[pix * nF + fwd_index(dy, dx, sr)]
+                                                              : pairs[nb * nF + fwd_index(-dy, -dx, sr)];
+            const float ss = __fadd_rn(sig2[pix], sig2[nb]);
+            const float d2 = __fsub_rn(e.x, __fmul_rn(e.y, ss));
+            const float dnorm = __fmul_rn(ss, sqrtf(__fmul_rn(2.0f, e.y)));
+            if (dnorm > 1.e-8f) {
+                w = __fdiv_rn(d2, dnorm);
+                dS = 1.0f / dnorm;
+                dg = -e.x / (ss * dnorm);
+            } else {
+                w = __fmul_rn(1e6f, e.y);
+            }
+        }
+        m = fmaxf(__fsub_rn(w, dthresh), 0.0f);
+        if (!(w - dthresh > 0.0f)) { dS = 0.0f; dg = 0.0f; }  // clamped: no derivative
+        W[c] = expf(__fmul_rn(__fmul_rn(-1.0f, m), lam2));
+    }
+    __syncthreads();
+    if (c == 0) {
+        float t = 0.0f;
+        for (int k = 0; k < winsz; ++k) t = __fadd_rn(t, W[k]);
+        T = t;
+    }
+    __syncthreads();
+    if (c < winsz) {
+        const int64_t o = pix * winsz + c;
+        wout[o] = __fdiv_rn(W[c], T);
+        mout[o] = m;
+        dsout[o] = dS;
+        dgout[o] = dg;
+    }
+}
+
 size_t tiled_smem(int sr, int ncols, size_t elem, bool weights) {
     const int wn = 2 * sr + 1;
     const int ncx = std::min(ncols, kTileX + 4 * sr);
@@ -1275,10 +1377,9 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
         nind < 0 || nind > npx || sr < 1 || sr > 3 || !(lam > 0.0f))
         return EBSD_E_ARG;
     if (2 * sr + 1 > nrows || 2 * sr + 1 > ncols) return EBSD_E_ARG;  // window must fit the scan
-    const size_t psm = pairs_smem(sr), asm_ = tiled_smem(sr, ncols, sizeof(float), false);
+    const size_t asm_ = tiled_smem(sr, ncols, sizeof(float), false);
     if (asm_ > 48 * 1024) return EBSD_E_UNSUPPORTED;
     const float mxval = saturation_protect ? datamax * 0.999f : datamax + 1.0f;
-    const float mxsig = saturation_protect ? datamax * 0.9961f : datamax + 1.0f;
     const float lam2 = 1.0f / (lam * lam);
     const int64_t npix = (int64_t)nrows * ncols;
     const int winsz = (2 * sr + 1) * (2 * sr + 1), nF = sr * (2 * sr + 1) + sr;
@@ -1290,17 +1391,8 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
     float2* sigp = pairs + npix * nF;
     cudaStream_t st = (cudaStream_t)stream;
     float2* raw = sigp + npix * 4;  // the edge pixels' window sums that are no pair sums
-    const int edge_rows = edge_blocks(sr, ncols), edge_all = edge_rows + edge_blocks(sr, nrows);
-    const int64_t pgrid = edge_all + (int64_t)((ncols + 2 * kPairLanes - 1) / (2 * kPairLanes)) * nrows;
-    if (pgrid > 0x7fffffff) return EBSD_E_UNSUPPORTED;
-    typedef void (*PairsFn)(const float*, int, int, int, const int32_t*, int, float, float, float, float2*, float2*, int, int,
-                            float2*);
-    PairsFn fn = compute_sigma ? (sr == 1 ? k_nlpar_pairs<1, true> : sr == 2 ? k_nlpar_pairs<2, true> : k_nlpar_pairs<3, true>)
-                               : (sr == 1 ? k_nlpar_pairs<1, false> : sr == 2 ? k_nlpar_pairs<2, false> : k_nlpar_pairs<3, false>);
-    EBSD_CUDA_TRY(cudaFuncSetAttribute((const void*)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
-    fn<<<(unsigned)pgrid, (unsigned)kPairThreads, psm, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, mxsig, 0.0f,
-                                                             pairs, sigp, edge_rows, edge_all, raw);
-    int rc = launch_status();
+    int rc = launch_pairs(st, d_data, nrows, ncols, npx, d_indices, nind, datamax, saturation_protect, sr, compute_sigma != 0,
+                          pairs, sigp, raw);
     if (rc != EBSD_OK) return rc;
     if (compute_sigma) {
         k_nlpar_sigma_pairs<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(sigp, nrows, ncols, d_sigma);
@@ -1324,6 +1416,38 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
         launch_average<uint16_t>(tgrid, tblock, asm_, st, d_data, nrows, ncols, npx, w, sr, (uint16_t*)d_out);
     else
         launch_average<float>(tgrid, tblock, asm_, st, d_data, nrows, ncols, npx, w, sr, (float*)d_out);
+    return launch_status();
+}
+
+int64_t ebsd_nlpar_sigma_weights_d_work(int32_t nrows, int32_t ncols, int32_t sr) {
+    if (nrows <= 0 || ncols <= 0 || sr < 1 || sr > 3 || 2 * sr + 1 > nrows || 2 * sr + 1 > ncols) return 0;
+    const int64_t npix = (int64_t)nrows * ncols, nedge = (int64_t)2 * sr * (ncols + nrows - 2 * sr);
+    return 2 * (npix * (sr * (2 * sr + 1) + sr + 4) + nedge * (2 * sr + 1) * (2 * sr + 1));
+}
+
+int ebsd_nlpar_sigma_weights_d(const float* d_data, int32_t nrows, int32_t ncols, int32_t npx, const int32_t* d_indices,
+                               int32_t nind, float datamax, float lam, int32_t sr, float dthresh, int compute_sigma,
+                               int saturation_protect, float* d_work, float* d_sig2, int32_t* d_arg, float* d_nsig,
+                               float* d_w, float* d_m, float* d_dS, float* d_dsig, void* stream) {
+    if (!d_data || !d_indices || !d_work || (uintptr_t)d_work % 8 != 0 || !d_sig2 || !d_w || !d_m || !d_dS || !d_dsig ||
+        (compute_sigma && (!d_arg || !d_nsig)) || nrows <= 0 || ncols <= 0 || npx <= 0 || nind < 0 || nind > npx || sr < 1 ||
+        sr > 3 || !(lam > 0.0f) || 2 * sr + 1 > nrows || 2 * sr + 1 > ncols)
+        return EBSD_E_ARG;
+    const int64_t npix = (int64_t)nrows * ncols;
+    if (npix > 0x7fffffff) return EBSD_E_ARG;
+    float2* pairs = (float2*)d_work;
+    float2* sigp = pairs + npix * (sr * (2 * sr + 1) + sr);
+    float2* raw = sigp + npix * 4;
+    cudaStream_t st = (cudaStream_t)stream;
+    int rc = launch_pairs(st, d_data, nrows, ncols, npx, d_indices, nind, datamax, saturation_protect, sr, compute_sigma != 0,
+                          pairs, sigp, raw);
+    if (rc != EBSD_OK) return rc;
+    if (compute_sigma) {
+        k_nlpar_sigma_arg_pairs<<<(unsigned)((npix + 255) / 256), 256, 0, st>>>(sigp, nrows, ncols, d_sig2, d_arg, d_nsig);
+        if ((rc = launch_status()) != EBSD_OK) return rc;
+    }
+    k_nlpar_weights_d_pairs<<<(unsigned)npix, 64, 0, st>>>(pairs, raw, nrows, ncols, sr, d_sig2, 1.0f / (lam * lam), dthresh,
+                                                           d_w, d_m, d_dS, d_dsig);
     return launch_status();
 }
 

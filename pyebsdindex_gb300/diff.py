@@ -43,6 +43,7 @@ def _bind():
         lib.ebsd_linop_create.argtypes = [C.c_int64, C.c_int64, P, P, P, C.c_int, C.POINTER(P)]
         lib.ebsd_linop_apply.argtypes = [P, C.c_int, P, C.c_int64, P, P]
         lib.ebsd_linop_apply_cols.argtypes = [P, C.c_int, P, C.c_int64, C.c_int64, P, C.c_int64, P]
+        lib.ebsd_linop_set_width.argtypes = [P, C.c_int64]
         lib.ebsd_linop_destroy.argtypes = [P]
         lib.ebsd_nlpar_weights.argtypes = [P, C.c_int32, C.c_int32, C.c_int32, P, C.c_int32, C.c_float, C.c_float,
                                            C.c_int32, C.c_float, P, C.c_int, P, P, P]
@@ -59,10 +60,16 @@ def _bind():
                                              C.c_float, C.c_int32, C.c_float, P, C.c_int, P, P, P, P, P]
         lib.ebsd_nlpar_weights_grad.argtypes = [C.c_int, P, P, C.c_int32, C.c_int32, C.c_int32, C.c_int32, P, P, P,
                                                 P, C.c_double, P, C.c_float, C.c_int, P, P, P, P, P, P]
+        lib.ebsd_nlpar_sigma_weights_d_work.argtypes = [C.c_int32, C.c_int32, C.c_int32]
+        lib.ebsd_nlpar_sigma_weights_d_work.restype = C.c_int64
+        lib.ebsd_nlpar_sigma_weights_d.argtypes = [P, C.c_int32, C.c_int32, C.c_int32, P, C.c_int32, C.c_float,
+                                                   C.c_float, C.c_int32, C.c_float, C.c_int, C.c_int, P, P, P, P, P, P,
+                                                   P, P, P]
+        lib.ebsd_nlpar_sigma_weights_d.restype = C.c_int
         lib.ebsd_nlpar_apply64.argtypes = lib.ebsd_nlpar_apply.argtypes
         lib.ebsd_nlpar_apply_t64.argtypes = lib.ebsd_nlpar_apply_t.argtypes
         lib.ebsd_nlpar_lambda_grad64.argtypes = lib.ebsd_nlpar_lambda_grad.argtypes
-        for f in ("ebsd_linop_create", "ebsd_linop_apply", "ebsd_linop_apply_cols", "ebsd_linop_destroy",
+        for f in ("ebsd_linop_create", "ebsd_linop_apply", "ebsd_linop_apply_cols", "ebsd_linop_set_width", "ebsd_linop_destroy",
                   "ebsd_nlpar_weights",
                   "ebsd_nlpar_apply", "ebsd_nlpar_apply_t", "ebsd_nlpar_lambda_grad", "ebsd_nlpar_apply64",
                   "ebsd_nlpar_apply_t64", "ebsd_nlpar_lambda_grad64", "ebsd_blur1d", "ebsd_softargmax",
@@ -146,9 +153,10 @@ def transpose_csr(rowptr, col, val, shape):
 
 
 class LinOp:
-    """A device CSR operator (ebsd_linop)."""
+    """A device CSR operator (ebsd_linop).  ``width``: the row length of the image that the
+    operator's rows index (0: none), where rows that meet the same columns lie close together."""
 
-    def __init__(self, rowptr, col, val, shape, device=0):
+    def __init__(self, rowptr, col, val, shape, device=0, width=0):
         lib = _bind()
         self._lib = lib
         self.rowptr = np.ascontiguousarray(rowptr, np.int64)
@@ -159,6 +167,7 @@ class LinOp:
         _lib.check(lib.ebsd_linop_create(self.shape[0], self.shape[1], self.rowptr.ctypes.data, self.col.ctypes.data,
                                          self.val.ctypes.data, int(device), C.byref(h)), "ebsd_linop_create")
         self.handle = h
+        _lib.check(lib.ebsd_linop_set_width(h, int(width)), "ebsd_linop_set_width")
 
     def __call__(self, x):
         """y = A x for a batch x [n, ncols] (float32 / float64 CUDA tensor) -> y [n, nrows], run
@@ -239,13 +248,10 @@ def _nlpar_fn():
             x32 = xd.to(torch.float32).contiguous()
             npx = x32.shape[1]
             dev = x.device
+            sig2 = torch.empty(npix, dtype=torch.float32, device=dev)
             if sigma is None:
-                sig2 = torch.empty(npix, dtype=torch.float32, device=dev)
                 arg = torch.empty(npix, dtype=torch.int32, device=dev)
                 nsig = torch.empty(npix, dtype=torch.float32, device=dev)
-                _lib.check(lib.ebsd_nlpar_sigma_arg(x32.data_ptr(), nrows, ncols, npx, ind.data_ptr(), ind.numel(),
-                                                    float(datamax), int(sat), sig2.data_ptr(), arg.data_ptr(),
-                                                    nsig.data_ptr(), st), "ebsd_nlpar_sigma_arg")
             else:
                 s32 = sigma.detach().to(torch.float32).reshape(-1).contiguous()
                 sig2 = (s32 * s32).contiguous()
@@ -254,10 +260,23 @@ def _nlpar_fn():
             w = torch.empty((npix, winsz), dtype=torch.float32, device=dev)
             m, dS, dsg = torch.empty_like(w), torch.empty_like(w), torch.empty_like(w)
             lamf = float(lam.detach().cpu())
-            _lib.check(lib.ebsd_nlpar_weights_d(x32.data_ptr(), nrows, ncols, npx, ind.data_ptr(), ind.numel(),
-                                                float(datamax), lamf, sr, float(dthresh), sig2.data_ptr(), int(sat),
-                                                w.data_ptr(), m.data_ptr(), dS.data_ptr(), dsg.data_ptr(), st),
-                       "ebsd_nlpar_weights_d")
+            nwork = int(lib.ebsd_nlpar_sigma_weights_d_work(nrows, ncols, sr))
+            if nwork > 0:  # radius 1-3: each pair's distance summed once
+                work = torch.empty(nwork, dtype=torch.float32, device=dev)
+                _lib.check(lib.ebsd_nlpar_sigma_weights_d(x32.data_ptr(), nrows, ncols, npx, ind.data_ptr(), ind.numel(),
+                                                          float(datamax), lamf, sr, float(dthresh), int(sigma is None),
+                                                          int(sat), work.data_ptr(), sig2.data_ptr(), arg.data_ptr(),
+                                                          nsig.data_ptr(), w.data_ptr(), m.data_ptr(), dS.data_ptr(),
+                                                          dsg.data_ptr(), st), "ebsd_nlpar_sigma_weights_d")
+            else:
+                if sigma is None:
+                    _lib.check(lib.ebsd_nlpar_sigma_arg(x32.data_ptr(), nrows, ncols, npx, ind.data_ptr(), ind.numel(),
+                                                        float(datamax), int(sat), sig2.data_ptr(), arg.data_ptr(),
+                                                        nsig.data_ptr(), st), "ebsd_nlpar_sigma_arg")
+                _lib.check(lib.ebsd_nlpar_weights_d(x32.data_ptr(), nrows, ncols, npx, ind.data_ptr(), ind.numel(),
+                                                    float(datamax), lamf, sr, float(dthresh), sig2.data_ptr(), int(sat),
+                                                    w.data_ptr(), m.data_ptr(), dS.data_ptr(), dsg.data_ptr(), st),
+                           "ebsd_nlpar_weights_d")
             y = torch.empty_like(xd)
             if xd.dtype == torch.float64:
                 w64 = w.to(torch.float64)
@@ -406,9 +425,12 @@ class BandSharpness:
         self.bg_radius = bg_radius if bg_radius is not None else max(3, min(H, W) // 4)
         self.dev = torch.device("cuda", device)
         r = radon_csr(bd)
-        self.R, self.RT = LinOp(*r, device=device), LinOp(*transpose_csr(*r), device=device)
+        nT = int(bd.radonPlan.nTheta)
+        self.R = LinOp(*r, device=device, width=nT)
+        self.RT = LinOp(*transpose_csr(*r), device=device, width=W)
         m = log_csr(bd)
-        self.M, self.MT = LinOp(*m, device=device), LinOp(*transpose_csr(*m), device=device)
+        self.M = LinOp(*m, device=device, width=nT)
+        self.MT = LinOp(*transpose_csr(*m), device=device, width=nT)
         self.rmask = torch.as_tensor(np.asarray(bd.rdnmask).reshape(-1), device=self.dev)
         self.cells = torch.as_tensor(np.nonzero(np.asarray(bd.rdnmask).reshape(-1))[0].astype(np.int32), device=self.dev)
         from .nlpar import NLPAR

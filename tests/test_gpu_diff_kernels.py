@@ -203,3 +203,52 @@ def test_weights_grad(cuda, nr, nc, npx, sr, f64):
             pair(arg[p], p, gam[p] / nsig[p], egam[p] / nsig[p], mxs)
     tol += (terms[:, None] + 1) * u * mag
     assert np.all(np.abs(gx.cpu().numpy() - want) <= 1.01 * tol + 1e-12 * mag)
+
+
+@pytest.mark.parametrize("nr,nc,npx,nind,sr", [(3, 3, 5, 5, 1), (4, 7, 1025, 900, 1), (5, 5, 64, 33, 2), (6, 70, 130, 65, 2),
+                                               (7, 8, 77, 31, 3), (9, 61, 300, 96, 3), (35, 7, 40, 1, 3), (5, 6, 9, 0, 2)])
+@pytest.mark.parametrize("given", [False, True])
+def test_sigma_weights_equal_the_pairwise_kernels(cuda, nr, nc, npx, nind, sr, given):
+    """Bit for bit, with saturated values and a NaN among the patterns."""
+    import torch
+    from pyebsdindex_gb300 import _lib
+    lib, g, n, ws = diff._bind(), np.random.default_rng(npx), nr * nc, (2 * sr + 1) ** 2
+    x = g.integers(0, 201, size=(n, npx)).astype(np.float32)
+    x[n // 2, npx // 2] = np.nan
+    xt = torch.from_numpy(x).to(cuda)
+    ind = torch.from_numpy(np.sort(g.permutation(npx)[:nind]).astype(np.int32)).to(cuda)
+    ip = (ind if nind else torch.zeros(1, dtype=torch.int32, device=cuda)).data_ptr()
+    st = torch.cuda.current_stream().cuda_stream
+
+    def outs():
+        sig2 = torch.full((n,), 3.0, device=cuda)
+        return [sig2, torch.zeros(n, dtype=torch.int32, device=cuda), torch.zeros(n, device=cuda)] + [
+            torch.zeros((n, ws), device=cuda) for _ in range(4)]
+    a, b = outs(), outs()
+    if not given:
+        _lib.check(lib.ebsd_nlpar_sigma_arg(xt.data_ptr(), nr, nc, npx, ip, nind, 200.0, 1,
+                                            *(t.data_ptr() for t in a[:3]), st), "sigma_arg")
+    _lib.check(lib.ebsd_nlpar_weights_d(xt.data_ptr(), nr, nc, npx, ip, nind, 200.0, 0.9, sr, 0.1, a[0].data_ptr(), 1,
+                                        *(t.data_ptr() for t in a[3:]), st), "weights_d")
+    work = torch.empty(int(lib.ebsd_nlpar_sigma_weights_d_work(nr, nc, sr)), device=cuda)
+    _lib.check(lib.ebsd_nlpar_sigma_weights_d(xt.data_ptr(), nr, nc, npx, ip, nind, 200.0, 0.9, sr, 0.1, int(not given),
+                                              1, work.data_ptr(), *(t.data_ptr() for t in b), st), "sigma_weights_d")
+    for s, t in zip(a, b):
+        assert torch.equal(s.view(torch.int32), t.view(torch.int32))
+
+
+@pytest.mark.parametrize("nrows,ncols,width", [(1, 1, 0), (1, 7, 1), (37, 50, 0), (61 * 9, 300, 61), (64, 20, 8), (35, 64, 5),
+                                               (33, 12, 33)])
+@pytest.mark.parametrize("f64", [False, True])
+def test_linop_tiles_equal_rows(cuda, nrows, ncols, width, f64):
+    """Tiles of neighbouring rows, ragged row lengths and empty rows: the same bits as a thread a row."""
+    import torch
+    g = np.random.default_rng(nrows)
+    cnt = g.integers(0, min(ncols, 40) + 1, size=nrows)
+    cnt[nrows // 2] = 0
+    rowptr = np.concatenate([[0], np.cumsum(cnt)])
+    col = np.concatenate([np.sort(g.permutation(ncols)[:c]) for c in cnt] + [[]]).astype(np.int32)
+    op = diff.LinOp(rowptr, col, g.normal(size=len(col)).astype(np.float32), (nrows, ncols), width=width)
+    for n in (1, 31, 33, 64, 65, 127, 130, 257):
+        x = torch.from_numpy(g.normal(size=(n, ncols))).to(cuda, torch.float64 if f64 else torch.float32)
+        assert torch.equal(op(x), op.apply_rows(x)), n
