@@ -15,8 +15,16 @@
 //   * the vote's library test |T - a| <= angTol (float64, T a library angle, a a float32 band
 //     angle) becomes a <= / >= test against the float32 interval of a that passes it, computed
 //     once per library on the host;
-//   * the warp tests 32 library triplets at once and applies the matches one by one in library
-//     order, so that every float32 vote sum adds in the reference's order.
+//   * a lane tests one band triplet against the library rows that can hold it, 32 triplets at
+//     once; the warp lists the matches in triplet and library order, a lane takes one match's
+//     weights, and the votes are cast in that order with a lane per band, so that every float32
+//     vote sum adds in the reference's order.
+//   * the TRIAD candidates of a band pair are tried several at once, a lane per candidate and
+//     band, and the first of the best scores is kept, as a scan in order would keep it.
+// What bounds the kernel is instructions issued.  FCC library (167 triplets, 50 poles), nine
+// bands: 84 band triplets, 85 matches and 14 candidates a pattern cost 63,800 warp instructions
+// with a warp per triplet, lane 0 casting the votes and a candidate at a time, and 15.2 ms per
+// 200,000 patterns; 18,900 and 6.0 ms now.
 #include "ebsd_internal.cuh"
 
 #include <algorithm>
@@ -34,9 +42,9 @@ struct ebsd_vote_plan_s {
     float* d_iv = nullptr;        // [6][ntrip] acceptance intervals lo0, hi0, lo1, hi1, lo2, hi2, rows sorted by lo0
     uint32_t* d_tfam = nullptr;   // [ntrip] f0 | f1 << 8 | f2 << 16
     double* d_tang = nullptr;     // [ntrip][3]
-    float* d_pole = nullptr;      // [3][npoles] float32 poles, component-major
+    float* d_pole = nullptr;      // [npoles][4] float32 poles with their family (int bits)
+    float* d_triad = nullptr;     // [nfam][npoles][8] TRIAD frame of (family's first pole, pole)
     double* d_pole64 = nullptr;   // [npoles][3]
-    int32_t* d_pfam = nullptr;    // [npoles]
     double* d_angtab = nullptr;   // [npoles][npoles]
     int32_t* d_famcnt = nullptr;  // [nfam]
     int32_t* d_famidx = nullptr;  // [nfam]
@@ -53,7 +61,7 @@ namespace ebsd {
 namespace {
 
 constexpr int kWarps = 8;
-constexpr int kList = 96;  // matches of one band triplet held for sorting into library order
+constexpr int kList = 160;  // matches held at once for casting in triplet and library order
 constexpr unsigned kFull = 0xffffffffu;
 constexpr double kRadeg = 57.29577951308232;  // 180 / pi
 constexpr float kRadegF = 57.29577951308232f;
@@ -73,8 +81,8 @@ struct VoteArgs {
     const uint32_t* tfam;
     const double* tang;
     const float* pole;
+    const float* triad;
     const double* pole64;
-    const int32_t* pfam;
     const double* angtab;
     const int32_t* famcnt;
     const int32_t* famidx;
@@ -164,22 +172,22 @@ __device__ __forceinline__ float acos_deg(float x) {
     return __fmul_rn(acosf(x), kRadegF);
 }
 
-__device__ __forceinline__ void sort3(const float* v, int& s0, int& s1, int& s2) {
-    int s[3] = {0, 1, 2};
-    int t;
-    if (v[s[0]] > v[s[2]]) { t = s[2]; s[2] = s[0]; s[0] = t; }
-    if (v[s[0]] > v[s[1]]) { t = s[1]; s[1] = s[0]; s[0] = t; }
-    if (v[s[1]] > v[s[2]]) { t = s[2]; s[2] = s[1]; s[1] = t; }
-    s0 = s[0]; s1 = s[1]; s2 = s[2];
-}
-
-__device__ __forceinline__ void sort3i(const int* v, int& s0, int& s1, int& s2) {
-    int s[3] = {0, 1, 2};
-    int t;
-    if (v[s[0]] > v[s[2]]) { t = s[2]; s[2] = s[0]; s[0] = t; }
-    if (v[s[0]] > v[s[1]]) { t = s[1]; s[1] = s[0]; s[0] = t; }
-    if (v[s[1]] > v[s[2]]) { t = s[2]; s[2] = s[1]; s[1] = t; }
-    s0 = s[0]; s1 = s[1]; s2 = s[2];
+// Sorts (v0, v1, v2) with the reference's exchanges; s0, s1, s2: where the sorted values were.
+template <class T>
+__device__ __forceinline__ void sort3(T& v0, T& v1, T& v2, int& s0, int& s1, int& s2) {
+    auto order = [](T& a, T& b, int& i, int& j) {
+        const bool x = a > b;
+        const T t = a;
+        const int k = i;
+        a = x ? b : a;
+        i = x ? j : i;
+        b = x ? t : b;
+        j = x ? k : j;
+    };
+    s0 = 0; s1 = 1; s2 = 2;
+    order(v0, v2, s0, s2);
+    order(v0, v1, s0, s1);
+    order(v1, v2, s1, s2);
 }
 
 __device__ __forceinline__ double np_maximum(double a, double b) {  // NaN-propagating
@@ -192,37 +200,31 @@ __host__ __device__ inline size_t align8(size_t words) { return (words + 1) & ~s
 
 // 4-byte words of one warp's region
 __host__ __device__ inline size_t warp_words(int nb, int nfam) {
-    return align8(3 * size_t(nb) + nb + nb * nb + 2 * size_t(nfam) * nb + nb + nb + 64 + kList);
+    return align8(3 * size_t(nb) + nb + nb * nb + 2 * size_t(nfam) * nb + nb + nb + kList);
 }
 
 __host__ __device__ inline size_t block_words(int ntrip, int npoles) {
     return align8(6 * size_t(ntrip) + ntrip + 3 * size_t(npoles) + npoles);
 }
 
-// Warp-cooperative search on a monotone predicate (true for a leading run of [0, n), then
-// false): the length of the run.  32-way: each round samples 32 evenly spaced indices.
+// Length of the run of [0, n) on which a monotone predicate holds.
 template <class P>
-__device__ __forceinline__ int warp_count_leading(int n, int lane, P pred) {
-    int lo = 0, hi = n;  // the answer lies in [lo, hi]
-    while (hi - lo > 32) {
-        const int step = (hi - lo + 31) / 32;
-        const int idx = lo + lane * step;
-        const int c = __popc(__ballot_sync(kFull, idx < hi && pred(idx)));
-        if (c == 0) return lo;
-        const int nlo = lo + (c - 1) * step + 1;
-        hi = min(hi, lo + c * step);
-        lo = nlo;
+__device__ __forceinline__ int count_leading(int n, P pred) {
+    int lo = 0, hi = n;
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (pred(mid)) lo = mid + 1;
+        else hi = mid;
     }
-    const int idx = lo + lane;
-    return lo + __popc(__ballot_sync(kFull, idx < hi && pred(idx)));
+    return lo;
 }
 
 // ---------------------------------------------------------------------------------------
 __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const float* s_iv,
-                              const int* s_orig, const float* s_pole, const int* s_pfam,
-                              float* w) {
+                              const int* s_orig, const float4* s_pole, float* w) {
     const int nb = A.nb, nfam = A.nfam, ntrip = A.ntrip, npoles = A.npoles;
     const float tolf = A.tol_f;
+    auto pole_family = [s_pole](int P) { return __float_as_int(s_pole[P].w); };
     float* bn = w;                       // [nb][3]
     float* inten = bn + 3 * nb;          // [nb]
     float* ang = inten + nb;             // [nb][nb]
@@ -230,8 +232,8 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     float* accn = accw + nfam * nb;      // [nfam][nb]
     int* rarg = (int*)(accn + nfam * nb);  // [nb] band order, ascending rank
     int* bfam = rarg + nb;               // [nb]
-    float* fscr = (float*)(bfam + nb);   // [64]
-    int* mlist = (int*)(fscr + 64);      // [kList]
+    int* mlist = bfam + nb;              // [kList] matches: triplet lane << 16 | library index
+    float* fscr = (float*)mlist;         // [32] band fits (after the vote)
     const unsigned lt_mask = (1u << lane) - 1u;
 
     for (int t = lane; t < 3 * nb; t += 32) bn[t] = A.norms[p * 3 * nb + t];
@@ -258,96 +260,157 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     __syncwarp();
 
     // ---- triplet vote, tripletvote.py:1023-1135 ----
-    for (int i = 0; i < nb; ++i) {
-        if (inten[i] < 1e-6f) continue;  // all its angles are 10000: no library triplet matches
-        for (int j = i + 1; j < nb; ++j) {
-            if (inten[j] < 1e-6f) continue;
-            for (int k = j + 1; k < nb; ++k) {
-                if (inten[k] < 1e-6f) continue;
-                float x[3] = {ang[i * nb + j], ang[i * nb + k], ang[j * nb + k]};
-                int s0, s1, s2;
-                sort3(x, s0, s1, s2);
-                const int code = A.lut[s0 * 9 + s1 * 3 + s2];
-                const int r[3] = {code & 3, (code >> 2) & 3, (code >> 4) & 3};
-                int u0, u1, u2;
-                sort3i(r, u0, u1, u2);
-                const float a0 = x[s0], a1 = x[s1], a2 = x[s2];
-                const bool e1 = fabsf(__fsub_rn(a0, a1)) < tolf;
-                const bool e2 = fabsf(__fsub_rn(a1, a2)) < tolf;
-                const bool e3 = fabsf(__fsub_rn(a2, a0)) < tolf;
-                // library entries whose first-angle interval can hold a0: sorted by its lower
-                // end, so [s, e) with lo0 in [a0 - win, a0]
-                const float tgt = a0 - A.win;
-                const int e = warp_count_leading(ntrip, lane, [&](int q) { return s_iv[q] <= a0; });
-                const int s = warp_count_leading(e, lane, [&](int q) { return s_iv[q] < tgt; });
-                auto test = [&](int q) {
-                    return a0 >= s_iv[q] && a0 <= s_iv[ntrip + q] && a1 >= s_iv[2 * ntrip + q] &&
-                           a1 <= s_iv[3 * ntrip + q] && a2 >= s_iv[4 * ntrip + q] && a2 <= s_iv[5 * ntrip + q];
-                };
-                // one match, in the reference's library order (lane 0 applies them all)
-                auto apply = [&](int q) {
-                    const double* T = A.tang + 3 * (size_t)q;
-                    const float t0 = __double2float_rn(fabs(__dsub_rn(T[0], (double)a0)));
-                    const float t1 = __double2float_rn(fabs(__dsub_rn(T[1], (double)a1)));
-                    const float t2 = __double2float_rn(fabs(__dsub_rn(T[2], (double)a2)));
-                    const uint32_t fw = A.tfam[q];
-                    const int fq[3] = {int(fw & 255u), int((fw >> 8) & 255u), int((fw >> 16) & 255u)};
-                    const int f0 = fq[u0], f1 = fq[u1], f2 = fq[u2];
-                    const float w1 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t0, t1)));
-                    const float w2 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t0, t2)));
-                    const float w3 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t1, t2)));
-                    auto vote = [&](int f, int b, float wt) {
-                        accw[f * nb + b] = __fadd_rn(accw[f * nb + b], wt);
-                        accn[f * nb + b] = __fadd_rn(accn[f * nb + b], 1.0f);
-                    };
-                    vote(f0, i, w1); vote(f1, j, w2); vote(f2, k, w3);
-                    if (e1) { vote(f0, j, w1); vote(f1, i, w2); vote(f2, k, w3); }
-                    if (e2) { vote(f0, i, w1); vote(f1, k, w2); vote(f2, j, w3); }
-                    if (e3) { vote(f0, k, w1); vote(f1, j, w2); vote(f2, i, w3); }
-                    if (e1 && e2 && e3) {
-                        vote(f0, k, w1); vote(f1, i, w2); vote(f2, j, w3);
-                        vote(f0, j, w1); vote(f1, k, w2); vote(f2, i, w3);
-                    }
-                };
-                int cnt = 0;
-                for (int base = s; base < e; base += 32) {
-                    const int q = base + lane;
-                    const bool hit = q < e && test(q);
-                    const unsigned m = __ballot_sync(kFull, hit);
-                    if (hit && cnt + __popc(m & lt_mask) < kList) mlist[cnt + __popc(m & lt_mask)] = s_orig[q];
-                    cnt += __popc(m);
-                }
-                __syncwarp();
-                if (cnt <= kList) {
-                    if (lane == 0) {
-                        for (int a = 1; a < cnt; ++a) {  // insertion sort into library order
-                            const int v = mlist[a];
-                            int b = a - 1;
-                            while (b >= 0 && mlist[b] > v) {
-                                mlist[b + 1] = mlist[b];
-                                --b;
-                            }
-                            mlist[b + 1] = v;
-                        }
-                        for (int a = 0; a < cnt; ++a) apply(mlist[a]);
-                    }
-                } else {
-                    // more matches than the list holds: take them one at a time, smallest
-                    // library index above the last one applied
-                    int last = -1;
-                    while (true) {
-                        int mine = INT_MAX;
-                        for (int q = s + lane; q < e; q += 32)
-                            if (test(q) && s_orig[q] > last && s_orig[q] < mine) mine = s_orig[q];
-                        const int next = __reduce_min_sync(kFull, mine);
-                        if (next == INT_MAX) break;
-                        if (lane == 0) apply(next);
-                        last = next;
-                        __syncwarp();
-                    }
-                }
-                __syncwarp();
+    // a match's votes, cast by the lanes of its three bands, each into its own column: meta holds
+    // the bands i, j, k (5 bits each), the families f0, f1, f2 (4 bits each) and e1, e2, e3
+    auto cast = [&](unsigned meta, float w1, float w2, float w3) {
+        const bool ri = lane == (int)(meta & 31u), rj = lane == (int)((meta >> 5) & 31u);
+        if (!(ri || rj || lane == (int)((meta >> 10) & 31u))) return;
+        const int f0 = (meta >> 15) & 15u, f1 = (meta >> 19) & 15u, f2 = (meta >> 23) & 15u;
+        auto vote = [&](int role) {  // 0: (f0, w1), 1: (f1, w2), 2: (f2, w3)
+            const int t = (role == 0 ? f0 : role == 1 ? f1 : f2) * nb + lane;
+            accw[t] = __fadd_rn(accw[t], role == 0 ? w1 : role == 1 ? w2 : w3);
+            accn[t] = __fadd_rn(accn[t], 1.0f);
+        };
+        vote(ri ? 0 : rj ? 1 : 2);
+        const unsigned ee = meta >> 27;
+        if (ee & 1u) vote(ri ? 1 : rj ? 0 : 2);
+        if (ee & 2u) vote(ri ? 0 : rj ? 2 : 1);
+        if (ee & 4u) vote(ri ? 2 : rj ? 1 : 0);
+        if (ee == 7u) {
+            vote(ri ? 1 : rj ? 2 : 0);
+            vote(ri ? 2 : rj ? 0 : 1);
+        }
+    };
+    // the weights and families of library triplet q for a band triplet (angles a0..a2; tri: its
+    // bands, the library's family order as 2-bit fields from bit 15, e1..e3 from bit 27)
+    auto weigh = [&](int q, float a0, float a1, float a2, unsigned tri, float& w1, float& w2, float& w3) -> unsigned {
+        const double* T = A.tang + 3 * (size_t)q;
+        const float t0 = __double2float_rn(fabs(__dsub_rn(T[0], (double)a0)));
+        const float t1 = __double2float_rn(fabs(__dsub_rn(T[1], (double)a1)));
+        const float t2 = __double2float_rn(fabs(__dsub_rn(T[2], (double)a2)));
+        const uint32_t fw = A.tfam[q];
+        w1 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t0, t1)));
+        w2 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t0, t2)));
+        w3 = __fsub_rn(tolf, __fmul_rn(0.5f, __fadd_rn(t1, t2)));
+        const unsigned f0 = (fw >> (8 * ((tri >> 15) & 3u))) & 15u, f1 = (fw >> (8 * ((tri >> 17) & 3u))) & 15u;
+        const unsigned f2 = (fw >> (8 * ((tri >> 19) & 3u))) & 15u;
+        return (tri & 0x38007fffu) | f0 << 15 | f1 << 19 | f2 << 23;
+    };
+    const int nt3 = nb * (nb - 1) * (nb - 2) / 6;
+    for (int t0 = 0; t0 < nt3; t0 += 32) {
+        // this lane's band triplet i < j < k, in the order of the nested loops over them
+        int i = 0, j, k;
+        {
+            int r = t0 + lane < nt3 ? t0 + lane : 0, c = (nb - 1) * (nb - 2) / 2;
+            while (r >= c) {
+                r -= c;
+                ++i;
+                c -= nb - 1 - i;
             }
+            j = i + 1;
+            c = nb - 1 - j;
+            while (r >= c) {
+                r -= c;
+                ++j;
+                --c;
+            }
+            k = j + 1 + r;
+        }
+        // (a band without intensity has angles 10000: no library triplet matches)
+        const bool on = t0 + lane < nt3 && !(inten[i] < 1e-6f) && !(inten[j] < 1e-6f) && !(inten[k] < 1e-6f);
+        float a0 = ang[i * nb + j], a1 = ang[i * nb + k], a2 = ang[j * nb + k];
+        int s0, s1, s2, u0, u1, u2;
+        sort3(a0, a1, a2, s0, s1, s2);
+        const int code = A.lut[s0 * 9 + s1 * 3 + s2];
+        int r0 = code & 3, r1 = (code >> 2) & 3, r2 = (code >> 4) & 3;
+        sort3(r0, r1, r2, u0, u1, u2);
+        unsigned tri = (unsigned)(i | j << 5 | k << 10 | u0 << 15 | u1 << 17 | u2 << 19);
+        tri |= (fabsf(__fsub_rn(a0, a1)) < tolf ? 1u << 27 : 0u) | (fabsf(__fsub_rn(a1, a2)) < tolf ? 2u << 27 : 0u) |
+               (fabsf(__fsub_rn(a2, a0)) < tolf ? 4u << 27 : 0u);
+        // library rows whose first-angle interval can hold a0: sorted by its lower end, so
+        // [s, e) with lo0 in [a0 - win, a0]
+        const float tgt = a0 - A.win;
+        const int e = on ? count_leading(ntrip, [&](int q) { return s_iv[q] <= a0; }) : 0;
+        const int s = count_leading(e, [&](int q) { return s_iv[q] < tgt; });
+        auto test = [&](int q) {
+            return a1 >= s_iv[2 * ntrip + q] && a1 <= s_iv[3 * ntrip + q] && a0 >= s_iv[q] && a0 <= s_iv[ntrip + q] &&
+                   a2 >= s_iv[4 * ntrip + q] && a2 <= s_iv[5 * ntrip + q];
+        };
+        int cnt = 0;
+        unsigned long long hits = 0;  // of the first 64 rows
+        for (int q = s; q < e; ++q)
+            if (test(q)) {
+                if (q - s < 64) hits |= 1ull << (q - s);
+                ++cnt;
+            }
+        int off = cnt;  // matches of the lanes before
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, off, o);
+            if (lane >= o) off += v;
+        }
+        const int total = __shfl_sync(kFull, off, 31);
+        off -= cnt;
+        for (int base = 0; base < total;) {
+            // the lanes whose matches fit in the list from `base` on
+            const bool in = cnt > 0 && off >= base && off + cnt <= base + kList;
+            const unsigned inm = __ballot_sync(kFull, in);
+            if (inm == 0) {
+                // one band triplet with more matches than the list holds: one at a time, the
+                // smallest library index above the last one cast
+                const int l = __ffs(__ballot_sync(kFull, cnt > 0 && off == base)) - 1;
+                const float b0 = __shfl_sync(kFull, a0, l), b1 = __shfl_sync(kFull, a1, l), b2 = __shfl_sync(kFull, a2, l);
+                const unsigned btri = __shfl_sync(kFull, tri, l);
+                const int bs = __shfl_sync(kFull, s, l), be = __shfl_sync(kFull, e, l);
+                int last = -1;
+                while (true) {
+                    int mine = INT_MAX;
+                    for (int q = bs + lane; q < be; q += 32)
+                        if (b0 >= s_iv[q] && b0 <= s_iv[ntrip + q] && b1 >= s_iv[2 * ntrip + q] &&
+                            b1 <= s_iv[3 * ntrip + q] && b2 >= s_iv[4 * ntrip + q] && b2 <= s_iv[5 * ntrip + q] &&
+                            s_orig[q] > last && s_orig[q] < mine)
+                            mine = s_orig[q];
+                    const int next = __reduce_min_sync(kFull, mine);
+                    if (next == INT_MAX) break;
+                    float w1, w2, w3;
+                    const unsigned meta = weigh(next, b0, b1, b2, btri, w1, w2, w3);
+                    cast(meta, w1, w2, w3);
+                    last = next;
+                }
+                base += __shfl_sync(kFull, cnt, l);
+                continue;
+            }
+            if (in) {  // into the lane's part of the list, sorted into library order
+                int* seg = mlist + (off - base);
+                int have = 0;
+                auto put = [&](int q) {
+                    const int v = lane << 16 | s_orig[q];
+                    int b = have - 1;
+                    while (b >= 0 && seg[b] > v) {
+                        seg[b + 1] = seg[b];
+                        --b;
+                    }
+                    seg[b + 1] = v;
+                    ++have;
+                };
+                for (unsigned long long m = hits; m; m &= m - 1) put(s + __ffsll((long long)m) - 1);
+                for (int q = s + 64; q < e && have < cnt; ++q)
+                    if (test(q)) put(q);
+            }
+            const int n = __shfl_sync(kFull, off + cnt, 31 - __clz(inm)) - base;
+            __syncwarp();
+            for (int m0 = 0; m0 < n; m0 += 32) {
+                const int v = m0 + lane < n ? mlist[m0 + lane] : 0, l = v >> 16;
+                const float b0 = __shfl_sync(kFull, a0, l), b1 = __shfl_sync(kFull, a1, l), b2 = __shfl_sync(kFull, a2, l);
+                const unsigned btri = __shfl_sync(kFull, tri, l);
+                float w1, w2, w3;
+                const unsigned meta = weigh(v & 0xffff, b0, b1, b2, btri, w1, w2, w3);
+                const int nm = n - m0 < 32 ? n - m0 : 32;
+                for (int m = 0; m < nm; ++m)
+                    cast(__shfl_sync(kFull, meta, m), __shfl_sync(kFull, w1, m), __shfl_sync(kFull, w2, m),
+                         __shfl_sync(kFull, w3, m));
+            }
+            __syncwarp();
+            base += n;
         }
     }
     __syncwarp();
@@ -381,6 +444,9 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     __syncwarp();
 
     // ---- TRIAD assignment over band pairs in rank order, tripletvote.py:1600-1690 ----
+    // groups of nb lanes try a candidate each, lane tj of a group with band tj
+    const int ngrp = 32 / nb, grp = lane / nb, tj = lane - grp * nb;
+    const unsigned grp_mask = nb == 32 ? kFull : (1u << nb) - 1u;
     int best_n = 0;
     float best_fit = 360.0f;
     int bij[4] = {-1, -1, -1, -1};
@@ -410,8 +476,9 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
                 float y[3];
                 cross3(v1, x, y);
                 const float B[3][3] = {{v1[0], v1[1], v1[2]}, {x[0], x[1], x[2]}, {y[0], y[1], y[2]}};
-                const float p1[3] = {s_pole[row], s_pole[npoles + row], s_pole[2 * npoles + row]};
-                const float* bj = bn + 3 * (lane < nb ? lane : 0);
+                const float4 p1 = s_pole[row];
+                const float* bj = bn + 3 * tj;
+                const float bj0 = bj[0], bj1 = bj[1], bj2 = bj[2];
                 float score = -1.0f;
                 bool any = false;
                 for (int cb = 0; cb < cnt; cb += 32) {
@@ -420,51 +487,58 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
                     unsigned m = __ballot_sync(kFull, hit);
                     any = any || m != 0;
                     while (m) {
-                        const int cand = lo + cb + __ffs(m) - 1;
-                        m &= m - 1;
-                        float p2[3] = {s_pole[cand], s_pole[npoles + cand], s_pole[2 * npoles + cand]};
-                        const float n2 = __fadd_rn(norm3(p2), 1.0e-35f);
-                        p2[0] = __fdiv_rn(p2[0], n2); p2[1] = __fdiv_rn(p2[1], n2); p2[2] = __fdiv_rn(p2[2], n2);
-                        float pc[3];
-                        cross3(p1, p2, pc);
-                        const float npc = __fadd_rn(norm3(pc), 1.0e-35f);
-                        pc[0] = __fdiv_rn(pc[0], npc); pc[1] = __fdiv_rn(pc[1], npc); pc[2] = __fdiv_rn(pc[2], npc);
-                        float a2[3];
-                        cross3(p1, pc, a2);
-                        const float Am[3][3] = {{p1[0], pc[0], a2[0]}, {p1[1], pc[1], a2[1]}, {p1[2], pc[2], a2[2]}};
-                        float AB[3][3];
+                        // the next ngrp candidates, one a group (a group past the last takes the first)
+                        int cand = lo + cb + __ffs(m) - 1, ntry = 0;
+                        for (; ntry < ngrp && m; ++ntry, m &= m - 1)
+                            if (ntry == grp) cand = lo + cb + __ffs(m) - 1;
+                        // the frame of (p1, candidate): p1, their unit cross product, the cross of the two
+                        const float4* fr = (const float4*)(A.triad + ((size_t)f1 * npoles + cand) * 8);
+                        const float4 fa = __ldg(fr), fb = __ldg(fr + 1);
+                        const float Am[3][3] = {{p1.x, fa.x, fa.w}, {p1.y, fa.y, fb.x}, {p1.z, fa.z, fb.y}};
+                        float t[3];
 #pragma unroll
-                        for (int r = 0; r < 3; ++r)
+                        for (int r = 0; r < 3; ++r) {
+                            float AB[3];
 #pragma unroll
                             for (int c = 0; c < 3; ++c)
-                                AB[r][c] = dot3(Am[r][0], Am[r][1], Am[r][2], B[0][c], B[1][c], B[2][c]);
+                                AB[c] = dot3(Am[r][0], Am[r][1], Am[r][2], B[0][c], B[1][c], B[2][c]);
+                            t[r] = dot3(AB[0], AB[1], AB[2], bj0, bj1, bj2);
+                        }
                         // this lane's band: rotated normal, best library pole
-                        const float t0 = dot3(AB[0][0], AB[0][1], AB[0][2], bj[0], bj[1], bj[2]);
-                        const float t1 = dot3(AB[1][0], AB[1][1], AB[1][2], bj[0], bj[1], bj[2]);
-                        const float t2 = dot3(AB[2][0], AB[2][1], AB[2][2], bj[0], bj[1], bj[2]);
                         float best = -INFINITY;
                         int arg = 0;
+#pragma unroll 4
                         for (int P = 0; P < npoles; ++P) {
-                            const float v = dot3(s_pole[P], s_pole[npoles + P], s_pole[2 * npoles + P], t0, t1, t2);
+                            const float4 po = s_pole[P];
+                            const float v = dot3(po.x, po.y, po.z, t[0], t[1], t[2]);
                             if (v > best) { best = v; arg = P; }
                         }
                         best = best < -1.0f ? -1.0f : best;
                         best = best > 1.0f ? 1.0f : best;
                         const float ftry = acos_deg(best);
-                        const bool ok = lane < nb && ftry < tolf;
-                        const unsigned okm = __ballot_sync(kFull, ok);
+                        const bool ok = grp < ntry && ftry < tolf;
+                        const unsigned okm = (__ballot_sync(kFull, ok) >> (grp * nb < 32 ? grp * nb : 0)) & grp_mask;
                         const int nmatch = __popc(okm);
-                        if (ok) fscr[__popc(okm & lt_mask)] = ftry;
+                        if (ok) fscr[grp * nb + __popc(okm & ((1u << tj) - 1u))] = ftry;
                         __syncwarp();
-                        float mean = 0.0f;
-                        if (lane == 0) mean = __fdiv_rn(np_sum(fscr, nmatch), (float)nmatch);
-                        mean = __shfl_sync(kFull, mean, 0);
-                        const float stry = __fdiv_rn((float)nmatch, __fadd_rn(mean, 1e-6f));
-                        if (stry > score) {
-                            score = stry;
-                            afit = ftry;
-                            pm = arg;
-                            pv = ftry < tolf;
+                        float stry = 0.0f;
+                        if (grp < ntry && tj == 0) {
+                            const float mean = __fdiv_rn(np_sum(fscr + lane, nmatch), (float)nmatch);
+                            stry = __fdiv_rn((float)nmatch, __fadd_rn(mean, 1e-6f));
+                        }
+                        int sel = -1;
+                        for (int g = 0; g < ntry; ++g) {
+                            const float sg = __shfl_sync(kFull, stry, g * nb);
+                            if (sg > score) {
+                                score = sg;
+                                sel = g;
+                            }
+                        }
+                        if (sel >= 0) {
+                            const int src = (sel * nb + lane) & 31;  // lanes from nb on hold no band
+                            afit = __shfl_sync(kFull, ftry, src);
+                            pm = __shfl_sync(kFull, arg, src);
+                            pv = afit < tolf;
                         }
                         __syncwarp();
                     }
@@ -503,7 +577,7 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         float sc = -1.0f;
         if (!A.simpleq) {
             if (good) {
-                const int a = s_pfam[best_pm];
+                const int a = pole_family(best_pm);
                 const float an = accn[a * nb + lane];
                 sc = __fdiv_rn(accw[a * nb + lane], an > 0.0f ? an : 1.0e-12f);
             }
@@ -530,7 +604,7 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         float num = 0.0f;
         for (int j = 0; j < nb; ++j) {
             const int pmj = __shfl_sync(kFull, best_pm, j);
-            if ((goodm >> j) & 1u) num = __fadd_rn(num, accw[s_pfam[pmj] * nb + j]);
+            if ((goodm >> j) & 1u) num = __fadd_rn(num, accw[pole_family(pmj) * nb + j]);
         }
         float den = 0.0f;
         if (lane == 0)  // accumulator.clip(1) summed over all families and bands
@@ -542,7 +616,7 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
 
     // ---- outputs ----
     const ebsd_index_out& o = A.out;
-    const int accc = __popc(__ballot_sync(kFull, good && s_pfam[best_pm > 0 ? best_pm : 0] == fam));
+    const int accc = __popc(__ballot_sync(kFull, good && pole_family(best_pm > 0 ? best_pm : 0) == fam));
     if (lane < nb) {
         const int64_t e = p * nb + lane;
         o.polematch[e] = best_pm;
@@ -568,7 +642,8 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
 //   par: the largest y in [0, 1] with acos_deg(y) > angTol, so that the pair test
 //        arccos(|c|) * RADEG > angTol (tripletvote.py:1517) is |c| <= par;
 //   cand[f][c] = [lo, hi]: the cosines x in [-1, 1] with |angTable[famIndex[f]][c] - acos_deg(x)|
-//        < angTol in float64 (tripletvote.py:1521-1522); empty as [+inf, -inf].
+//        < angTol in float64 (tripletvote.py:1521-1522); empty as [+inf, -inf];
+//   triad[f][c]: what the TRIAD solution of a candidate c needs of the library alone.
 __device__ __forceinline__ int64_t okey(float f) {
     const uint32_t u = __float_as_uint(f);
     return (int64_t)((u & 0x80000000u) ? ~u : (u | 0x80000000u));
@@ -579,8 +654,8 @@ __device__ __forceinline__ float okey_float(int64_t k) {
 }
 
 __global__ void k_vote_thresholds(const double* __restrict__ angtab, const int32_t* __restrict__ famidx,
-                                  int nfam, int npoles, double tol, float tolf, float* __restrict__ cand,
-                                  float* __restrict__ par) {
+                                  const float4* __restrict__ pole, int nfam, int npoles, double tol, float tolf,
+                                  float* __restrict__ cand, float* __restrict__ par, float* __restrict__ triad) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t == 0) {
         int64_t a = okey(0.0f), b = okey(1.0f);
@@ -596,6 +671,25 @@ __global__ void k_vote_thresholds(const double* __restrict__ angtab, const int32
     }
     if (t >= nfam * npoles) return;
     const int f = t / npoles, c = t - f * npoles;
+    {  // the frame of the family's first pole and pole c: their unit cross product, its cross with the first
+        const float4 a = pole[famidx[f]], b = pole[c];
+        const float p1[3] = {a.x, a.y, a.z};
+        float p2[3] = {b.x, b.y, b.z};
+        const float n2 = __fadd_rn(norm3(p2), 1.0e-35f);
+        p2[0] = __fdiv_rn(p2[0], n2); p2[1] = __fdiv_rn(p2[1], n2); p2[2] = __fdiv_rn(p2[2], n2);
+        float pc[3];
+        cross3(p1, p2, pc);
+        const float npc = __fadd_rn(norm3(pc), 1.0e-35f);
+        pc[0] = __fdiv_rn(pc[0], npc); pc[1] = __fdiv_rn(pc[1], npc); pc[2] = __fdiv_rn(pc[2], npc);
+        float a2[3];
+        cross3(p1, pc, a2);
+        float* fr = triad + (size_t)t * 8;
+        for (int i = 0; i < 3; ++i) {
+            fr[i] = pc[i];
+            fr[3 + i] = a2[i];
+        }
+        fr[6] = fr[7] = 0.0f;
+    }
     const double T = angtab[(size_t)famidx[f] * npoles + c];
     const int64_t k0 = okey(-1.0f), k1 = okey(1.0f);
     // d(x) = T - acos_deg(x) does not decrease with x; the test is -tol < d < tol
@@ -788,20 +882,18 @@ __global__ void k_quest_fit(const QuestInput* __restrict__ qin, const float* __r
 
 __global__ void __launch_bounds__(kWarps * 32, 3) k_band_index(VoteArgs A) {
     extern __shared__ __align__(16) float vsm[];
-    float* s_iv = vsm;
+    float4* s_pole = (float4*)vsm;
+    float* s_iv = vsm + 4 * A.npoles;
     int* s_orig = (int*)(s_iv + 6 * A.ntrip);
-    float* s_pole = (float*)(s_orig + A.ntrip);
-    int* s_pfam = (int*)(s_pole + 3 * A.npoles);
     for (int t = threadIdx.x; t < 6 * A.ntrip; t += blockDim.x) s_iv[t] = A.iv[t];
     for (int t = threadIdx.x; t < A.ntrip; t += blockDim.x) s_orig[t] = A.orig[t];
-    for (int t = threadIdx.x; t < 3 * A.npoles; t += blockDim.x) s_pole[t] = A.pole[t];
-    for (int t = threadIdx.x; t < A.npoles; t += blockDim.x) s_pfam[t] = A.pfam[t];
+    for (int t = threadIdx.x; t < A.npoles; t += blockDim.x) s_pole[t] = ((const float4*)A.pole)[t];
     __syncthreads();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     float* w = vsm + block_words(A.ntrip, A.npoles) + warp * warp_words(A.nb, A.nfam);
     const int64_t stride = (int64_t)gridDim.x * kWarps;
     for (int64_t p = (int64_t)blockIdx.x * kWarps + warp; p < A.n; p += stride)
-        index_pattern(A, p, lane, s_iv, s_orig, s_pole, s_pfam, w);
+        index_pattern(A, p, lane, s_iv, s_orig, s_pole, w);
 }
 
 // ---- band weights and pattern quality, _ebsd_index_single.py:751-763 ----
@@ -932,9 +1024,12 @@ extern "C" int ebsd_vote_plan_create(const ebsd_triplib_desc* d, int device, ebs
         if (iv0[q] <= iv0[nt + q]) wmax = std::max(wmax, (double)iv0[nt + q] - (double)iv0[q]);
     }
     p->win = (float)(wmax + 1e-3);
-    std::vector<float> pole(3 * (size_t)np_);
-    for (int i = 0; i < np_; ++i)
-        for (int c = 0; c < 3; ++c) pole[c * np_ + i] = (float)d->poles_cart[3 * i + c];
+    std::vector<float> pole(4 * (size_t)np_);
+    for (int i = 0; i < np_; ++i) {
+        for (int c = 0; c < 3; ++c) pole[4 * (size_t)i + c] = (float)d->poles_cart[3 * i + c];
+        const int32_t fam = d->pole_family[i];
+        std::memcpy(&pole[4 * (size_t)i + 3], &fam, 4);
+    }
     std::vector<int32_t> fidx(nf);
     for (int f = 0; f < nf; ++f) fidx[f] = (int32_t)d->fam_index[f];
 
@@ -949,17 +1044,17 @@ extern "C" int ebsd_vote_plan_create(const ebsd_triplib_desc* d, int device, ebs
     if (!rc) rc = up((void**)&p->d_tang, d->trip_angles, 3 * (size_t)nt * 8);
     if (!rc) rc = up((void**)&p->d_pole, pole.data(), pole.size() * 4);
     if (!rc) rc = up((void**)&p->d_pole64, d->poles_cart, 3 * (size_t)np_ * 8);
-    if (!rc) rc = up((void**)&p->d_pfam, d->pole_family, (size_t)np_ * 4);
     if (!rc) rc = up((void**)&p->d_angtab, d->ang_table, (size_t)np_ * np_ * 8);
     if (!rc) rc = up((void**)&p->d_famcnt, d->fam_count, (size_t)nf * 4);
     if (!rc) rc = up((void**)&p->d_famidx, fidx.data(), (size_t)nf * 4);
     if (!rc) rc = up((void**)&p->d_orig, order.data(), (size_t)nt * 4);
     if (!rc && cudaMalloc((void**)&p->d_cand, (size_t)nf * np_ * 2 * 4) != cudaSuccess) rc = EBSD_E_NOMEM;
+    if (!rc && cudaMalloc((void**)&p->d_triad, (size_t)nf * np_ * 8 * 4) != cudaSuccess) rc = EBSD_E_NOMEM;
     if (!rc && cudaMalloc((void**)&p->d_par, 4) != cudaSuccess) rc = EBSD_E_NOMEM;
     if (!rc) {
         const int total = nf * np_;
-        k_vote_thresholds<<<(total + 127) / 128, 128>>>(p->d_angtab, p->d_famidx, nf, np_, p->tol, (float)p->tol,
-                                                        p->d_cand, p->d_par);
+        k_vote_thresholds<<<(total + 127) / 128, 128>>>(p->d_angtab, p->d_famidx, (const float4*)p->d_pole, nf, np_,
+                                                        p->tol, (float)p->tol, p->d_cand, p->d_par, p->d_triad);
         rc = launch_status();
         if (!rc && cudaMemcpy(&p->par, p->d_par, 4, cudaMemcpyDeviceToHost) != cudaSuccess) rc = EBSD_E_LAUNCH;
     }
@@ -979,7 +1074,7 @@ extern "C" int ebsd_vote_plan_destroy(ebsd_vote_plan_t p) {
     cudaFree(p->d_tang);
     cudaFree(p->d_pole);
     cudaFree(p->d_pole64);
-    cudaFree(p->d_pfam);
+    cudaFree(p->d_triad);
     cudaFree(p->d_angtab);
     cudaFree(p->d_famcnt);
     cudaFree(p->d_famidx);
@@ -1015,7 +1110,7 @@ extern "C" int ebsd_band_index(ebsd_vote_plan_t p, const float* d_norms, const f
     A.tang = p->d_tang;
     A.pole = p->d_pole;
     A.pole64 = p->d_pole64;
-    A.pfam = p->d_pfam;
+    A.triad = p->d_triad;
     A.angtab = p->d_angtab;
     A.famcnt = p->d_famcnt;
     A.famidx = p->d_famidx;
