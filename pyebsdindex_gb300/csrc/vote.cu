@@ -24,7 +24,7 @@
 // What bounds the kernel is instructions issued.  FCC library (167 triplets, 50 poles), nine
 // bands: 84 band triplets, 85 matches and 14 candidates a pattern cost 63,800 warp instructions
 // with a warp per triplet, lane 0 casting the votes and a candidate at a time, and 15.2 ms per
-// 200,000 patterns; 18,900 and 6.0 ms now.
+// 200,000 patterns; 19,800 and 5.0 ms now (four blocks an SM; three: 6.0).
 #include "ebsd_internal.cuh"
 
 #include <algorithm>
@@ -225,12 +225,11 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     const int nb = A.nb, nfam = A.nfam, ntrip = A.ntrip, npoles = A.npoles;
     const float tolf = A.tol_f;
     auto pole_family = [s_pole](int P) { return __float_as_int(s_pole[P].w); };
-    float* bn = w;                       // [nb][3]
+    float2* acc = (float2*)w;            // [nfam][nb] vote weight and count
+    float* bn = w + 2 * nfam * nb;       // [nb][3]
     float* inten = bn + 3 * nb;          // [nb]
     float* ang = inten + nb;             // [nb][nb]
-    float* accw = ang + nb * nb;          // [nfam][nb]
-    float* accn = accw + nfam * nb;      // [nfam][nb]
-    int* rarg = (int*)(accn + nfam * nb);  // [nb] band order, ascending rank
+    int* rarg = (int*)(ang + nb * nb);   // [nb] band order, ascending rank
     int* bfam = rarg + nb;               // [nb]
     int* mlist = bfam + nb;              // [kList] matches: triplet lane << 16 | library index
     float* fscr = (float*)mlist;         // [32] band fits (after the vote)
@@ -238,7 +237,7 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
 
     for (int t = lane; t < 3 * nb; t += 32) bn[t] = A.norms[p * 3 * nb + t];
     for (int t = lane; t < nb; t += 32) inten[t] = A.inten ? A.inten[p * nb + t] : 1.0f;
-    for (int t = lane; t < 2 * nfam * nb; t += 32) accw[t] = 0.0f;
+    for (int t = lane; t < nfam * nb; t += 32) acc[t] = make_float2(0.0f, 0.0f);
     __syncwarp();
 
     // band-band angles, tripletvote.py:1181-1188 (the vote reads the upper triangle only)
@@ -265,11 +264,15 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     auto cast = [&](unsigned meta, float w1, float w2, float w3) {
         const bool ri = lane == (int)(meta & 31u), rj = lane == (int)((meta >> 5) & 31u);
         if (!(ri || rj || lane == (int)((meta >> 10) & 31u))) return;
-        const int f0 = (meta >> 15) & 15u, f1 = (meta >> 19) & 15u, f2 = (meta >> 23) & 15u;
+        float2* const a0 = acc + (int)((meta >> 15) & 15u) * nb + lane;
+        float2* const a1 = acc + (int)((meta >> 19) & 15u) * nb + lane;
+        float2* const a2 = acc + (int)((meta >> 23) & 15u) * nb + lane;
         auto vote = [&](int role) {  // 0: (f0, w1), 1: (f1, w2), 2: (f2, w3)
-            const int t = (role == 0 ? f0 : role == 1 ? f1 : f2) * nb + lane;
-            accw[t] = __fadd_rn(accw[t], role == 0 ? w1 : role == 1 ? w2 : w3);
-            accn[t] = __fadd_rn(accn[t], 1.0f);
+            float2* const t = role == 0 ? a0 : role == 1 ? a1 : a2;
+            float2 v = *t;
+            v.x = __fadd_rn(v.x, role == 0 ? w1 : role == 1 ? w2 : w3);
+            v.y = __fadd_rn(v.y, 1.0f);
+            *t = v;
         };
         vote(ri ? 0 : rj ? 1 : 2);
         const unsigned ee = meta >> 27;
@@ -332,14 +335,15 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         const float tgt = a0 - A.win;
         const int e = on ? count_leading(ntrip, [&](int q) { return s_iv[q] <= a0; }) : 0;
         const int s = count_leading(e, [&](int q) { return s_iv[q] < tgt; });
-        auto test = [&](int q) {
-            return a1 >= s_iv[2 * ntrip + q] && a1 <= s_iv[3 * ntrip + q] && a0 >= s_iv[q] && a0 <= s_iv[ntrip + q] &&
-                   a2 >= s_iv[4 * ntrip + q] && a2 <= s_iv[5 * ntrip + q];
+        auto test = [&](const float* r, float b0, float b1, float b2) {
+            return (b1 >= r[2 * ntrip]) & (b1 <= r[3 * ntrip]) & (b0 >= r[0]) & (b0 <= r[ntrip]) & (b2 >= r[4 * ntrip]) &
+                   (b2 <= r[5 * ntrip]);
         };
         int cnt = 0;
         unsigned long long hits = 0;  // of the first 64 rows
+#pragma unroll 2
         for (int q = s; q < e; ++q)
-            if (test(q)) {
+            if (test(s_iv + q, a0, a1, a2)) {
                 if (q - s < 64) hits |= 1ull << (q - s);
                 ++cnt;
             }
@@ -350,34 +354,32 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         }
         const int total = __shfl_sync(kFull, off, 31);
         off -= cnt;
+        int last = -1;
         for (int base = 0; base < total;) {
             // the lanes whose matches fit in the list from `base` on
             const bool in = cnt > 0 && off >= base && off + cnt <= base + kList;
             const unsigned inm = __ballot_sync(kFull, in);
+            int n;
             if (inm == 0) {
-                // one band triplet with more matches than the list holds: one at a time, the
-                // smallest library index above the last one cast
+                // one band triplet with more matches than the list holds: 32 at a time, each the
+                // smallest library index above the last one
                 const int l = __ffs(__ballot_sync(kFull, cnt > 0 && off == base)) - 1;
                 const float b0 = __shfl_sync(kFull, a0, l), b1 = __shfl_sync(kFull, a1, l), b2 = __shfl_sync(kFull, a2, l);
-                const unsigned btri = __shfl_sync(kFull, tri, l);
                 const int bs = __shfl_sync(kFull, s, l), be = __shfl_sync(kFull, e, l);
-                int last = -1;
-                while (true) {
+                for (n = 0; n < 32; ++n) {
                     int mine = INT_MAX;
                     for (int q = bs + lane; q < be; q += 32)
-                        if (b0 >= s_iv[q] && b0 <= s_iv[ntrip + q] && b1 >= s_iv[2 * ntrip + q] &&
-                            b1 <= s_iv[3 * ntrip + q] && b2 >= s_iv[4 * ntrip + q] && b2 <= s_iv[5 * ntrip + q] &&
-                            s_orig[q] > last && s_orig[q] < mine)
-                            mine = s_orig[q];
-                    const int next = __reduce_min_sync(kFull, mine);
-                    if (next == INT_MAX) break;
-                    float w1, w2, w3;
-                    const unsigned meta = weigh(next, b0, b1, b2, btri, w1, w2, w3);
-                    cast(meta, w1, w2, w3);
-                    last = next;
+                        if (test(s_iv + q, b0, b1, b2) && s_orig[q] > last && s_orig[q] < mine) mine = s_orig[q];
+                    last = __reduce_min_sync(kFull, mine);
+                    if (last == INT_MAX) break;
+                    if (lane == 0) mlist[n] = l << 16 | last;
                 }
-                base += __shfl_sync(kFull, cnt, l);
-                continue;
+                if (last == INT_MAX) {
+                    base += __shfl_sync(kFull, cnt, l);
+                    last = -1;
+                }
+            } else {
+                n = __shfl_sync(kFull, off + cnt, 31 - __clz(inm)) - base;
             }
             if (in) {  // into the lane's part of the list, sorted into library order
                 int* seg = mlist + (off - base);
@@ -394,9 +396,9 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
                 };
                 for (unsigned long long m = hits; m; m &= m - 1) put(s + __ffsll((long long)m) - 1);
                 for (int q = s + 64; q < e && have < cnt; ++q)
-                    if (test(q)) put(q);
+                    if (test(s_iv + q, a0, a1, a2)) put(q);
             }
-            const int n = __shfl_sync(kFull, off + cnt, 31 - __clz(inm)) - base;
+            if (inm != 0) base += n;
             __syncwarp();
             for (int m0 = 0; m0 < n; m0 += 32) {
                 const int v = m0 + lane < n ? mlist[m0 + lane] : 0, l = v >> 16;
@@ -410,7 +412,6 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
                          __shfl_sync(kFull, w3, m));
             }
             __syncwarp();
-            base += n;
         }
     }
     __syncwarp();
@@ -421,7 +422,7 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
     if (lane < nb) {
         float sum = 0.0f, mx = -1.0e12f, m1 = -INFINITY, m2 = -INFINITY;
         for (int f = 0; f < nfam; ++f) {
-            const float v = accw[f * nb + lane];
+            const float v = acc[f * nb + lane].x;
             sum = __fadd_rn(sum, v);
             if (v > mx) { mx = v; fam = f; }
             if (v > m1) { m2 = m1; m1 = v; } else if (v > m2) { m2 = v; }
@@ -578,8 +579,8 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         if (!A.simpleq) {
             if (good) {
                 const int a = pole_family(best_pm);
-                const float an = accn[a * nb + lane];
-                sc = __fdiv_rn(accw[a * nb + lane], an > 0.0f ? an : 1.0e-12f);
+                const float2 v = acc[a * nb + lane];
+                sc = __fdiv_rn(v.x, v.y > 0.0f ? v.y : 1.0e-12f);
             }
         } else if (good) {
             sc = inten[__popc(goodm & lt_mask)];
@@ -604,11 +605,11 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         float num = 0.0f;
         for (int j = 0; j < nb; ++j) {
             const int pmj = __shfl_sync(kFull, best_pm, j);
-            if ((goodm >> j) & 1u) num = __fadd_rn(num, accw[pole_family(pmj) * nb + j]);
+            if ((goodm >> j) & 1u) num = __fadd_rn(num, acc[pole_family(pmj) * nb + j].x);
         }
         float den = 0.0f;
         if (lane == 0)  // accumulator.clip(1) summed over all families and bands
-            den = np_sum_get<float>([accw](int t) { const float v = accw[t]; return (v != v || v >= 1.0f) ? v : 1.0f; },
+            den = np_sum_get<float>([acc](int t) { const float v = acc[t].x; return (v != v || v >= 1.0f) ? v : 1.0f; },
                                     nfam * nb);
         den = __shfl_sync(kFull, den, 0);
         cm2 = __fdiv_rn(num, den);
@@ -625,9 +626,9 @@ __device__ void index_pattern(const VoteArgs& A, int64_t p, int lane, const floa
         if (o.polevalid) o.polevalid[e] = (uint8_t)best_pv;
     }
     if (o.accw)
-        for (int t = lane; t < nfam * nb; t += 32) o.accw[p * nfam * nb + t] = accw[t];
+        for (int t = lane; t < nfam * nb; t += 32) o.accw[p * nfam * nb + t] = acc[t].x;
     if (o.accn)
-        for (int t = lane; t < nfam * nb; t += 32) o.accn[p * nfam * nb + t] = accn[t];
+        for (int t = lane; t < nfam * nb; t += 32) o.accn[p * nfam * nb + t] = acc[t].y;
     if (lane == 0) {
         o.cm[p] = cm2;
         o.nmatch[p] = best_n;
@@ -880,7 +881,7 @@ __global__ void k_quest_fit(const QuestInput* __restrict__ qin, const float* __r
     }
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 3) k_band_index(VoteArgs A) {
+__global__ void __launch_bounds__(kWarps * 32, 4) k_band_index(VoteArgs A) {
     extern __shared__ __align__(16) float vsm[];
     float4* s_pole = (float4*)vsm;
     float* s_iv = vsm + 4 * A.npoles;
