@@ -121,16 +121,18 @@ int ebsd_plan_reserve(ebsd_plan_t plan, int method, int64_t max_chunk);
 int ebsd_find_bands(ebsd_plan_t plan, int method, int dtype, const void* d_pats, int64_t n,
                     const ebsd_bands* d_out, int64_t chunk, void* stream);
 
-/* Mixed pattern sizes in one persistent launch: the FP32 fused method for up to 8 plans at
+/* Mixed pattern sizes in one call: the FP32 fused method for up to 8 plans at
  * once (e.g. one plan per detector size), plan k's d_pats[k] [n[k]][H_k][W_k] of `dtype`
  * into d_out[k].  The reference runs one size per BandDetect plan and rebuilds the plan when
- * the size changes (band_detect.py:138-155); here every persistent CTA strides over the
- * patterns of all plans, each pattern detected in theta slabs with its plan's tables.  All
+ * the size changes (band_detect.py:138-155); here integer patterns run size by size on the
+ * strip kernels, and where those do not serve (float patterns, a plan without its scratch) one
+ * persistent launch strides over the patterns of all plans in theta slabs.  All
  * plans live on one device and share the LoG size; each must report
  * ebsd_method_supported(plan, EBSD_FUSED_F32) and qualify for the slab kernel (uint8 /
  * uint16 input; float32 where its pattern tile fits), else EBSD_E_UNSUPPORTED.  Records equal
  * those of ebsd_find_bands with EBSD_FUSED_F32 on each plan alone, up to the last bit of
- * normmax.  Asynchronous on `stream`; allocates nothing. */
+ * normmax.  Asynchronous on `stream`; allocates nothing but a plan's strip scratch, once (never
+ * during a stream capture). */
 int ebsd_find_bands_mixed(const ebsd_plan_t* plans, int nplans, int dtype, const void* const* d_pats,
                           const int64_t* n, const ebsd_bands* d_out, void* stream);
 
@@ -145,7 +147,9 @@ int ebsd_find_bands_host(ebsd_plan_t plan, int method, int dtype, const void* h_
  * the kernels read it in place over the CPU-GPU link when the device uses the host's page
  * tables (GB300's NVLink-C2C), else copy engines stage it chunk by chunk; 0: always stage
  * with copies; 1: always read in place.  Either way every input byte crosses the link once
- * per call.  Pageable input is always staged through pinned buffers. */
+ * per call.  Pageable input is staged through pinned buffers, except by -1 in a call of one
+ * chunk of integer patterns (at most 64 MB) that the strip kernels serve: such input is read in
+ * place too. */
 int ebsd_plan_set_host_input(ebsd_plan_t plan, int mode);
 
 /* 1 when pinned host input is read in place under the plan's current mode, 0 when copied. */
@@ -156,7 +160,8 @@ int ebsd_plan_host_input_in_place(ebsd_plan_t plan);
 int64_t ebsd_last_launch_count(ebsd_plan_t plan);
 
 /* Autotuner -- no counterpart in the reference, whose OpenCL path sizes its work by fixed
- * rules (band_detect_cl.py:252-286).  Times the fused-kernel variants that give identical
+ * rules (band_detect_cl.py:252-286).  Calls that the strip kernels serve (EBSD_FUSED_F32 on
+ * integer patterns) have one variant: it returns at once, with 8 (uint8) or 1.  Else it times the fused-kernel variants that give identical
  * records for (method, dtype) on the caller's device-resident sample d_pats [n][H][W] and keeps
  * the fastest in the plan for later calls.  The variants are the Radon tile shapes the plan
  * can take: the whole padded Radon image as one tile with one, two, four or eight patterns per

@@ -239,7 +239,8 @@ class GPUFindBands:
     def autotune(self, sample, method=None, gpu_id=None, cache=None):
         """Time the record-identical variants of the fused kernel on ``sample`` ([n, H, W]
         numpy or torch, uint8/uint16/float32) and keep the fastest in the device plan for later
-        ``find_bands`` calls.  The variants are Radon tile shapes: the whole padded Radon image
+        ``find_bands`` calls (integer patterns that the strip kernels serve have one variant: nothing
+        is timed).  The variants are Radon tile shapes: the whole padded Radon image
         as one tile with one, two, four or eight patterns per block pass, and theta slabs of
         several widths (``DevicePlan.get_tile`` reads the choice back; it is also kept in
         ``self.tuned``).  No counterpart in the reference.  Returns the chosen patterns per
@@ -629,7 +630,8 @@ class MixedBandDetect:
     def find_bands_device(self, batches, method=None, stream=None, out=None):
         """batches: {(H, W): CUDA tensor [n, H, W]} (one input type) -> {(H, W): dict of device
         band arrays}, asynchronous on ``stream`` (default: the current stream).  With the fused
-        method and at most eight sizes that the slab kernel takes, one launch serves them all.
+        method and at most eight sizes that the slab kernel takes, one library call serves them
+        all (integer patterns size by size on the strip kernels, float ones in one launch).
         ``out``: the dict a previous call returned, written again instead of new arrays (the
         same sizes and counts) -- with it the call allocates nothing and can be captured in a
         CUDA graph (after a first call has set the kernels up)."""
@@ -677,7 +679,8 @@ class MixedBandDetect:
                 for f in _lib.BAND_FIELDS}
 
     def autotune(self, batches, stream=None, max_extra=3):
-        """Choose each size's theta-slab width for the one-launch mixed path.  For every size in
+        """Choose each size's theta-slab width for the one-launch mixed path (which float patterns
+        take; integer patterns run on the strip kernels whatever the width).  For every size in
         ``batches`` ({(H, W): CUDA tensor [n, H, W]}, a sample of each), the slab counts from
         the widest slabs that fit to ``max_extra`` narrower ones are timed on that size alone
         (the slab kernel, CUDA events on ``stream``, best of two runs after a warm-up), and the

@@ -692,7 +692,8 @@ __device__ void edge_sums(float* sm, int block, const float* __restrict__ data, 
 // pixels stream into a second buffer (cp.async) while the current ones are summed, stored with the scan
 // columns along the fast axis.  A chunk with no value at or above a saturation level (nor a NaN) is
 // summed without the per-term tests and counted whole.  Measured, 128x160 scan of 80x80, radius 3: 1.35
-// ms with one pair per thread and step (11 instructions a term, staging exposed).
+// ms with one pair per thread and step (11 instructions a term, staging exposed), 1.01 ms now; bound by
+// the summing warps' dependent packed operations (a third staging buffer: 1.15 ms, one block fewer an SM).
 constexpr int kPairLanes = 30;                 // 60 pixels and 2 SR halo columns
 constexpr int kPairPitch = 66;                 // staged columns (2 modulo 32: a column's 32 pixels in 16 banks)
 
