@@ -17,6 +17,7 @@
 
 #include <cstring>
 #include <new>
+#include <type_traits>
 
 struct ebsd_linop_s {
     int device = 0;
@@ -55,8 +56,8 @@ __global__ void k_csr_gather(const int64_t* __restrict__ rowptr, const int32_t* 
 // takes kCsrRows neighbouring rows at once and 32 NV patterns: a nonzero costs one 8-byte
 // broadcast, and NV coalesced loads feed NV multiply-adds of independent chains.  Bound by the
 // L1's 128 bytes a cycle.  1024 patterns, 120x120 pixels, 180x180 rays: Radon 1261 us with a row
-// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 912 now; its adjoint 1235, 1110
-// now; the LoG 451, 318 now.
+// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 582 now; its adjoint 1235, 836
+// now; the LoG 451, 215 now (with an address per load of a nonzero: 912, 1110, 318).
 constexpr int kCsrTileY = 4, kCsrTileX = 8, kCsrRows = 4;
 
 template <typename T> struct CsrEnt;
@@ -98,41 +99,43 @@ __global__ void __launch_bounds__(256) k_csr_gather_cols(const int64_t* __restri
         len[i] = (int)(__ldg(rowptr + r + 1) - e[i]);
         common = len[i] < common ? len[i] : common;
     }
-    int64_t off[NV];  // patterns past the last read column 0 and are not stored
+    // kWhole: every pattern of the block exists, so that a nonzero's loads differ by constants from
+    // one address; else patterns past the last read column 0 and are not stored
+    auto run = [&](auto whole) {
+        constexpr bool kWhole = decltype(whole)::value;
+        const T* xb = kWhole ? xT + b0 : xT;
+        int64_t off[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) off[v] = b0 + 32 * v < n ? b0 + 32 * v : 0;
-    T acc[kCsrRows][NV];
+        for (int v = 0; v < NV; ++v) off[v] = kWhole ? 32 * v : (b0 + 32 * v < n ? b0 + 32 * v : 0);
+        T acc[kCsrRows][NV];
 #pragma unroll
-    for (int i = 0; i < kCsrRows; ++i)
+        for (int i = 0; i < kCsrRows; ++i)
 #pragma unroll
-        for (int v = 0; v < NV; ++v) acc[i][v] = (T)0;
+            for (int v = 0; v < NV; ++v) acc[i][v] = (T)0;
+        auto add = [&](int i, int64_t at) {
+            int c;
+            T a;
+            ent.get(at, c, a);
+            const T* xr = xb + (int64_t)c * ldx;
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
+        };
 #pragma unroll 2
-    for (int t = 0; t < common; ++t)
+        for (int t = 0; t < common; ++t)
+#pragma unroll
+            for (int i = 0; i < kCsrRows; ++i) add(i, e[i] + t);
 #pragma unroll
         for (int i = 0; i < kCsrRows; ++i) {
-            int c;
-            T a;
-            ent.get(e[i] + t, c, a);
-            const T* xr = xT + (int64_t)c * ldx;
-#pragma unroll
-            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
-        }
-#pragma unroll
-    for (int i = 0; i < kCsrRows; ++i) {
 #pragma unroll 4
-        for (int t = common; t < len[i]; ++t) {
-            int c;
-            T a;
-            ent.get(e[i] + t, c, a);
-            const T* xr = xT + (int64_t)c * ldx;
+            for (int t = common; t < len[i]; ++t) add(i, e[i] + t);
+            if (gx + i < width && row + i < nrows)
 #pragma unroll
-            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
+                for (int v = 0; v < NV; ++v)
+                    if (kWhole || b0 + 32 * v < n) yT[(row + i) * ldy + b0 + 32 * v] = acc[i][v];
         }
-        if (gx + i < width && row + i < nrows)
-#pragma unroll
-            for (int v = 0; v < NV; ++v)
-                if (b0 + 32 * v < n) yT[(row + i) * ldy + b0 + 32 * v] = acc[i][v];
-    }
+    };
+    if ((int64_t)(blockIdx.y + 1) * (32 * NV) <= n) run(std::true_type());
+    else run(std::false_type());
 }
 
 // Patterns a warp: 128 in float, 64 in double; a batch of fewer takes what it fills.
@@ -141,8 +144,9 @@ void launch_csr_cols(cudaStream_t st, const int64_t* rowptr, CsrEnt<T> ent, cons
                      int64_t nrows, int64_t width, int64_t n) {
     const unsigned tiles = (unsigned)(((width + kCsrTileX - 1) / kCsrTileX) * ((nrows + width * kCsrTileY - 1) / (width * kCsrTileY)));
     const dim3 block(32, 8);
-    if (n > 64 && sizeof(T) == 4)
-        k_csr_gather_cols<T, 4><<<dim3(tiles, (unsigned)((n + 127) / 128)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
+    constexpr int kMost = sizeof(T) == 4 ? 4 : 2;
+    if (n > 64 && kMost == 4)
+        k_csr_gather_cols<T, kMost><<<dim3(tiles, (unsigned)((n + 32 * kMost - 1) / (32 * kMost))), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
     else if (n > 32)
         k_csr_gather_cols<T, 2><<<dim3(tiles, (unsigned)((n + 63) / 64)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
     else
