@@ -692,8 +692,10 @@ __device__ void edge_sums(float* sm, int block, const float* __restrict__ data, 
 // pixels stream into a second buffer (cp.async) while the current ones are summed, stored with the scan
 // columns along the fast axis.  A chunk with no value at or above a saturation level (nor a NaN) is
 // summed without the per-term tests and counted whole.  Measured, 128x160 scan of 80x80, radius 3: 1.35
-// ms with one pair per thread and step (11 instructions a term, staging exposed), 1.01 ms now; bound by
-// the summing warps' dependent packed operations (a third staging buffer: 1.15 ms, one block fewer an SM).
+// ms with one pair per thread and step (11 instructions a term, staging exposed), 0.84 ms now; bound by
+// the summing warps' dependent packed operations: the offsets' differences, squares and sums are issued
+// kind by kind and eight pixels unrolled (offset by offset, four pixels: 0.87; a third staging buffer,
+// one block fewer an SM: 7 % more).
 constexpr int kPairLanes = 30;                 // 60 pixels and 2 SR halo columns
 constexpr int kPairPitch = 66;                 // staged columns (2 modulo 32: a column's 32 pixels in 16 banks)
 
@@ -769,14 +771,20 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
 #pragma unroll
         for (int k = 0; k <= SR; ++k)
             if (kKind != 0 || 2 * k + 1 > SR) v[k] = *(const Pair2*)(pb + 2 * k);
+        constexpr int e0 = kKind == 0 ? SR + 1 : 0;
+        Pair2 t[WN];
 #pragma unroll
-        for (int e = kKind == 0 ? SR + 1 : 0; e < WN; ++e) {
+        for (int e = e0; e < WN; ++e) {
             const Pair2 b = (e & 1) ? p2_pack(p2_unpack(v[e / 2]).y, p2_unpack(v[e / 2 + 1]).x) : v[e / 2];
-            const Pair2 t = p2_sub(a, b, m1);
-            const Pair2 tt = p2_mul(t, t, z);
-            d[e] = p2_add(d[e], tt);
-            if (kSig && kKind == 0 && e == SR + 1) ds[0] = p2_add(ds[0], tt);
-            if (kSig && kKind == 1 && e >= SR - 1 && e <= SR + 1) ds[e - SR + 1] = p2_add(ds[e - SR + 1], tt);
+            t[e] = p2_sub(a, b, m1);
+        }
+#pragma unroll
+        for (int e = e0; e < WN; ++e) t[e] = p2_mul(t[e], t[e], z);
+#pragma unroll
+        for (int e = e0; e < WN; ++e) {
+            d[e] = p2_add(d[e], t[e]);
+            if (kSig && kKind == 0 && e == SR + 1) ds[0] = p2_add(ds[0], t[e]);
+            if (kSig && kKind == 1 && e >= SR - 1 && e <= SR + 1) ds[e - SR + 1] = p2_add(ds[e - SR + 1], t[e]);
         }
     };
     if (helper >= 0) stage(0, 0);
@@ -817,13 +825,13 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         } else if (mine) {
             // every term of the chunk counts (the counts are exact integers either way)
             if (dy == 0) {
-#pragma unroll 4
+#pragma unroll 8
                 for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 0, std::integral_constant<int, 0>());
             } else if (dy == 1) {
-#pragma unroll 4
+#pragma unroll 8
                 for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 1, std::integral_constant<int, 1>());
             } else {
-#pragma unroll 4
+#pragma unroll 8
                 for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, dy, std::integral_constant<int, 2>());
             }
             n0 += (float)qn;
@@ -1032,7 +1040,7 @@ int launch_pairs(cudaStream_t st, const float* data, int nrows, int ncols, int n
 // ---- the weights with the pieces of their derivative, from the pair sums ----------------------
 // 1024 pixels of 14400 values, radius 2: k_sigma_arg and k_nlpar_weights_d, which sum every pair once
 // for each of its pixels and slots with a serial, uncoalesced pair_ssd, took 1010 + 1165 us; the pair
-// kernel (844, its 32 blocks' serial chains) and these two (6 + 6) take their place at radius 1-3.
+// kernel (648, its 32 blocks' serial chains) and these two (6 + 6) take their place at radius 1-3.
 // sigma^2 with the neighbour that attains the minimum and its pair count: k_sigma_arg's scan of the
 // eight neighbours in raster order, the sums read instead of made.
 __global__ void k_nlpar_sigma_arg_pairs(const float2* __restrict__ sigp, int nrows, int ncols, float* __restrict__ sig2,
