@@ -56,9 +56,10 @@ __global__ void k_csr_gather(const int64_t* __restrict__ rowptr, const int32_t* 
 // takes kCsrRows neighbouring rows at once and 32 NV patterns: a nonzero costs one 8-byte
 // broadcast, and NV coalesced loads feed NV multiply-adds of independent chains.  Bound by the
 // L1's 128 bytes a cycle.  1024 patterns, 120x120 pixels, 180x180 rays: Radon 1261 us with a row
-// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 582 now; its adjoint 1235, 836
-// now; the LoG 451, 215 now (with an address per load of a nonzero: 912, 1110, 318).
-constexpr int kCsrTileY = 4, kCsrTileX = 8, kCsrRows = 4;
+// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 515 now; its adjoint 1235, 580
+// now; the LoG 451, 194 now.  With an address per load of a nonzero: 912, 1110, 318; four rows a warp
+// in 4 x 8 tiles (78 registers, 24 warps an SM): 582, 836, 215; one row: 520, 550, 193.
+constexpr int kCsrTileY = 4, kCsrTileX = 4, kCsrRows = 2;
 
 template <typename T> struct CsrEnt;
 template <> struct CsrEnt<float> {
@@ -399,7 +400,7 @@ __global__ void k_blur1d_t(const T* __restrict__ v, T* __restrict__ out, int64_t
 // (triangles unrolled), those between reach all of them.  What bounds it is issue: of the ~12
 // instructions a position costs 8 are the multiply-adds; the one-output-a-thread kernels above
 // spend 21 a tap.  1024 120x120 patterns, r = 30, per pass: 643 / 452 us along y / x before,
-// 94 / 109 now (the adjoint 384 / 526 before, 86 / 106 now).
+// 74 / 88 now (the adjoint 384 / 526 before, 75 / 91 now).
 constexpr int kBlurR = 8, kBlurWarps = 4, kBlurLines = 32, kBlurPitch = 33, kBlurPad = 20;
 
 __host__ __device__ inline int blur_tap_off(int r) { return kBlurPad + ((4 - ((2 * r + 2 + kBlurPad) & 3)) & 3); }
@@ -451,6 +452,19 @@ __device__ __forceinline__ void blur_sum(float (&acc)[kBlurR], const float* __re
         for (int i = 0; i < 2 * kBlurR / 4; ++i) {
             const float4 f = t4[i];
             t[4 * i] = f.x; t[4 * i + 1] = f.y; t[4 * i + 2] = f.z; t[4 * i + 3] = f.w;
+        }
+        if (o0 >= 0 && o0 + kBlurR <= L && o0 + kBlurR - 1 <= m1) {  // inside the line: one address
+            const float* lp = line + o0 * kBlurPitch;
+#pragma unroll
+            for (int s = 0; s < kBlurR; ++s) {
+                const float v = lp[s * kBlurPitch];
+#pragma unroll
+                for (int j = 0; j < kBlurR; ++j) {
+                    float& a = acc[kRev ? kBlurR - 1 - j : j];
+                    a = fmaf(t[kBlurR - 1 - s + j], v, a);
+                }
+            }
+            continue;
         }
 #pragma unroll
         for (int s = 0; s < kBlurR; ++s) {
