@@ -149,10 +149,12 @@ int ebsd_find_bands_host(ebsd_plan_t plan, int method, int dtype, const void* h_
  * with copies; 1: always read in place.  Either way every input byte crosses the link once
  * per call.  Pageable input is staged through pinned buffers, except by -1 in a call of one
  * chunk of integer patterns (at most 64 MB) that the strip kernels serve: such input is read in
- * place too. */
+ * place too, and pinned integer input of a larger call that they serve is staged with copies
+ * (their packing would wait for the link). */
 int ebsd_plan_set_host_input(ebsd_plan_t plan, int mode);
 
-/* 1 when pinned host input is read in place under the plan's current mode, 0 when copied. */
+/* 1 when pinned host input is read in place under the plan's current mode, 0 when copied
+ * (under -1, 1 means: except the larger calls that ebsd_plan_set_host_input names). */
 int ebsd_plan_host_input_in_place(ebsd_plan_t plan);
 
 /* Number of kernel launches the last ebsd_find_bands / ebsd_find_bands_host call on this

@@ -585,16 +585,6 @@ void launch_average(dim3 tgrid, dim3 tblock, size_t tsmem, cudaStream_t st, cons
 // kernel also sums the four forward 3x3 neighbours under sigma_numba's saturation level, from
 // which k_nlpar_sigma_pairs takes the noise sigma without another pass over the patterns.
 __device__ __forceinline__ int fwd_count(int sr) { return sr * (2 * sr + 1) + sr; }
-__device__ __forceinline__ void fwd_offset(int f, int sr, int& dy, int& dx) {
-    if (f < sr) {
-        dy = 0;
-        dx = f + 1;
-    } else {
-        const int g = f - sr, w = 2 * sr + 1;
-        dy = 1 + g / w;
-        dx = g - (dy - 1) * w - sr;
-    }
-}
 __device__ __forceinline__ int fwd_index(int dy, int dx, int sr) {
     return dy == 0 ? dx - 1 : sr + (dy - 1) * (2 * sr + 1) + (dx + sr);
 }

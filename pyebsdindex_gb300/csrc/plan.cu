@@ -295,6 +295,14 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
             in_place = (const char*)pa.devicePointer;
         cudaGetLastError();
     }
+    // ... unless the strip path serves a call of more than kInPlaceBytes: its packing kernel would wait
+    // for the link in front of every chunk's sums (a million 80x80 patterns 4.8 M/s, staged by the copy
+    // engines beside them 6.7 M/s); without memory to stage it, it is read in place after all
+    if (in_place && p->host_input_mode == -1 && (size_t)n * src.pat_bytes > kInPlaceBytes &&
+        strip_serves(p, method, dtype)) {
+        if (regrow(p->h_in_dev, 2, &p->h_in_bytes, in_bytes, false) == EBSD_OK) in_place = nullptr;
+        cudaGetLastError();
+    }
     if (ring && src.mem && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
         strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0])) {
         int coherent = 0;
