@@ -38,15 +38,14 @@ METRIC = "band-detect patterns/sec on 1 GB300: batched FP16 vs plain FP32, at <=
 H = W = 80
 NRHO, NTHETA, NBANDS = 120, 180, 9
 BYTES_PER_PATTERN = H * W * 1 + 41 * NBANDS   # algorithmic bytes: pattern in, band fields out
-# DRAM bytes (read + write) per pattern of the fused kernel at eight patterns per pass, from an
-# ncu capture of the same launch configuration on 40,000 patterns (dram__bytes_read.sum +
-# dram__bytes_write.sum = 0.648 GB + 2.273 GB); the traffic grows with the patterns, so a
-# launch's traffic is this times its patterns.  Most of it is the write-back of the parked
-# ray means (seven rows per CTA per eight patterns), not input re-reads.
-DRAM_BYTES_PER_PATTERN = (648_438_528 + 2_272_787_200) / 40_000
-# warp instructions per pattern of the same kernel (ncu smsp__inst_executed.sum, same capture):
-# the issue roofline of an issue-bound kernel is 4 warp-instructions per SM per clock
-WARP_INST_PER_PATTERN = 6.546e9 / 40_000
+# DRAM bytes (read + write) per pattern of the strip kernels, from an ncu capture on 24,320
+# patterns (dram__bytes_read.sum + dram__bytes_write.sum, caches left as they are); the traffic
+# grows with the patterns.  Most of it is the Radon means (92 KB a pattern) on their way from the
+# word-sum kernel to the peak kernel, not input re-reads.
+DRAM_BYTES_PER_PATTERN = (2_646_938_368 + 2_656_966_656) / 24_320
+# warp instructions per pattern of the same kernels (ncu smsp__inst_executed.sum, same patterns):
+# the issue limit is 4 warp-instructions per SM per clock
+WARP_INST_PER_PATTERN = 1_555_847_103 / 24_320
 ACCURACY_PATTERNS = 32_768      # timed-batch patterns graded against plain64 (FP64 GPU oracle)
 ORACLE_PATTERNS = 2_048         # of those, graded against the oracle's FFT path (CPU leg)
 SEED = 1_000_000
@@ -794,7 +793,7 @@ def main():
         total_ms = float(t.item())
     value = world * N * args.steps / (total_ms / 1000.0)
 
-    # roofline: the dominant kernel (one fused launch per chunk, or the per-stage sequence)
+    # roofline of one step's kernels (the strip kernels chunk by chunk, or the per-stage sequence)
     hbm = None
     try:
         with open(os.path.join(ROOT, "MEASURED_PEAKS.json")) as f:
@@ -802,26 +801,23 @@ def main():
         hbm, peak_src = float(peaks["hbm_gbs"]), "measured"
     except Exception:
         hbm, peak_src = 6800.0, "fallback"
-    # fused methods launch the fused kernel plus a small float64 epilogue pass per chunk; the
-    # per-launch time is the step time per fused launch (the epilogue is ~0.01% of it)
-    fused_launches = max(launches_per_step // 2, 1)
-    launch_ms = float(np.mean(per_step)) / fused_launches if method.startswith("fused") else float(np.mean(per_step))
-    units_per_launch = N / fused_launches if method.startswith("fused") else N
+    launch_ms, units_per_launch = float(np.mean(per_step)), N
     achieved = BYTES_PER_PATTERN * units_per_launch / (launch_ms / 1000.0) / 1e9
     traffic = DRAM_BYTES_PER_PATTERN * units_per_launch if method == "fused" and ppp in (8, "rule: 8 for uint8 without background") else None
     roof = {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
-            "traffic": traffic, "traffic_source": "ncu capture, 40,000 patterns, scaled per pattern" if traffic else None,
+            "traffic": traffic, "traffic_source": "ncu capture, 24,320 patterns, scaled per pattern" if traffic else None,
             "peak_source": peak_src,
-            "kernel": "k_fused (+ k_band_epilogue)" if method.startswith("fused") else "per-stage sequence (7 kernels/chunk)"}
+            "kernel": {"fused": "k_strip_pack, k_strip_radon, k_strip_peaks, k_strip_fit per chunk",
+                       "fused16": "k_fused (+ k_band_epilogue)"}.get(method, "per-stage sequence (7 kernels/chunk)")}
     if method == "fused" and clocks.get("sm_mhz"):
-        # the roofline that binds this kernel: instruction issue, 4 warp-instructions per SM
-        # per clock at the sampled SM clock; warp-instructions per pattern from ncu
+        # instruction issue: 4 warp-instructions per SM per clock at the sampled SM clock;
+        # warp-instructions per pattern from ncu
         sms = torch.cuda.get_device_properties(dev).multi_processor_count
         issue_peak = 4.0 * sms * clocks["sm_mhz"] * 1e6
         issue_achieved = WARP_INST_PER_PATTERN * units_per_launch / (launch_ms / 1000.0)
         roof.update({"issue_achieved": issue_achieved, "issue_peak": issue_peak, "issue_unit": "warp-inst/s",
                      "issue_frac": issue_achieved / issue_peak,
-                     "issue_source": "smsp__inst_executed.sum per pattern from ncu (40,000 patterns); peak = 4 x SMs x "
+                     "issue_source": "smsp__inst_executed.sum per pattern from ncu (24,320 patterns); peak = 4 x SMs x "
                                      "median sampled SM clock"})
 
     # accuracy of the timed records: against the FP64 per-stage method (plain64, the FP64 GPU
@@ -873,8 +869,7 @@ def main():
         for _ in range(e2e_steps):
             soa_step()
         dt_soa = time.perf_counter() - t0
-        in_place = plan.host_input_in_place()
-        # the same with the input staged by copy engines instead of read in place
+        # the same with staging by copy engines asked for
         plan.set_host_input(0)
         soa_step()
         t0 = time.perf_counter()
@@ -889,8 +884,7 @@ def main():
                "call_s": [round(v, 4) for v in step_s],
                "c_abi_value": N * e2e_steps / dt_soa * world,
                "c_abi_call": "ebsd_find_bands_host, pinned patterns and pinned band-field arrays",
-               "c_abi_input_path": ("pinned patterns read in place by the kernels over NVLink-C2C (every byte crosses "
-                                    "the link each step)") if in_place else "pinned patterns staged by copy engines",
+               "c_abi_input_path": "the plan's default for pinned patterns: this many integer ones staged by copy engines",
                "c_abi_copy_engine_value": N * e2e_steps / dt_copy * world}
         del host, hout, host_np
 
