@@ -1147,7 +1147,7 @@ int ebsd_linop_apply_cols(ebsd_linop_t op, int fp64, const void* d_xT, int64_t l
     if (!op || n < 0 || (n > 0 && (!d_xT || !d_yT)) || ldx < n || ldy < n || (n + 31) / 32 > 65535) return EBSD_E_ARG;
     if (n == 0) return EBSD_OK;
     if (cudaSetDevice(op->device) != cudaSuccess) return EBSD_E_DEVICE;
-    // without an image the rows stand as one of kCsrTileX columns: a tile is 32 rows in a row
+    // without an image the rows stand as one of kCsrTileX columns: a tile is kCsrTileY * kCsrTileX rows in a row
     const int64_t width = op->width > 0 ? op->width : kCsrTileX;
     if ((op->nrows + kCsrTileY * width - 1) / (kCsrTileY * width) * ((width + kCsrTileX - 1) / kCsrTileX) > 0x7fffffff) return EBSD_E_ARG;
     cudaStream_t st = (cudaStream_t)stream;
