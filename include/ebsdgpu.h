@@ -150,7 +150,8 @@ int ebsd_find_bands_host(ebsd_plan_t plan, int method, int dtype, const void* h_
  * per call.  Pageable input is staged through pinned buffers, except by -1 in a call of one
  * chunk of integer patterns (at most 64 MB) that the strip kernels serve: such input is read in
  * place too, and pinned integer input of a larger call that they serve is staged with copies
- * (their packing would wait for the link). */
+ * (their packing would wait for the link).  Input whose address is no multiple of its type's
+ * size is staged in every mode. */
 int ebsd_plan_set_host_input(ebsd_plan_t plan, int mode);
 
 /* 1 when pinned host input is read in place under the plan's current mode, 0 when copied

@@ -283,10 +283,13 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         return EBSD_OK;
     };
     bool ring = !(src.mem && src.mem_pinned);
+    // Kernels load whole pixels, so input at an address that is no multiple of the pixel's size (a view
+    // of a byte buffer, a packed record's field) is never read in place: copies take any address.
+    const bool aligned = (uintptr_t)src.mem % elem_size(dtype) == 0;
     // pinned input read in place by the kernels over the CPU-GPU link (no staging copy) when
     // the device uses the host page tables (GB300's NVLink-C2C) or the caller asked for it
     const char* in_place = nullptr;
-    if (!ring && p->host_input_mode != 0) {
+    if (!ring && aligned && p->host_input_mode != 0) {
         int coherent = 0;
         cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
         cudaPointerAttributes pa;
@@ -303,7 +306,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         if (regrow(p->h_in_dev, 2, &p->h_in_bytes, in_bytes, false) == EBSD_OK) in_place = nullptr;
         cudaGetLastError();
     }
-    if (ring && src.mem && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
+    if (ring && src.mem && aligned && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
         strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0])) {
         int coherent = 0;
         cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
