@@ -359,7 +359,8 @@ struct PeakArgs {
     int64_t out_offset;
     float* cap;                         // slabs: [pattern][slab][capf]
     int capf;
-    double stat_scale;                  // 2^-20 / cells of the statistics slice
+    float stat_unit;                    // statistics sums are integers in units of 1 / stat_unit
+    double stat_scale;                  // 1 / stat_unit / cells of the statistics slice
 };
 
 __device__ __forceinline__ bool ahead(float v, int p, float w, int q) { return v > w || (v == w && p < q); }
@@ -412,9 +413,21 @@ __device__ __forceinline__ int merge_lists(V val, I pos, int nlist, int nB, int 
     return mine;
 }
 
-// Statistics sums are kept in units of 2^-20 as integers: exact in any order, so a record does not
-// depend on how a pattern was split over slabs and warps.
-constexpr float kStatUnit = 1048576.0f;
+// Statistics sums are kept as integers in a unit of the plan's: exact in any order, so a record does not
+// depend on how a pattern was split over slabs and warps.  The unit is the finest power of two for which no
+// sum of the plan's cells leaves 62 bits (80x80: 2^-37 for uint8, 2^-29 for uint16), far below the
+// float sums of four cells that are added in it, a dim pattern's too; the weights of those sums carry it, so
+// that it costs no instruction.
+double stat_unit(const ebsd_plan_s* p, int dtype, int statR) {
+    double gu = 0.0, gw = 0.0;
+    for (int k = 0; k < p->k0; ++k) gu += std::fabs((double)p->h_ku[k]);
+    for (int k = 0; k < p->k1; ++k) gw += std::fabs((double)p->h_kw[k]);
+    // means lie in [-1, 255] or [-1, 65535]; the float convolution's own rounding stays far below 1/256
+    const double most = (dtype == EBSD_U8 ? 256.0 : 65536.0) * gu * gw * ((double)std::max(statR, 1) * p->nTheta);
+    int e = 0;
+    std::frexp(most, &e);
+    return std::ldexp(1.0, 62 - e);
+}
 
 template <int K0, int K1, int NP>
 __global__ void __launch_bounds__(kPThreads, 2) k_strip_peaks(const __grid_constant__ PeakArgs a) {
@@ -497,9 +510,10 @@ __global__ void __launch_bounds__(kPThreads, 2) k_strip_peaks(const __grid_const
             const int i = oc + k - kOff;
             wgt[k] = !live || i < 0 ? 0.0f : (i < a.nRho + H0 ? (i < a.stat_hi ? 1.0f : 0.0f) : (i == a.nRho + H0 ? a.stat_last : 0.0f));
             out_of[k] = wgt[k] > 0.0f ? 0.0f : INFINITY;
+            wgt[k] *= a.stat_unit;
         }
         const bool tail = seg == a.nseg - 1 && a.nspecial > 0 && last_lane && live;
-        const float tail_out = tail ? 0.0f : INFINITY, tail_sum = tail ? a.special_sum : 0.0f;
+        const float tail_out = tail ? 0.0f : INFINITY, tail_sum = tail ? a.special_sum * a.stat_unit : 0.0f;
         // outside the Radon mask nothing is a candidate: values are cut off at -infinity there
         const uint8_t* mrow = a.mask + ((ptrdiff_t)ubase * a.FW + seg * 32 + lane);
         const unsigned mfix = live ? __ldg(a.mask + seg * 32 + lane) : 0u;
@@ -568,7 +582,7 @@ __global__ void __launch_bounds__(kPThreads, 2) k_strip_peaks(const __grid_const
                     for (int z = 0; z < H0; ++z) smin = fminf(smin, fmaf(e, a.special[z], tail_out));
                     smin = min3(smin, o[0] + out_of[0], o[1] + out_of[1]);
                     smin = min3(smin, o[2] + out_of[2], o[3] + out_of[3]);
-                    ssum += __float2ll_rn(rsum * kStatUnit);
+                    ssum += __float2ll_rn(rsum);
                 }
                 float left = __shfl_up_sync(0xffffffffu, o[3], 1), right = __shfl_down_sync(0xffffffffu, o[0], 1);
                 if (lane == 0) left = -INFINITY;
@@ -1297,7 +1311,9 @@ int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, co
     }
     for (int z = pa.nspecial; z < 4; ++z) pa.special[z] = pa.special[0];
     pa.special_sum = (float)ssum;
-    pa.stat_scale = 1.0 / ((double)kStatUnit * statR * p->nTheta);
+    const double unit = stat_unit(p, dtype, statR);
+    pa.stat_unit = (float)unit;
+    pa.stat_scale = 1.0 / (unit * statR * p->nTheta);
     pa.topk = p->nB + 6;
     for (int k = 0; k < 9; ++k) {
         pa.ku[k] = k < p->k0 ? p->h_ku[k] : 0.0f;
