@@ -155,8 +155,7 @@ struct ebsd_plan_s {
     // ---- workspaces ----
     std::mutex mtx;
     ebsd::Workspace st_ws;         // strip path: interleaved pixels, Radon means, slab peaks
-    cudaEvent_t st_event = nullptr;    // end of the last call that used st_ws, and its stream
-    cudaStream_t st_stream = nullptr;
+    cudaEvent_t st_event = nullptr;    // end of the last call that used st_ws
     ebsd::Workspace ws;            // per-stage intermediates
     ebsd::Workspace stats;         // per-pattern min/mean
     int64_t ws_chunk = 0;

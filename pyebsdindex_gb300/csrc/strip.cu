@@ -1328,11 +1328,12 @@ int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, co
     pa.cap = (float*)(ws + lay.cap);
     pa.capf = g.capf;
 
-    // the scratch passes from stream to stream in call order (captured work is ordered by its graph)
+    // the scratch passes from stream to stream in call order (captured work is ordered by its graph).  The wait
+    // is issued whatever the stream: a handle may be another stream's by now, or name one per thread.
     cudaStreamCaptureStatus capt = cudaStreamCaptureStatusNone;
     EBSD_CUDA_TRY(cudaStreamIsCapturing(st, &capt));
     const bool live = capt == cudaStreamCaptureStatusNone;
-    if (live && p->st_event && p->st_stream != st) EBSD_CUDA_TRY(cudaStreamWaitEvent(st, p->st_event, 0));
+    if (live && p->st_event) EBSD_CUDA_TRY(cudaStreamWaitEvent(st, p->st_event, 0));
 
     const size_t px = (size_t)p->nPx * elem_size(dtype);
     for (int64_t s = 0; s < n; s += g.chunk) {
@@ -1373,7 +1374,6 @@ int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, co
     if (live) {
         if (!p->st_event) EBSD_CUDA_TRY(cudaEventCreateWithFlags(&p->st_event, cudaEventDisableTiming));
         EBSD_CUDA_TRY(cudaEventRecord(p->st_event, st));
-        p->st_stream = st;
     }
     return launch_status();
 }
