@@ -16,6 +16,10 @@
  *     void*.  Plans own their device tables; callers own pattern and output buffers.
  *   - A plan may be used from one host thread at a time.  Calls on one plan with different
  *     streams are serialised by the plan's internal workspace lock.
+ *   - Band detection may be captured into CUDA graphs.  Integer patterns on the strip kernels get a
+ *     scratch of the graph's own, which goes back to the plan when the graph and its executables are
+ *     destroyed: replays may run beside other graphs and calls of the plan (not beside a second
+ *     executable of the same graph).  The other paths' workspace is the plan's: one plan per stream.
  */
 #ifndef EBSDGPU_H
 #define EBSDGPU_H
@@ -131,8 +135,8 @@ int ebsd_find_bands(ebsd_plan_t plan, int method, int dtype, const void* d_pats,
  * ebsd_method_supported(plan, EBSD_FUSED_F32) and qualify for the slab kernel (uint8 /
  * uint16 input; float32 where its pattern tile fits), else EBSD_E_UNSUPPORTED.  Records equal
  * those of ebsd_find_bands with EBSD_FUSED_F32 on each plan alone, up to the last bit of
- * normmax.  Asynchronous on `stream`; allocates nothing but a plan's strip scratch, once (never
- * during a stream capture). */
+ * normmax.  Asynchronous on `stream`; allocates nothing but a plan's strip scratch, once (and
+ * once for a graph that it is captured into). */
 int ebsd_find_bands_mixed(const ebsd_plan_t* plans, int nplans, int dtype, const void* const* d_pats,
                           const int64_t* n, const ebsd_bands* d_out, void* stream);
 

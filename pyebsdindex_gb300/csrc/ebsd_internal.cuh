@@ -5,6 +5,7 @@
 #include <cstdint>
 #include <cstddef>
 #include <algorithm>
+#include <memory>
 #include <mutex>
 #include <vector>
 
@@ -87,6 +88,13 @@ struct Workspace {
     size_t bytes = 0;
 };
 
+// The strip path's scratch: a buffer and the patterns that it holds at a time.
+struct StripScratch {
+    void* ptr = nullptr;
+    int64_t cap = 0;
+};
+struct StripCaptures;                  // the scratch buffers of captured calls (strip.cu)
+
 }  // namespace ebsd
 
 struct ebsd_plan_s {
@@ -154,8 +162,9 @@ struct ebsd_plan_s {
 
     // ---- workspaces ----
     std::mutex mtx;
-    ebsd::Workspace st_ws;         // strip path: interleaved pixels, Radon means, slab peaks
+    ebsd::StripScratch st_ws;      // strip path: interleaved pixels, Radon means, slab peaks
     cudaEvent_t st_event = nullptr;    // end of the last call that used st_ws
+    std::shared_ptr<ebsd::StripCaptures> st_captures;  // the like of st_ws for captured calls
     ebsd::Workspace ws;            // per-stage intermediates
     ebsd::Workspace stats;         // per-pattern min/mean
     int64_t ws_chunk = 0;
@@ -250,8 +259,8 @@ int slab_run_chunk(ebsd_plan_s* p, int method, int dtype, const void* d_pats, in
 int strip_prepare(ebsd_plan_s* p, const ebsd_plan_desc* d);
 void strip_release(ebsd_plan_s* p);
 bool strip_serves(const ebsd_plan_s* p, int method, int dtype);
-int strip_reserve(ebsd_plan_s* p);
-bool strip_ready(ebsd_plan_s* p, cudaStream_t st);
+int strip_reserve(ebsd_plan_s* p, int64_t n);
+bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got = nullptr);
 int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
                     cudaStream_t st, int64_t* launches);
 

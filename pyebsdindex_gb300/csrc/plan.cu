@@ -88,7 +88,7 @@ size_t workspace_bytes(const ebsd_plan_s* p, int method, int64_t chunk) {
 // Scratch of a call: the strip path's for the input types it takes, else (or when the device has no
 // room for that) the method's own.
 int reserve(ebsd_plan_s* p, int method, int64_t chunk, int dtype, cudaStream_t st) {
-    if (strip_serves(p, method, dtype) && strip_ready(p, st)) return EBSD_OK;
+    if (strip_serves(p, method, dtype) && strip_ready(p, st, chunk)) return EBSD_OK;
     size_t need = workspace_bytes(p, method, chunk);
     if (need > p->ws.bytes) {
         cudaFree(p->ws.ptr);
@@ -258,14 +258,14 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
     if (chunk <= 0) chunk = is_plain(method) ? default_chunk(p, method) : 65536;
     if (is_plain(method)) chunk = std::min<int64_t>(chunk, 65535);
     chunk = std::min(chunk, n);
+    for (int i = 0; i < 2; ++i) {
+        if (!p->hstream[i]) EBSD_CUDA_TRY(cudaStreamCreateWithFlags(&p->hstream[i], cudaStreamNonBlocking));
+    }
     int rc = reserve(p, method, chunk, dtype, p->hstream[0]);
     if (rc != EBSD_OK) return rc;
     const int nB = p->nB;
     const size_t in_bytes = (size_t)chunk * src.pat_bytes;
     const size_t out_bytes = (size_t)chunk * nB * (10 * sizeof(float) + 1) + 256;
-    for (int i = 0; i < 2; ++i) {
-        if (!p->hstream[i]) EBSD_CUDA_TRY(cudaStreamCreateWithFlags(&p->hstream[i], cudaStreamNonBlocking));
-    }
     for (cudaEvent_t& e : p->hpipe)
         if (!e) EBSD_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     auto regrow = [](void** bufs, int count, size_t* have, size_t want, bool host) -> int {
@@ -307,7 +307,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         cudaGetLastError();
     }
     if (ring && src.mem && aligned && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
-        strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0])) {
+        strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0], n)) {
         int coherent = 0;
         cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
         if (coherent) {
@@ -712,7 +712,7 @@ int ebsd_plan_reserve(ebsd_plan_t p, int method, int64_t max_chunk) {
     std::lock_guard<std::mutex> lk(p->mtx);
     if (cudaSetDevice(p->device) != cudaSuccess) return EBSD_E_DEVICE;
     // every input type: the strip path's scratch (integers) and the method's own
-    if (method == EBSD_FUSED_F32) strip_reserve(p);
+    if (method == EBSD_FUSED_F32) strip_reserve(p, max_chunk);
     return reserve(p, method, is_plain(method) ? std::min<int64_t>(max_chunk, 65535) : max_chunk, EBSD_F32, nullptr);
 }
 
@@ -769,7 +769,8 @@ int ebsd_find_bands_mixed(const ebsd_plan_t* plans, int nplans, int dtype, const
     int64_t launches = 0;
     cudaStream_t st = (cudaStream_t)stream;
     bool strips = true;
-    for (ebsd_plan_s* p : ps) strips = strips && strip_serves(p, EBSD_FUSED_F32, dtype) && strip_ready(p, st);
+    for (int k = 0; k < nplans && strips; ++k)
+        strips = strip_serves(ps[k], EBSD_FUSED_F32, dtype) && strip_ready(ps[k], st, n[k]);
     int rc = EBSD_OK;
     if (strips) {  // size by size: each fills the GPU by itself
         for (int k = 0; k < nplans && rc == EBSD_OK; ++k)
@@ -934,7 +935,7 @@ int ebsd_plan_autotune(ebsd_plan_t p, int method, int dtype, const void* d_pats,
     }
     rc = reserve(p, method, n, dtype, st);
     if (rc != EBSD_OK) return rc;
-    if (strip_serves(p, method, dtype) && strip_ready(p, st)) {
+    if (strip_serves(p, method, dtype) && strip_ready(p, st, n)) {
         // one variant: the strip path takes these calls whatever the tile shape
         p->fused_ppp = -1;
         if (patterns_per_pass) *patterns_per_pass = dtype == EBSD_U8 ? 8 : 1;

@@ -1153,6 +1153,57 @@ int strip_prepare(ebsd_plan_s* p, const ebsd_plan_desc* d) {
     return EBSD_OK;
 }
 
+// The scratch of a captured call belongs to the graph that the capture builds: its replays run whenever they
+// are launched, beside other graphs and direct calls of the plan.  The graph holds a user object whose
+// destructor, when the graph and its executables are gone, marks the buffer free for a later capture.
+// The plan frees the buffers with its tables.
+struct StripCaptures {
+    struct Slot {
+        StripScratch mem;
+        bool held = false;
+        unsigned long long id = 0;      // the capture and the stream: calls captured one after the other on
+        cudaStream_t stream = nullptr;  // one stream share the buffer
+    };
+    std::mutex m;                       // never held over a call of the runtime
+    std::vector<std::unique_ptr<Slot>> slots;
+};
+
+namespace {
+
+struct CaptureHold {
+    std::shared_ptr<StripCaptures> pool;
+    StripCaptures::Slot* slot;
+};
+
+void CUDART_CB capture_gone(void* arg) {
+    CaptureHold* h = (CaptureHold*)arg;
+    {
+        std::lock_guard<std::mutex> lk(h->pool->m);
+        h->slot->held = false;
+        h->slot->id = 0;
+    }
+    delete h;
+}
+
+void captures_release(ebsd_plan_s* p) {
+    if (!p->st_captures) return;
+    for (auto& s : p->st_captures->slots) {  // (the plan's lock guards the list and the buffers)
+        cudaFree(s->mem.ptr);
+        s->mem = StripScratch{};
+    }
+    p->st_captures.reset();
+}
+
+// This thread's allocations neither fail in nor end a capture that runs in the process: its own, on
+// whatever stream, or another thread's in global mode.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+}  // namespace
+
 void strip_release(ebsd_plan_s* p) {
     cudaFree(p->d_st_tasks);
     cudaFree(p->d_st_lut);
@@ -1167,7 +1218,8 @@ void strip_release(ebsd_plan_s* p) {
     p->d_st_mask = nullptr;
     p->d_st_used = nullptr;
     cudaFree(p->st_ws.ptr);
-    p->st_ws = Workspace{};
+    p->st_ws = StripScratch{};
+    captures_release(p);
     if (p->st_event) cudaEventDestroy(p->st_event);
     p->st_event = nullptr;
     p->st = StripGeom{};
@@ -1189,13 +1241,14 @@ struct StripLayout {
     size_t elems, means, cap, total;
 };
 
-StripLayout strip_layout(const StripGeom& g) {
+// of a scratch that holds n patterns
+StripLayout strip_layout(const StripGeom& g, int64_t n) {
     StripLayout l;
     l.elems = 0;
     // uint16 patterns go four to a unit, uint8 eight
-    l.means = align256(((size_t)g.chunk + 3) / 4 * g.unit_elems * 8);
-    l.cap = l.means + align256((size_t)g.chunk * g.nRaysPad * 4);
-    const size_t blocks = std::max<size_t>((size_t)g.chunk * g.nslab, (size_t)8 * g.sms);
+    l.means = align256(((size_t)n + 3) / 4 * g.unit_elems * 8);
+    l.cap = l.means + align256((size_t)n * g.nRaysPad * 4);
+    const size_t blocks = std::max<size_t>((size_t)n * g.nslab, (size_t)8 * g.sms);
     l.total = l.cap + align256(blocks * g.capf * 4);
     return l;
 }
@@ -1224,41 +1277,119 @@ int strip_attr(const void* fn, int device, int smem) {
 
 }  // namespace
 
-// The plan's scratch, allocated once for any number of patterns.
-int strip_reserve(ebsd_plan_s* p) {
-    if (!p->st.ok || p->st_ws.ptr) return EBSD_OK;
-    const size_t need = strip_layout(p->st).total;
+namespace {
+
+// Patterns of a scratch for calls of n: a whole pass.
+int64_t scratch_cap(const StripGeom& g, int64_t) { return g.chunk; }
+
+int scratch_alloc(const StripGeom& g, int64_t cap, StripScratch* out) {
     void* ptr = nullptr;
-    const cudaError_t e = cudaMalloc(&ptr, need);
+    const cudaError_t e = cudaMalloc(&ptr, strip_layout(g, cap).total);
     if (e != cudaSuccess) {
         cudaGetLastError();
         return e == cudaErrorMemoryAllocation ? EBSD_E_NOMEM : EBSD_E_LAUNCH;
     }
-    p->st_ws.ptr = ptr;
-    p->st_ws.bytes = need;
+    *out = StripScratch{ptr, cap};
     return EBSD_OK;
 }
 
-// Whether a call on `st` can use the scratch: allocated now if it is not, unless the stream is being
-// captured (an allocation would end the capture) or memory is short -- the single-kernel paths then
-// serve the call.
-bool strip_ready(ebsd_plan_s* p, cudaStream_t st) {
-    if (p->st_ws.ptr) return true;
+// Scratch for n patterns of a call on `st`, which is being captured into `graph`.
+bool capture_scratch(ebsd_plan_s* p, cudaStream_t st, unsigned long long id, cudaGraph_t graph, int64_t n, StripScratch* got) {
+    if (!p->st_captures) p->st_captures = std::make_shared<StripCaptures>();
+    StripCaptures& c = *p->st_captures;
+    const int64_t cap = scratch_cap(p->st, n);
+    StripCaptures::Slot *slot = nullptr, *small = nullptr;
+    {
+        std::lock_guard<std::mutex> lk(c.m);
+        for (auto& s : c.slots) {
+            const bool fits = s->mem.cap >= cap;
+            if (s->held && s->id == id && s->stream == st && fits) {
+                *got = s->mem;
+                return true;
+            }
+            if (s->held) continue;
+            if (!fits) small = s.get();
+            else if (!slot || s->mem.cap < slot->mem.cap) slot = s.get();
+        }
+        if (!slot) slot = small;  // a buffer that no graph holds makes room for a larger one
+        if (!slot) {
+            c.slots.emplace_back(new StripCaptures::Slot());
+            slot = c.slots.back().get();
+        }
+        slot->held = true;
+    }
+    auto give_back = [&] {
+        std::lock_guard<std::mutex> lk(c.m);
+        slot->held = false;
+        return false;
+    };
+    const RelaxedCapture relaxed;
+    if (slot->mem.cap < cap) {
+        cudaFree(slot->mem.ptr);
+        slot->mem = StripScratch{};
+        if (scratch_alloc(p->st, cap, &slot->mem) != EBSD_OK) return give_back();
+    }
+    CaptureHold* hold = new CaptureHold{p->st_captures, slot};
+    cudaUserObject_t obj = nullptr;
+    if (cudaUserObjectCreate(&obj, hold, capture_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
+        cudaGetLastError();
+        delete hold;
+        return give_back();
+    }
+    if (cudaGraphRetainUserObject(graph, obj, 1, cudaGraphUserObjectMove) != cudaSuccess) {
+        cudaGetLastError();
+        cudaUserObjectRelease(obj, 1);  // capture_gone gives it back
+        return false;
+    }
+    std::lock_guard<std::mutex> lk(c.m);
+    slot->id = id;
+    slot->stream = st;
+    *got = slot->mem;
+    return true;
+}
+
+}  // namespace
+
+// The plan's own scratch, for calls of up to n patterns, or of any number in passes.
+int strip_reserve(ebsd_plan_s* p, int64_t n) {
+    if (!p->st.ok) return EBSD_OK;
+    const int64_t cap = scratch_cap(p->st, n);
+    if (p->st_ws.ptr && p->st_ws.cap >= cap) return EBSD_OK;
+    const RelaxedCapture relaxed;
+    cudaFree(p->st_ws.ptr);  // (waits for the calls in flight that use it)
+    p->st_ws = StripScratch{};
+    return scratch_alloc(p->st, cap, &p->st_ws);
+}
+
+// Whether a call of n patterns on `st` has scratch, allocated now if need be: the plan's own, or the
+// graph's if the call is being captured.  Where memory is short the single-kernel paths serve the call.
+bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) {
+    unsigned long long id = 0;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(st, &cap, &id, &graph, nullptr, nullptr, nullptr) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return cap == cudaStreamCaptureStatusNone && strip_reserve(p) == EBSD_OK;
+    StripScratch s;
+    if (cap == cudaStreamCaptureStatusActive) {
+        if (!capture_scratch(p, st, id, graph, n, &s)) return false;
+    } else {
+        if (cap != cudaStreamCaptureStatusNone || strip_reserve(p, n) != EBSD_OK) return false;
+        s = p->st_ws;
+    }
+    if (got) *got = s;
+    return true;
 }
 
 int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
                     cudaStream_t st, int64_t* launches) {
     if (n <= 0) return EBSD_OK;
     const StripGeom& g = p->st;
-    if (!p->st_ws.ptr) return EBSD_E_NOMEM;
-    const StripLayout lay = strip_layout(g);
-    char* ws = (char*)p->st_ws.ptr;
+    StripScratch scratch;
+    if (!strip_ready(p, st, n, &scratch)) return EBSD_E_NOMEM;
+    const StripLayout lay = strip_layout(g, scratch.cap);
+    char* ws = (char*)scratch.ptr;
     const int K0 = p->k0, H0 = K0 / 2, nR = p->nRho;
     const int per = dtype == EBSD_U8 ? 8 : 4;
     void* rfn = radon_kernel(g.SB, dtype);
@@ -1328,16 +1459,14 @@ int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, co
     pa.cap = (float*)(ws + lay.cap);
     pa.capf = g.capf;
 
-    // the scratch passes from stream to stream in call order (captured work is ordered by its graph).  The wait
-    // is issued whatever the stream: a handle may be another stream's by now, or name one per thread.
-    cudaStreamCaptureStatus capt = cudaStreamCaptureStatusNone;
-    EBSD_CUDA_TRY(cudaStreamIsCapturing(st, &capt));
-    const bool live = capt == cudaStreamCaptureStatusNone;
+    // the plan's own scratch passes from stream to stream in call order (a graph's is ordered by the graph).
+    // The wait is issued whatever the stream: a handle may be another stream's by now, or name one per thread.
+    const bool live = scratch.ptr == p->st_ws.ptr;
     if (live && p->st_event) EBSD_CUDA_TRY(cudaStreamWaitEvent(st, p->st_event, 0));
 
     const size_t px = (size_t)p->nPx * elem_size(dtype);
-    for (int64_t s = 0; s < n; s += g.chunk) {
-        const int64_t m = std::min<int64_t>(g.chunk, n - s);
+    for (int64_t s = 0; s < n; s += scratch.cap) {
+        const int64_t m = std::min<int64_t>(scratch.cap, n - s);
         const unsigned units = (unsigned)((m + per - 1) / per);
         const void* in = (const char*)d_pats + (size_t)s * px;
         // tiles over both copies: x up to max(U0, W + apron) and y likewise, from -kApron
