@@ -711,8 +711,11 @@ int ebsd_plan_reserve(ebsd_plan_t p, int method, int64_t max_chunk) {
     if (rc != EBSD_OK) return rc;
     std::lock_guard<std::mutex> lk(p->mtx);
     if (cudaSetDevice(p->device) != cudaSuccess) return EBSD_E_DEVICE;
-    // every input type: the strip path's scratch (integers) and the method's own
-    if (method == EBSD_FUSED_F32) strip_reserve(p, max_chunk);
+    // the strip path's scratch, which is all that integer calls take; the one-tile kernel's own is for uint8
+    // patterns that the strip path does not serve
+    if (method == EBSD_FUSED_F32 && strip_serves(p, method, EBSD_U16) && strip_reserve(p, max_chunk) == EBSD_OK &&
+        strip_serves(p, method, EBSD_U8))
+        return EBSD_OK;
     return reserve(p, method, is_plain(method) ? std::min<int64_t>(max_chunk, 65535) : max_chunk, EBSD_F32, nullptr);
 }
 

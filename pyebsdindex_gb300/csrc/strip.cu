@@ -1279,8 +1279,13 @@ int strip_attr(const void* fn, int device, int smem) {
 
 namespace {
 
-// Patterns of a scratch for calls of n: a whole pass.
-int64_t scratch_cap(const StripGeom& g, int64_t) { return g.chunk; }
+// Patterns of a scratch for calls of n: powers of two up to a whole pass (0.3 GB at 80x80), so that a plan
+// of small calls stays small and calls of growing size allocate a few times at most.
+int64_t scratch_cap(const StripGeom& g, int64_t n) {
+    int64_t cap = 64;
+    while (cap < n && cap < g.chunk) cap *= 2;
+    return std::min(cap, g.chunk);
+}
 
 int scratch_alloc(const StripGeom& g, int64_t cap, StripScratch* out) {
     void* ptr = nullptr;
