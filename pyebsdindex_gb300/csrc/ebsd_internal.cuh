@@ -260,8 +260,9 @@ int strip_prepare(ebsd_plan_s* p, const ebsd_plan_desc* d);
 void strip_release(ebsd_plan_s* p);
 bool strip_serves(const ebsd_plan_s* p, int method, int dtype);
 int strip_reserve(ebsd_plan_s* p, int64_t n);
-bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got = nullptr);
-int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
+bool strip_has(const ebsd_plan_s* p, int64_t n);
+bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got);
+int strip_run_chunk(ebsd_plan_s* p, const StripScratch& scratch, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
                     cudaStream_t st, int64_t* launches);
 
 // mixed pattern sizes in one launch: up to 8 plans of one input type and LoG size

@@ -88,7 +88,8 @@ size_t workspace_bytes(const ebsd_plan_s* p, int method, int64_t chunk) {
 // Scratch of a call: the strip path's for the input types it takes, else (or when the device has no
 // room for that) the method's own.
 int reserve(ebsd_plan_s* p, int method, int64_t chunk, int dtype, cudaStream_t st) {
-    if (strip_serves(p, method, dtype) && strip_ready(p, st, chunk)) return EBSD_OK;
+    StripScratch strip;
+    if (strip_serves(p, method, dtype) && (strip_has(p, chunk) || strip_ready(p, st, chunk, &strip))) return EBSD_OK;
     size_t need = workspace_bytes(p, method, chunk);
     if (need > p->ws.bytes) {
         cudaFree(p->ws.ptr);
@@ -307,7 +308,7 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
         cudaGetLastError();
     }
     if (ring && src.mem && aligned && p->host_input_mode == -1 && chunk == n && in_bytes <= kInPlaceBytes &&
-        strip_serves(p, method, dtype) && strip_ready(p, p->hstream[0], n)) {
+        strip_serves(p, method, dtype) && strip_has(p, n)) {
         int coherent = 0;
         cudaDeviceGetAttribute(&coherent, cudaDevAttrPageableMemoryAccessUsesHostPageTables, p->device);
         if (coherent) {
@@ -771,13 +772,18 @@ int ebsd_find_bands_mixed(const ebsd_plan_t* plans, int nplans, int dtype, const
     std::vector<ebsd_plan_s*> ps(plans, plans + nplans);
     int64_t launches = 0;
     cudaStream_t st = (cudaStream_t)stream;
+    StripScratch scratch;
     bool strips = true;
     for (int k = 0; k < nplans && strips; ++k)
-        strips = strip_serves(ps[k], EBSD_FUSED_F32, dtype) && strip_ready(ps[k], st, n[k]);
+        strips = strip_serves(ps[k], EBSD_FUSED_F32, dtype) && strip_ready(ps[k], st, n[k], &scratch);
     int rc = EBSD_OK;
     if (strips) {  // size by size: each fills the GPU by itself
-        for (int k = 0; k < nplans && rc == EBSD_OK; ++k)
-            rc = strip_run_chunk(ps[k], dtype, d_pats[k], n[k], &d_out[k], 0, st, &launches);
+        for (int k = 0; k < nplans && rc == EBSD_OK; ++k) {
+            // (looked up again: a plan that is listed twice may have grown its scratch above)
+            rc = strip_ready(ps[k], st, n[k], &scratch)
+                     ? strip_run_chunk(ps[k], scratch, dtype, d_pats[k], n[k], &d_out[k], 0, st, &launches)
+                     : EBSD_E_NOMEM;
+        }
     } else {
         rc = slab_run_mixed(ps.data(), nplans, dtype, d_pats, n, d_out, st, &launches);
     }
@@ -938,7 +944,8 @@ int ebsd_plan_autotune(ebsd_plan_t p, int method, int dtype, const void* d_pats,
     }
     rc = reserve(p, method, n, dtype, st);
     if (rc != EBSD_OK) return rc;
-    if (strip_serves(p, method, dtype) && strip_ready(p, st, n)) {
+    StripScratch strip;
+    if (strip_serves(p, method, dtype) && (strip_has(p, n) || strip_ready(p, st, n, &strip))) {
         // one variant: the strip path takes these calls whatever the tile shape
         p->fused_ppp = -1;
         if (patterns_per_pass) *patterns_per_pass = dtype == EBSD_U8 ? 8 : 1;

@@ -1355,18 +1355,20 @@ bool capture_scratch(ebsd_plan_s* p, cudaStream_t st, unsigned long long id, cud
 
 }  // namespace
 
+// Whether the plan's own scratch is there for calls of n patterns.
+bool strip_has(const ebsd_plan_s* p, int64_t n) { return p->st_ws.ptr && p->st_ws.cap >= scratch_cap(p->st, n); }
+
 // The plan's own scratch, for calls of up to n patterns, or of any number in passes.
 int strip_reserve(ebsd_plan_s* p, int64_t n) {
     if (!p->st.ok) return EBSD_OK;
-    const int64_t cap = scratch_cap(p->st, n);
-    if (p->st_ws.ptr && p->st_ws.cap >= cap) return EBSD_OK;
+    if (strip_has(p, n)) return EBSD_OK;
     const RelaxedCapture relaxed;
     cudaFree(p->st_ws.ptr);  // (waits for the calls in flight that use it)
     p->st_ws = StripScratch{};
-    return scratch_alloc(p->st, cap, &p->st_ws);
+    return scratch_alloc(p->st, scratch_cap(p->st, n), &p->st_ws);
 }
 
-// Whether a call of n patterns on `st` has scratch, allocated now if need be: the plan's own, or the
+// Whether a call of n patterns on `st` has scratch (*got), allocated now if need be: the plan's own, or the
 // graph's if the call is being captured.  Where memory is short the single-kernel paths serve the call.
 bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
@@ -1376,23 +1378,16 @@ bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got) 
         cudaGetLastError();
         return false;
     }
-    StripScratch s;
-    if (cap == cudaStreamCaptureStatusActive) {
-        if (!capture_scratch(p, st, id, graph, n, &s)) return false;
-    } else {
-        if (cap != cudaStreamCaptureStatusNone || strip_reserve(p, n) != EBSD_OK) return false;
-        s = p->st_ws;
-    }
-    if (got) *got = s;
+    if (cap == cudaStreamCaptureStatusActive) return capture_scratch(p, st, id, graph, n, got);
+    if (cap != cudaStreamCaptureStatusNone || strip_reserve(p, n) != EBSD_OK) return false;
+    *got = p->st_ws;
     return true;
 }
 
-int strip_run_chunk(ebsd_plan_s* p, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out, int64_t out_offset,
-                    cudaStream_t st, int64_t* launches) {
+int strip_run_chunk(ebsd_plan_s* p, const StripScratch& scratch, int dtype, const void* d_pats, int64_t n, const ebsd_bands* out,
+                    int64_t out_offset, cudaStream_t st, int64_t* launches) {
     if (n <= 0) return EBSD_OK;
     const StripGeom& g = p->st;
-    StripScratch scratch;
-    if (!strip_ready(p, st, n, &scratch)) return EBSD_E_NOMEM;
     const StripLayout lay = strip_layout(g, scratch.cap);
     char* ws = (char*)scratch.ptr;
     const int K0 = p->k0, H0 = K0 / 2, nR = p->nRho;
