@@ -181,12 +181,14 @@ int64_t ebsd_last_launch_count(ebsd_plan_t plan);
 int ebsd_plan_autotune(ebsd_plan_t plan, int method, int dtype, const void* d_pats, int64_t n,
                        void* stream, int* patterns_per_pass);
 
-/* Pins the fused kernel's patterns per block pass for later calls: 1, 2, 4 or 8 (capped at what
- * a call allows), or 0 for the rule (the most a call allows).  For callers that tuned
- * offline; no counterpart in the reference.  Records do not depend on the choice. */
+/* Pins the one-tile kernel's patterns per block pass for later calls: 1, 2, 4 or 8 (capped at what
+ * a call allows), or 0 for the rule (the most a call allows).  It matters where that kernel runs
+ * (EBSD_FUSED_F16, or EBSD_FUSED_F32 with tile 1 pinned or where the strip kernels do not serve).  For
+ * callers that tuned offline; no counterpart in the reference.  Records do not depend on the choice. */
 int ebsd_plan_set_patterns_per_pass(ebsd_plan_t plan, int patterns_per_pass);
 
-/* The plan's Radon tile shape for EBSD_FUSED_F32 calls (no counterpart in the reference). */
+/* The plan's Radon tile shape for the EBSD_FUSED_F32 calls that ebsd_plan_strip_serves does not name
+ * (no counterpart in the reference). */
 typedef struct {
     int tile;               /* 1: the whole padded Radon image as one tile (when it fits);
                                2: theta slabs; 0: neither fits (per-stage methods only) */
@@ -203,8 +205,15 @@ typedef struct {
 
 int ebsd_plan_get_tile(ebsd_plan_t plan, ebsd_tile_info* info);
 
-/* Pins the Radon tile shape for later EBSD_FUSED_F32 calls: tile 1 one tile, 2 theta slabs,
- * 0 the rule (one tile when it fits); slabs = the slab count for the slab tables, in
+/* 1 when the strip kernels serve `method` on `dtype` under the plan's settings (EBSD_FUSED_F32 on
+ * integer patterns of a plan they can take, no tile shape pinned), else 0 or a negative code.  A
+ * call without memory for their scratch takes the tile shape instead. */
+int ebsd_plan_strip_serves(ebsd_plan_t plan, int method, int dtype);
+
+/* Pins the Radon tile shape for later EBSD_FUSED_F32 calls, integer ones and ebsd_find_bands_mixed
+ * among them: tile 1 one tile, 2 theta slabs (a mixed call runs slabs in either case), 0 the rule
+ * (the strip kernels where they serve, else one tile when it fits); ebsd_plan_autotune chooses
+ * afresh and ends the pin.  slabs = the slab count for the slab tables, in
  * [slabs_min, slabs_max], or 0 for the widest.  The slab tables also serve
  * ebsd_find_bands_mixed.  EBSD_E_UNSUPPORTED for a shape the plan cannot take.  Waits for
  * the device when it rebuilds the slab tables, and frees the old ones: a CUDA graph captured

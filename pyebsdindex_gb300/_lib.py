@@ -111,6 +111,8 @@ def load():
         lib.ebsd_plan_get_tile.restype = C.c_int
         lib.ebsd_plan_set_tile.argtypes = [P, C.c_int, C.c_int]
         lib.ebsd_plan_set_tile.restype = C.c_int
+        lib.ebsd_plan_strip_serves.argtypes = [P, C.c_int, C.c_int]
+        lib.ebsd_plan_strip_serves.restype = C.c_int
         lib.ebsd_strerror.argtypes = [C.c_int]
         lib.ebsd_strerror.restype = C.c_char_p
         lib.ebsd_version.argtypes = []
@@ -193,7 +195,7 @@ class DevicePlan:
         return int(self._lib.ebsd_last_launch_count(self.handle))
 
     def set_patterns_per_pass(self, ppp: int):
-        """Pin the fused kernel's patterns per block pass (1, 2, 4, 8; 0 = rule)."""
+        """Pin the one-tile kernel's patterns per block pass (1, 2, 4, 8; 0 = rule)."""
         check(self._lib.ebsd_plan_set_patterns_per_pass(self.handle, int(ppp)), "ebsd_plan_set_patterns_per_pass")
 
     def get_tile(self) -> dict:
@@ -204,8 +206,17 @@ class DevicePlan:
         check(self._lib.ebsd_plan_get_tile(self.handle, C.byref(t)), "ebsd_plan_get_tile")
         return {f: int(getattr(t, f)) for f, _ in TileInfo._fields_}
 
+    def strip_serves(self, method, dtype) -> bool:
+        """Whether the strip kernels run calls of ``method`` on ``dtype`` (an EBSD_* code): integer
+        patterns, FP32 fused method, no tile shape pinned (``ebsd_plan_strip_serves``)."""
+        r = self._lib.ebsd_plan_strip_serves(self.handle, method_id(method), int(dtype))
+        if r < 0:
+            check(r, "ebsd_plan_strip_serves")
+        return r == 1
+
     def set_tile(self, tile: int, slabs: int = 0):
-        """Pin the Radon tile shape: ``tile`` 1 one tile, 2 theta slabs, 0 the rule; ``slabs``
+        """Pin the Radon tile shape: ``tile`` 1 one tile, 2 theta slabs, 0 the rule (the strip
+        kernels where they serve, else one tile if it fits); ``slabs``
         the slab count (0 = the widest that fit).  A new slab count rebuilds the slab tables
         (the device is synchronised and the old tables freed): capture CUDA graphs after it."""
         check(self._lib.ebsd_plan_set_tile(self.handle, int(tile), int(slabs)), "ebsd_plan_set_tile")

@@ -274,9 +274,15 @@ class GPUFindBands:
             if hit is not None and int(hit.get("patterns_per_pass", 0)) in (1, 2, 4, 8):
                 ppp = int(hit["patterns_per_pass"])
                 tile, slabs = int(hit.get("tile", 0)), int(hit.get("slabs", 0))
+                slabs = slabs if tile == 2 else 0
+                integer = dt in (_lib.EBSD_U8, _lib.EBSD_U16) and m in ("fused", "fused32")
                 try:
                     if tile in (1, 2):
-                        plan.set_tile(tile, slabs if tile == 2 else 0)
+                        # the tables' slab count, and no shape pinned where the strip kernels serve
+                        if integer:
+                            plan.set_tile(0, slabs)
+                        if not (integer and plan.strip_serves(m, dt)):
+                            plan.set_tile(tile, slabs)
                     plan.set_patterns_per_pass(ppp)
                 except RuntimeError:
                     hit = None  # a shape this plan cannot take: tune afresh

@@ -150,6 +150,7 @@ struct ebsd_plan_s {
     // FP32 fused calls that both kernels can serve: 0 rule (the single tile when it fits),
     // 1 the single tile, 2 theta slabs (ebsd_plan_set_tile, ebsd_plan_autotune)
     int tile_mode = 0;
+    bool tile_pinned = false;      // set by ebsd_plan_set_tile: integer calls run that shape too, not the strip kernels
 
     // strip-word tables (see strip.cu)
     ebsd::StripGeom st;

@@ -909,7 +909,16 @@ int ebsd_plan_set_tile(ebsd_plan_t p, int tile, int slabs) {
         if (rc != EBSD_OK) return rc;
     }
     p->tile_mode = tile;
+    p->tile_pinned = tile != 0;
     return EBSD_OK;
+}
+
+int ebsd_plan_strip_serves(ebsd_plan_t p, int method, int dtype) {
+    if (!p) return EBSD_E_ARG;
+    if (dtype != EBSD_U8 && dtype != EBSD_U16 && dtype != EBSD_F32) return EBSD_E_DTYPE;
+    if (!is_plain(method) && !is_fused(method)) return EBSD_E_ARG;
+    std::lock_guard<std::mutex> lk(p->mtx);
+    return strip_serves(p, method, dtype) ? 1 : 0;
 }
 
 int ebsd_plan_get_tile(ebsd_plan_t p, ebsd_tile_info* info) {
@@ -942,11 +951,12 @@ int ebsd_plan_autotune(ebsd_plan_t p, int method, int dtype, const void* d_pats,
         if (patterns_per_pass) *patterns_per_pass = 1;
         return EBSD_OK;
     }
+    p->tile_pinned = false;  // the choice is this call's from here on
     rc = reserve(p, method, n, dtype, st);
     if (rc != EBSD_OK) return rc;
     StripScratch strip;
     if (strip_serves(p, method, dtype) && (strip_has(p, n) || strip_ready(p, st, n, &strip))) {
-        // one variant: the strip path takes these calls whatever the tile shape
+        // one variant: the strip path takes these calls while no tile shape is pinned
         p->fused_ppp = -1;
         if (patterns_per_pass) *patterns_per_pass = dtype == EBSD_U8 ? 8 : 1;
         return EBSD_OK;

@@ -1229,8 +1229,9 @@ void strip_release(ebsd_plan_s* p) {
 // the eight-pattern one-tile kernel (fused.cu) takes: there the peak kernel's register ring spills, and
 // 30,011 patterns of 60x60 took 5.4 ms here against 4.85 ms (80x80, too large for that tile: 8.2 ms for
 // 20,000 against 11.6 in theta slabs; with five taps 60x60 is faster here as well).
+// Nor are they served here while the caller pins a tile shape.
 bool strip_serves(const ebsd_plan_s* p, int method, int dtype) {
-    if (!p->st.ok || method != EBSD_FUSED_F32) return false;
+    if (!p->st.ok || method != EBSD_FUSED_F32 || p->tile_pinned) return false;
     if (dtype == EBSD_U8) return !(p->k1 >= 9 && p->fg.ok_f32 && p->fg.quad);
     return dtype == EBSD_U16;
 }
