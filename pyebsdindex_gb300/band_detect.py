@@ -685,8 +685,10 @@ class MixedBandDetect:
                 for f in _lib.BAND_FIELDS}
 
     def autotune(self, batches, stream=None, max_extra=3):
-        """Choose each size's theta-slab width for the one-launch mixed path (which float patterns
-        take; integer patterns run on the strip kernels whatever the width).  For every size in
+        """Choose each size's theta-slab width for the one-launch mixed path.  Where the strip
+        kernels serve every size of ``batches`` (integer patterns, no tile shape pinned) the mixed
+        call does not take that path: nothing is timed and the plans keep their slab tables
+        (``ms`` is empty).  Else, for every size in
         ``batches`` ({(H, W): CUDA tensor [n, H, W]}, a sample of each), the slab counts from
         the widest slabs that fit to ``max_extra`` narrower ones are timed on that size alone
         (the slab kernel, CUDA events on ``stream``, best of two runs after a warm-up), and the
@@ -697,11 +699,15 @@ class MixedBandDetect:
         dev = torch.device("cuda", self.gpu_id)
         st = stream if stream is not None else torch.cuda.current_stream(dev)
         chosen = {}
+        strips = all(self.plan(*key)._device_plan().strip_serves("fused", _input_code(t)) for key, t in batches.items())
         for key, t in batches.items():
             t, dt = _device_input(t, dev)
             plan = self.plan(*key)._device_plan()
             info = plan.get_tile()
             if info["slabs"] == 0 or not plan.supported("fused", dt):
+                continue
+            if strips:
+                chosen[key] = {"slabs": info["slabs"], "ms": {}}
                 continue
             outs = {f: v.data_ptr() for f, v in self._device_outputs(t.shape[0], dev).items()}
             e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
