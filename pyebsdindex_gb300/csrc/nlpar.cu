@@ -729,6 +729,7 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
             }
         }
         asm volatile("cp.async.commit_group;\ncp.async.wait_all;" ::: "memory");
+        __syncwarp();  // the aligned barrier takes whole warps; lanes past the chunk's end skipped the copies
         asm volatile("bar.sync 1, %0;" ::"n"(kHelpers * 32) : "memory");
         bool bad = false;
         for (int r = 0; r < nr; ++r) {
