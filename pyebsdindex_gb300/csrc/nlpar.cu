@@ -879,8 +879,7 @@ __global__ void k_nlpar_sigma_pairs(const float2* __restrict__ sigp, int nrows, 
 // pixels whose windows are centred; the edge pixels take k_nlpar_weights_edge.
 template <int MP>
 __global__ void __launch_bounds__(kTileX * kTy) k_nlpar_weights_pairs(
-        const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind,
-        int nind, float mxval, const float2* __restrict__ pairs, const float* __restrict__ sigma, float lam2,
+        int nrows, int ncols, const float2* __restrict__ pairs, const float* __restrict__ sigma, float lam2,
         float dthresh, int sr, float* __restrict__ wout, const float* __restrict__ coff) {
     __shared__ float W[kTileX * 49];
     __shared__ float T[kTileX];
@@ -906,15 +905,11 @@ __global__ void __launch_bounds__(kTileX * kTy) k_nlpar_weights_pairs(
             if (nb == pix) {
                 w = -1.0e6f;
             } else {
-                float d2, n2;
-                if (dy >= -sr && dy <= sr && dx >= -sr && dx <= sr) {
-                    const float2 e = (dy > 0 || (dy == 0 && dx > 0)) ? pairs[pix * nF + fwd_index(dy, dx, sr)]
-                                                                    : pairs[nb * nF + fwd_index(-dy, -dx, sr)];
-                    d2 = e.x;
-                    n2 = e.y;
-                } else {  // (not reached: the windows of these blocks are centred)
-                    pair_ssd(data + pix * npx, data + nb * npx, ind, nind, mxval, 0.0f, d2, n2);
-                }
+                // (the windows here are centred: every slot lies within +-sr)
+                const float2 e = (dy > 0 || (dy == 0 && dx > 0)) ? pairs[pix * nF + fwd_index(dy, dx, sr)]
+                                                                : pairs[nb * nF + fwd_index(-dy, -dx, sr)];
+                const float n2 = e.y;
+                float d2 = e.x;
                 float s0 = sigma[pix], s1 = sigma[nb];
                 s0 = __fmul_rn(s0, s0);
                 s1 = __fmul_rn(s1, s1);
@@ -1379,7 +1374,6 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
     if (2 * sr + 1 > nrows || 2 * sr + 1 > ncols) return EBSD_E_ARG;  // window must fit the scan
     const size_t asm_ = tiled_smem(sr, ncols, sizeof(float), false);
     if (asm_ > 48 * 1024) return EBSD_E_UNSUPPORTED;
-    const float mxval = saturation_protect ? datamax * 0.999f : datamax + 1.0f;
     const float lam2 = 1.0f / (lam * lam);
     const int64_t npix = (int64_t)nrows * ncols;
     const int winsz = (2 * sr + 1) * (2 * sr + 1), nF = sr * (2 * sr + 1) + sr;
@@ -1399,8 +1393,8 @@ int ebsd_nlpar_pairs_out(const float* d_data, int32_t nrows, int32_t ncols, int3
         if ((rc = launch_status()) != EBSD_OK) return rc;
     }
     const dim3 tgrid((unsigned)((ncols + kTileX - 1) / kTileX), (unsigned)nrows), tblock(kTileX, kTy);
-    k_nlpar_weights_pairs<4><<<tgrid, tblock, 0, st>>>(d_data, nrows, ncols, npx, d_indices, nind, mxval, pairs,
-                                                       d_sigma, lam2, dthresh, sr, w, d_centre_offset);
+    k_nlpar_weights_pairs<4><<<tgrid, tblock, 0, st>>>(nrows, ncols, pairs, d_sigma, lam2, dthresh, sr, w,
+                                                       d_centre_offset);
     if ((rc = launch_status()) != EBSD_OK) return rc;
     {
         // edge pixels: their weights
