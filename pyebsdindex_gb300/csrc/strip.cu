@@ -487,7 +487,10 @@ __global__ void __launch_bounds__(kPThreads, 2) k_strip_peaks(const __grid_const
         const int r_end = min(r_beg + a.strip_rows, CT);
         float best = 0.0f;
         __syncwarp();                                // the row buffers' last reads
-        if (r_beg < CT) {
+        if (r_beg >= CT) {                           // the slab has fewer strips than the widest
+            bests[task * 32 + lane] = 0.0f;
+            continue;
+        }
         const int c0 = seg * a.SW;
         const int cols = min(a.FC - c0, a.SW);       // this segment's columns
         const int first = c0 - kOff - H0;            // rho of the row buffer's first entry
@@ -616,7 +619,6 @@ __global__ void __launch_bounds__(kPThreads, 2) k_strip_peaks(const __grid_const
 #pragma unroll
             for (int k = 0; k < 4; ++k)
                 if (v1[k] >= fmaxf(t2[k], t1[k])) best = fmaxf(best, v1[k]);
-        }
         }
         bests[task * 32 + lane] = best;
         gbest = fmaxf(gbest, best);
@@ -1057,7 +1059,7 @@ int strip_prepare(ebsd_plan_s* p, const ebsd_plan_desc* d) {
     std::vector<StripTask> tasks;
     std::vector<uint16_t> lut;
     std::vector<uint32_t> act;
-        for (int o = 0; o < 4; ++o) {
+    for (int o = 0; o < 4; ++o) {
         struct Grp {
             int id, work;
         };
