@@ -580,13 +580,16 @@ __global__ void __launch_bounds__(32 * kBlurWarps) k_blur_lines(const float* __r
 }
 
 // Whether the blocked kernel takes the call: three and more taps a side (the triangles need
-// 2 r + 2 >= kBlurR) and lines that leave two blocks an SM (<= 96 KB of shared memory);
-// the others keep a thread per output.
+// 2 r + 2 >= kBlurR), lines that leave two blocks an SM (<= 96 KB of shared memory), and blocks enough:
+// with few of them each warp's chain of taps is all the time there is, and a thread per output fills
+// the chip.  120x120, r = 30: 30 blocks 10.7 .. 14.4 us blocked, 8.3 .. 10.4 with a thread per output; 60
+// blocks 11.5 .. 14.5 and 10.4 .. 16.5; 90 blocks 11.9 .. 14.4 and 14.4 .. 22.6.  Short filters need more:
+// r = 3, 120 blocks 6.4 .. 10.3 and 8.0 .. 8.4, 180 blocks 7.2 .. 10.3 and 8.4 .. 10.4.
 constexpr size_t kBlurSmemMax = 96 * 1024;
 inline bool blur_blocked(int64_t n, int H, int W, int axis, int r) {
-    const int64_t lines = axis == 0 ? n * W : n * H;
+    const int64_t lines = axis == 0 ? n * W : n * H, blocks = (lines + kBlurLines - 1) / kBlurLines;
     return r >= (kBlurR - 2) / 2 && blur_smem(axis == 0 ? H : W, axis, r) <= kBlurSmemMax &&
-           (lines + kBlurLines - 1) / kBlurLines <= 0x7fffffff;
+           blocks >= (r < 12 ? 152 : 64) && blocks <= 0x7fffffff;
 }
 
 template <int kAxis, bool kAdj>
