@@ -52,14 +52,14 @@ __global__ void k_csr_gather(const int64_t* __restrict__ rowptr, const int32_t* 
 //
 // Rows that neighbour in the image they index (rays of near angle and offset, near pixels) meet
 // the same columns at about the same place of their rows, so a block takes a tile of
-// kCsrTileY x kCsrTileX rows of that image and its reads of x^T hit L1 instead of L2.  A warp
-// takes kCsrRows neighbouring rows at once and 32 NV patterns: a nonzero costs one 8-byte
-// broadcast, and NV coalesced loads feed NV multiply-adds of independent chains.  Bound by the
-// L1's 128 bytes a cycle.  1024 patterns, 120x120 pixels, 180x180 rays: Radon 1261 us with a row
-// a warp and 32 patterns (16 TB/s, eight instructions a nonzero), 515 now; its adjoint 1235, 580
-// now; the LoG 451, 194 now.  With an address per load of a nonzero: 912, 1110, 318; four rows a warp
-// in 4 x 8 tiles (78 registers, 24 warps an SM): 582, 836, 215; one row: 520, 550, 193.
-constexpr int kCsrTileY = 4, kCsrTileX = 4, kCsrRows = 2;
+// kCsrTileY x kCsrTileX rows of that image and its reads of x^T hit L1 instead of L2.  A warp takes a
+// row and 32 NV patterns: a nonzero costs one 8-byte broadcast, and NV coalesced loads feed NV
+// multiply-adds of independent chains, eight nonzeros in flight.  Bound by the L1's 128 bytes a cycle.
+// 1024 patterns, 120x120 pixels, 180x180 rays: Radon 1260 us with a row a warp and 32 patterns, unrolled by
+// four (16 TB/s, eight instructions a nonzero), 479 now; its adjoint 1235, 496 now; the LoG 450, 183 now.
+// Two rows a warp, unrolled by two: 509, 566, 193, and half the warps where a batch is small (one
+// pattern of 60x60: the adjoint 58 us, 21 now).
+constexpr int kCsrTileY = 2, kCsrTileX = 4;
 
 template <typename T> struct CsrEnt;
 template <> struct CsrEnt<float> {
@@ -83,23 +83,14 @@ template <typename T, int NV>
 __global__ void __launch_bounds__(256) k_csr_gather_cols(const int64_t* __restrict__ rowptr, CsrEnt<T> ent,
                                                          const T* __restrict__ xT, int64_t ldx, T* __restrict__ yT,
                                                          int64_t ldy, int64_t nrows, int64_t width, int64_t n) {
-    static_assert(kCsrTileY * kCsrTileX == 8 * kCsrRows, "eight warps a tile");
-    constexpr int kWarpsX = kCsrTileX / kCsrRows;
+    static_assert(kCsrTileY * kCsrTileX == 8, "eight warps a tile");
     const int64_t tx = (width + kCsrTileX - 1) / kCsrTileX, ty = blockIdx.x / tx;
-    const int64_t gx = (blockIdx.x - ty * tx) * kCsrTileX + (threadIdx.y % kWarpsX) * kCsrRows;
-    const int64_t gy = ty * kCsrTileY + threadIdx.y / kWarpsX, row = gy * width + gx;
+    const int64_t gx = (blockIdx.x - ty * tx) * kCsrTileX + threadIdx.y % kCsrTileX;
+    const int64_t gy = ty * kCsrTileY + threadIdx.y / kCsrTileX, row = gy * width + gx;
     if (gx >= width || row >= nrows) return;
     const int64_t b0 = (int64_t)blockIdx.y * (32 * NV) + threadIdx.x;
-    int64_t e[kCsrRows];
-    int len[kCsrRows];
-    int common = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < kCsrRows; ++i) {
-        const int64_t r = gx + i < width && row + i < nrows ? row + i : row;  // past the image: the first row again
-        e[i] = __ldg(rowptr + r);
-        len[i] = (int)(__ldg(rowptr + r + 1) - e[i]);
-        common = len[i] < common ? len[i] : common;
-    }
+    const int64_t e0 = __ldg(rowptr + row);
+    const int len = (int)(__ldg(rowptr + row + 1) - e0);
     // kWhole: every pattern of the block exists, so that a nonzero's loads differ by constants from
     // one address; else patterns past the last read column 0 and are not stored
     auto run = [&](auto whole) {
@@ -108,50 +99,41 @@ __global__ void __launch_bounds__(256) k_csr_gather_cols(const int64_t* __restri
         int64_t off[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) off[v] = kWhole ? 32 * v : (b0 + 32 * v < n ? b0 + 32 * v : 0);
-        T acc[kCsrRows][NV];
+        T acc[NV];
 #pragma unroll
-        for (int i = 0; i < kCsrRows; ++i)
-#pragma unroll
-            for (int v = 0; v < NV; ++v) acc[i][v] = (T)0;
-        auto add = [&](int i, int64_t at) {
+        for (int v = 0; v < NV; ++v) acc[v] = (T)0;
+#pragma unroll 8
+        for (int t = 0; t < len; ++t) {
             int c;
             T a;
-            ent.get(at, c, a);
+            ent.get(e0 + t, c, a);
             const T* xr = xb + (int64_t)c * ldx;
 #pragma unroll
-            for (int v = 0; v < NV; ++v) acc[i][v] = fma(a, __ldg(xr + off[v]), acc[i][v]);
-        };
-#pragma unroll 2
-        for (int t = 0; t < common; ++t)
-#pragma unroll
-            for (int i = 0; i < kCsrRows; ++i) add(i, e[i] + t);
-#pragma unroll
-        for (int i = 0; i < kCsrRows; ++i) {
-#pragma unroll 4
-            for (int t = common; t < len[i]; ++t) add(i, e[i] + t);
-            if (gx + i < width && row + i < nrows)
-#pragma unroll
-                for (int v = 0; v < NV; ++v)
-                    if (kWhole || b0 + 32 * v < n) yT[(row + i) * ldy + b0 + 32 * v] = acc[i][v];
+            for (int v = 0; v < NV; ++v) acc[v] = fma(a, __ldg(xr + off[v]), acc[v]);
         }
+#pragma unroll
+        for (int v = 0; v < NV; ++v)
+            if (kWhole || b0 + 32 * v < n) yT[row * ldy + b0 + 32 * v] = acc[v];
     };
     if ((int64_t)(blockIdx.y + 1) * (32 * NV) <= n) run(std::true_type());
     else run(std::false_type());
 }
 
-// Patterns a warp: 128 in float, 64 in double; a batch of fewer takes what it fills.
+// Patterns a warp: in float as many as the batch fills, up to 128 (1024 patterns of 120x120: 479 us with 128,
+// 657 with 64, 1188 with 32; 64 of 60x60: 31, 16 and 25).  In double 32: the FP64 pipe bounds it, and wider
+// warps only pad the batch (200 patterns of 60x60: 246 us, 279 with 64, 279 with 128).
 template <typename T>
 void launch_csr_cols(cudaStream_t st, const int64_t* rowptr, CsrEnt<T> ent, const T* xT, int64_t ldx, T* yT, int64_t ldy,
                      int64_t nrows, int64_t width, int64_t n) {
     const unsigned tiles = (unsigned)(((width + kCsrTileX - 1) / kCsrTileX) * ((nrows + width * kCsrTileY - 1) / (width * kCsrTileY)));
-    const dim3 block(32, 8);
-    constexpr int kMost = sizeof(T) == 4 ? 4 : 2;
-    if (n > 64 && kMost == 4)
-        k_csr_gather_cols<T, kMost><<<dim3(tiles, (unsigned)((n + 32 * kMost - 1) / (32 * kMost))), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
-    else if (n > 32)
-        k_csr_gather_cols<T, 2><<<dim3(tiles, (unsigned)((n + 63) / 64)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
-    else
-        k_csr_gather_cols<T, 1><<<dim3(tiles, (unsigned)((n + 31) / 32)), block, 0, st>>>(rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
+    auto go = [&](auto nv) {
+        constexpr int NV = decltype(nv)::value;
+        k_csr_gather_cols<T, NV><<<dim3(tiles, (unsigned)((n + 32 * NV - 1) / (32 * NV))), dim3(32, 8), 0, st>>>(
+            rowptr, ent, xT, ldx, yT, ldy, nrows, width, n);
+    };
+    if (sizeof(T) == 8 || n <= 32) go(std::integral_constant<int, 1>());
+    else if (n <= 64) go(std::integral_constant<int, sizeof(T) == 4 ? 2 : 1>());
+    else go(std::integral_constant<int, sizeof(T) == 4 ? 4 : 1>());
 }
 
 __device__ __forceinline__ void window(int i, int sr, int n, int& start, int& end) {
