@@ -680,8 +680,11 @@ __device__ void edge_sums(float* sm, int block, const float* __restrict__ data, 
 // 2 SR + 2 values of row y + dy under both windows are loaded once as pairs and feed 2 SR + 1 packed
 // (two-pixel) differences, squares and sums, each rounded as its own.  The patterns' next kChunk
 // pixels stream into a second buffer (cp.async) while the current ones are summed, stored with the scan
-// columns along the fast axis.  A chunk with no value at or above a saturation level (nor a NaN) is
-// summed without the per-term tests and counted whole.  Measured, 128x160 scan of 80x80, radius 3: 1.35
+// columns along the fast axis.  A pattern pixel with no value at or above a saturation level (nor a NaN)
+// in the block's columns is summed without the per-term tests and counted whole; the others add zero
+// for a term that does not count (3 of 10,000 values saturated, 60x61 scan of 60x60, radius 2, with the
+// weights: 340 us; none 228; whole chunks term by term, branching: 1169 and 218; a sum per pair and slot,
+// which saturation does not slow: 1087).  Measured, 128x160 scan of 80x80, radius 3: 1.35
 // ms with one pair per thread and step (11 instructions a term, staging exposed), 0.84 ms now; bound by
 // the summing warps' dependent packed operations: the offsets' differences, squares and sums are issued
 // kind by kind and eight pixels unrolled (offset by offset, four pixels: 0.87; a third staging buffer,
@@ -689,8 +692,9 @@ __device__ void edge_sums(float* sm, int block, const float* __restrict__ data, 
 constexpr int kPairLanes = 30;                 // 60 pixels and 2 SR halo columns
 constexpr int kPairPitch = 66;                 // staged columns (2 modulo 32: a column's 32 pixels in 16 banks)
 
+// (Radius 3: the three blocks an SM that shared memory allows; left to itself the compiler spills with sigma.)
 template <int SR, bool kSig>
-__global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
+__global__ void __launch_bounds__(kPairThreads, SR == 3 ? 3 : 0) k_nlpar_pairs(
         const float* __restrict__ data, int nrows, int ncols, int npx, const int32_t* __restrict__ ind,
         int nind, float mxval, float mxsig, float zero, float2* __restrict__ pairs, float2* __restrict__ sigp,
         int edge_rows, int edge_all, float2* __restrict__ raw) {
@@ -701,7 +705,7 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         edge_sums(sm, blockIdx.x, data, nrows, ncols, npx, ind, nind, mxval, SR, edge_rows, raw);
         return;
     }
-    __shared__ int bad_s[2];                                      // the buffers' chunks hold a saturated value or a NaN
+    __shared__ unsigned bad_s[2];                                 // the pixels of the buffers' chunks with a saturated value or a NaN
     const int nxb = (ncols + 2 * kPairLanes - 1) / (2 * kPairLanes);
     const int y = ((int)blockIdx.x - edge_all) / nxb, x0 = ((int)blockIdx.x - edge_all - y * nxb) * 2 * kPairLanes;
     const int nr = min(SR + 1, nrows - y);                        // rows y .. y + nr - 1 exist
@@ -716,7 +720,7 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
     auto stage = [&](int q0, int b) {
         float* buf = sm + b * kBufF;
         const int q = q0 + lane, qn = min(kChunk, nind - q0);
-        if (helper == 0 && lane == 0) bad_s[b] = 0;
+        if (helper == 0 && lane == 0) bad_s[b] = 0u;
         if (q < nind) {
             const float* src = data + ((int64_t)y * ncols + x0 - SR) * npx + __ldg(ind + q);
             float* dst = buf + lane * kPairPitch;
@@ -740,7 +744,18 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
                 bad |= !(v.x < lim) | !(v.y < lim);
             }
         }
-        if (bad) bad_s[b] = 1;
+        if (bad) {  // which pixels: rarely needed, so looked for in a pass of its own
+            unsigned mask = 0u;
+            for (int r = 0; r < nr; ++r) {
+                const float2* row = (const float2*)(buf + r * kRowF);
+#pragma unroll 1
+                for (int i = helper * 32 + lane; i < qn * (kPairPitch / 2); i += kHelpers * 32) {
+                    const float2 v = row[i];
+                    if (!(v.x < lim) | !(v.y < lim)) mask |= 1u << (i / (kPairPitch / 2));
+                }
+            }
+            atomicOr(&bad_s[b], mask);
+        }
     };
     const bool mine = lane < kPairLanes && dy < nr && helper < 0;
     const int cl = mine ? 2 * lane : 0;                           // first staged column under pixel x = x0 + 2 lane
@@ -753,8 +768,10 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
     for (int e = 0; e < 3; ++e) ds[e] = 0ull, nsa[e] = 0.0f, nsb[e] = 0.0f;
     // sigma's forward neighbours: dx 1 in the same row; dx -1, 0, 1 in the next
     const bool near1 = kSig && dy == 1, near0 = kSig && dy == 0;
-    auto terms = [&](const float* q, int dyv, auto tag) {  // one pattern pixel, every term counted
+    // one pattern pixel; checked: a term counts if both its values lie below the level, else every term
+    auto terms = [&](const float* q, int dyv, auto tag, auto checked) {
         constexpr int kKind = decltype(tag)::value;        // 0: the same row (dx > 0), 1: the next, 2: others
+        constexpr bool kCheck = decltype(checked)::value;
         const float* pa = q + cl + SR;
         const Pair2 a = (SR & 1) ? p2_pack(pa[0], pa[1]) : *(const Pair2*)pa;
         const float* pb = q + dyv * kRowF + cl;
@@ -771,11 +788,44 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         }
 #pragma unroll
         for (int e = e0; e < WN; ++e) t[e] = p2_mul(t[e], t[e], z);
+        if (kCheck) {
+            // a sum of squares plus zero is the sum, so a term that does not count adds zero
+            const float2 av = p2_unpack(a);
+            auto value = [&](int c) { return (c & 1) ? p2_unpack(v[c / 2]).y : p2_unpack(v[c / 2]).x; };
+#pragma unroll
+            for (int e = e0; e < WN; ++e) {
+                const float2 u = p2_unpack(t[e]);
+                const bool oka = av.x < mxval && value(e) < mxval, okb = av.y < mxval && value(e + 1) < mxval;
+                d[e] = p2_add(d[e], p2_pack(oka ? u.x : 0.0f, okb ? u.y : 0.0f));
+                na[e] += oka ? 1.0f : 0.0f;
+                nb[e] += okb ? 1.0f : 0.0f;
+                const int g = kKind == 0 ? 0 : e - SR + 1;  // sigma's sums
+                if (kSig && (kKind == 0 ? e == SR + 1 : kKind == 1 && g >= 0 && g <= 2)) {
+                    const bool sa = av.x < mxsig && value(e) < mxsig, sb = av.y < mxsig && value(e + 1) < mxsig;
+                    ds[g] = p2_add(ds[g], p2_pack(sa ? u.x : 0.0f, sb ? u.y : 0.0f));
+                    nsa[g] += sa ? 1.0f : 0.0f;
+                    nsb[g] += sb ? 1.0f : 0.0f;
+                }
+            }
+            return;
+        }
 #pragma unroll
         for (int e = e0; e < WN; ++e) {
             d[e] = p2_add(d[e], t[e]);
             if (kSig && kKind == 0 && e == SR + 1) ds[0] = p2_add(ds[0], t[e]);
             if (kSig && kKind == 1 && e >= SR - 1 && e <= SR + 1) ds[e - SR + 1] = p2_add(ds[e - SR + 1], t[e]);
+        }
+    };
+    // a chunk of qn pixels, every term counted; and one with the pixels of the mask `bad` term by term
+    auto whole = [&](const float* cur, int qn, int dyv, auto tag) {
+#pragma unroll 8
+        for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, dyv, tag, std::false_type());
+    };
+    auto mixed = [&](const float* cur, int qn, unsigned bad, int dyv, auto tag) {
+#pragma unroll 1
+        for (int qq = 0; qq < qn; ++qq) {
+            if ((bad >> qq) & 1u) terms(cur + qq * kPairPitch, dyv, tag, std::true_type());
+            else terms(cur + qq * kPairPitch, dyv, tag, std::false_type());
         }
     };
     if (helper >= 0) stage(0, 0);
@@ -785,47 +835,20 @@ __global__ void __launch_bounds__(kPairThreads) k_nlpar_pairs(
         const int qn = min(kChunk, nind - q0);
         if (helper >= 0) {
             if (q0 + kChunk < nind) stage(q0 + kChunk, (it + 1) & 1);
-        } else if (bad_s[it & 1]) {
-            if (mine) {
-                for (int qq = 0; qq < qn; ++qq) {
-                    const float* q = cur + qq * kPairPitch;
-                    const float xa = q[cl + SR], xb = q[cl + SR + 1];
-#pragma unroll
-                    for (int e = 0; e < WN; ++e) {
-                        const float ya = q[dy * kRowF + cl + e], yb = q[dy * kRowF + cl + e + 1];
-                        const float ta = __fsub_rn(xa, ya), tb = __fsub_rn(xb, yb);
-                        const float sa = __fmul_rn(ta, ta), sb = __fmul_rn(tb, tb);
-                        float2 s = p2_unpack(d[e]);  // pair_ssd's order: count, difference, square
-                        if (ya < mxval && xa < mxval) s.x = __fadd_rn(s.x, sa), na[e] += 1.0f;
-                        if (yb < mxval && xb < mxval) s.y = __fadd_rn(s.y, sb), nb[e] += 1.0f;
-                        d[e] = p2_pack(s.x, s.y);
-                        const int g = e - SR + 1;
-                        if (kSig && ((near1 && g >= 0 && g <= 2) || (near0 && g == 2))) {
-#pragma unroll
-                            for (int z = 0; z < 3; ++z) {
-                                if (z != (near0 ? 0 : g)) continue;
-                                float2 w = p2_unpack(ds[z]);
-                                if (ya < mxsig && xa < mxsig) w.x = __fadd_rn(w.x, sa), nsa[z] += 1.0f;
-                                if (yb < mxsig && xb < mxsig) w.y = __fadd_rn(w.y, sb), nsb[z] += 1.0f;
-                                ds[z] = p2_pack(w.x, w.y);
-                            }
-                        }
-                    }
-                }
-            }
         } else if (mine) {
-            // every term of the chunk counts (the counts are exact integers either way)
-            if (dy == 0) {
-#pragma unroll 8
-                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 0, std::integral_constant<int, 0>());
+            const unsigned bad = bad_s[it & 1];
+            if (bad == 0u) {
+                if (dy == 0) whole(cur, qn, 0, std::integral_constant<int, 0>());
+                else if (dy == 1) whole(cur, qn, 1, std::integral_constant<int, 1>());
+                else whole(cur, qn, dy, std::integral_constant<int, 2>());
+            } else if (dy == 0) {
+                mixed(cur, qn, bad, 0, std::integral_constant<int, 0>());
             } else if (dy == 1) {
-#pragma unroll 8
-                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, 1, std::integral_constant<int, 1>());
+                mixed(cur, qn, bad, 1, std::integral_constant<int, 1>());
             } else {
-#pragma unroll 8
-                for (int qq = 0; qq < qn; ++qq) terms(cur + qq * kPairPitch, dy, std::integral_constant<int, 2>());
+                mixed(cur, qn, bad, dy, std::integral_constant<int, 2>());
             }
-            n0 += (float)qn;
+            n0 += (float)(qn - __popc(bad));               // (the counts are exact integers either way)
         }
         __syncthreads();  // the next chunk is in place, this one's buffer free
     }
