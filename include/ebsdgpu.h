@@ -153,7 +153,7 @@ int ebsd_find_bands_host(ebsd_plan_t plan, int method, int dtype, const void* h_
  * with copies; 1: always read in place.  Either way every input byte crosses the link once
  * per call.  Pageable input is staged through pinned buffers, except by -1 in a call of one
  * chunk of integer patterns (at most 64 MB) that the strip kernels serve: such input is read in
- * place too, and pinned integer input of a larger call that they serve is staged with copies
+ * place too, and pinned integer input of a call above 1 MB that they serve is staged with copies
  * (their packing would wait for the link).  Input whose address is no multiple of its type's
  * size is staged in every mode. */
 int ebsd_plan_set_host_input(ebsd_plan_t plan, int mode);

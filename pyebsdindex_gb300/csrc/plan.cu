@@ -238,6 +238,12 @@ ebsd_bands chunk_fields(char* base, size_t nb) {
 // reads pageable memory at 24 GB/s only.  The strip path's kernels read every input byte once.
 constexpr size_t kInPlaceBytes = (size_t)64 << 20;
 
+// Pinned input that the strip path serves is read in place up to here: beyond, its packing kernel would wait
+// for the link in front of the sums, and the copy engines are faster at every size (60x60 uint8, 4 MB: 500 us
+// in place, 490 staged; 16 MB: 1395, 1317; 60 MB: 3642, 3289, and 3296 for the one-tile kernel in place; a
+// million 80x80 patterns in chunks: 4.8 M/s, 6.5 M/s); below, the staging buffers are not worth having.
+constexpr size_t kPinnedInPlaceBytes = (size_t)1 << 20;
+
 // The host touches the input's pages first, so that a page the system has yet to provide is faulted in
 // here and not under the GPU.
 void touch_pages(const char* mem, size_t bytes) {
@@ -299,10 +305,9 @@ int host_pipeline(ebsd_plan_s* p, int method, int dtype, const ChunkSource& src,
             in_place = (const char*)pa.devicePointer;
         cudaGetLastError();
     }
-    // ... unless the strip path serves a call of more than kInPlaceBytes: its packing kernel would wait
-    // for the link in front of every chunk's sums (a million 80x80 patterns 4.8 M/s, staged by the copy
-    // engines beside them 6.7 M/s); without memory to stage it, it is read in place after all
-    if (in_place && p->host_input_mode == -1 && (size_t)n * src.pat_bytes > kInPlaceBytes &&
+    // ... unless the strip path serves a call of more than kPinnedInPlaceBytes; without memory to stage it,
+    // it is read in place after all
+    if (in_place && p->host_input_mode == -1 && (size_t)n * src.pat_bytes > kPinnedInPlaceBytes &&
         strip_serves(p, method, dtype)) {
         if (regrow(p->h_in_dev, 2, &p->h_in_bytes, in_bytes, false) == EBSD_OK) in_place = nullptr;
         cudaGetLastError();
