@@ -26,6 +26,7 @@
 #include "label.cuh"
 
 #include <cstring>
+#include <new>
 #include <type_traits>
 
 namespace ebsd {
@@ -1337,7 +1338,8 @@ bool capture_scratch(ebsd_plan_s* p, cudaStream_t st, unsigned long long id, cud
         slot->mem = StripScratch{};
         if (scratch_alloc(p->st, cap, &slot->mem) != EBSD_OK) return give_back();
     }
-    CaptureHold* hold = new CaptureHold{p->st_captures, slot};
+    CaptureHold* hold = new (std::nothrow) CaptureHold{p->st_captures, slot};
+    if (!hold) return give_back();
     cudaUserObject_t obj = nullptr;
     if (cudaUserObjectCreate(&obj, hold, capture_gone, 1, cudaUserObjectNoDestructorSync) != cudaSuccess) {
         cudaGetLastError();
@@ -1381,7 +1383,13 @@ bool strip_ready(ebsd_plan_s* p, cudaStream_t st, int64_t n, StripScratch* got) 
         cudaGetLastError();
         return false;
     }
-    if (cap == cudaStreamCaptureStatusActive) return capture_scratch(p, st, id, graph, n, got);
+    if (cap == cudaStreamCaptureStatusActive) {
+        try {
+            return capture_scratch(p, st, id, graph, n, got);
+        } catch (const std::bad_alloc&) {
+            return false;
+        }
+    }
     if (cap != cudaStreamCaptureStatusNone || strip_reserve(p, n) != EBSD_OK) return false;
     *got = p->st_ws;
     return true;
