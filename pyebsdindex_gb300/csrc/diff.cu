@@ -599,6 +599,7 @@ int launch_blur(const float* in, int64_t n, int H, int W, const float* taps, int
 // (P. Markstein, IBM J. Res. Dev. 34(1), 1990).
 // 1024 patterns of 180x180 cells: 1660 us before, 911 now, the same bits.  Arguments and gradient in pairs of
 // floats took 473, but kept 45 bits of c / tau only, which shows in the gradient from c / tau = 2^24 on.
+
 // (double)f by integer operations (a conversion instruction runs at the FP64 pipe's rate)
 __device__ __forceinline__ double widen(float f) {
     const unsigned u = __float_as_uint(f), sign = u & 0x80000000u;
